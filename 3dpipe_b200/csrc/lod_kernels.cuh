@@ -1,0 +1,89 @@
+// lod_kernels.cuh -- one LOD of the tuned join as a chain of task kernels
+// (csrc/lod_kernels.cu).  All state stays in device memory; no kernel needs a
+// count on the host.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "common.cuh"
+#include "join_kernels.cuh"
+
+namespace tdp {
+
+constexpr int kLodCtrWords = 8;   // counters of one pass over the items
+constexpr int kMaxPasses = 10;    // up to 8 LODs, the redo pass, one spare
+
+// A queued cluster pair of item w: z and y are its lower bounds of the
+// Hausdorff-widened upper and lower bound (less the item's FP32 margin), so
+// that a later look at the running caps can drop it without its clusters.
+struct alignas(16) LodTask {
+    uint32_t w, ij;
+    float z, y;
+};
+
+// A queued triangle pair: item, triangles, lower bound (less the margin) of
+// its upper bound; -inf where its lower bound matters too.
+struct alignas(16) LodEval {
+    uint32_t w, a, b;
+    float z;
+};
+
+struct LodDev {
+    JoinDev d;
+    const float* box1;  // 6 floats per object (low, high)
+    const float* box2;
+    int self;      // tile 2 is tile 1: one set of cluster records
+    int level;     // Hausdorff level
+    int nl;        // LODs of the join
+    const uint32_t* vt1[8];
+    const uint32_t* vt2[8];
+    const float4* tri1[8];
+    const float4* tri2[8];
+    int li[8];
+    // items of the current pass
+    RefineItem* items;
+    int4* ext;     // per item: voxel pair, object pair, first A cluster, first B cluster
+    int2* vox;     // per item: A voxel, B voxel
+    float4* mg;    // per item: FP32 margin of its bounds, slack, preset, 1 once it is in `over`
+    // caps
+    unsigned long long* pbest;  // per pair: (core distance, item) of the first LOD's closest cores
+    float* pcap;   // per pair: smallest upper bound so far
+    float* pd;     // per pair: the last LOD's running distance
+    uint8_t* pown; // per pair: 1 = caps per voxel pair (vmx) instead of pcap
+    uint8_t* pmiss;  // per pair: 1 = nothing of its last LOD came below its cap: done again without it
+    float* vres;   // per voxel pair: distance minimum (last LOD; levels 0 and 1)
+    // cluster records of the voxels in use at the current LOD
+    float4* cl1;
+    float4* cl2;
+    float4* vb1;   // 2 float4 per voxel: exact box of its triangles at this LOD
+    float4* vb2;
+    int* flag1;    // per voxel: LOD stamp of its cluster records
+    int* flag2;
+    int* list1;    // voxels whose records are built at this LOD
+    int* list2;
+    long nvox1, nvox2;
+    // cluster pairs that survive the cull
+    LodTask* tasks;
+    unsigned task_cap;
+    LodEval* evals;  // triangle pairs that survive their tests
+    unsigned eval_cap;
+    unsigned* over;  // items whose tasks or triangle pairs did not fit
+    unsigned* ctr;   // kLodCtrWords words per pass, zeroed
+    unsigned* n_items;         // per LOD item counts (zeroed)
+    unsigned long long* tri_pairs;
+    unsigned long long* n_full;
+    int use_preset;  // last LOD of a join with within queries: no distance above the query's
+    float tau;
+    int num_sms;
+};
+
+cudaError_t launch_lod_items(const LodDev& L, int k, cudaStream_t s);
+// clusters, (first LOD) seeds, cull, evaluation of LOD k's items
+cudaError_t launch_lod_refine(const LodDev& L, int k, int highest, cudaStream_t s);
+// the pairs' bounds, evictions and the within decision; at the last LOD also
+// the items of the pairs that have to be done again without their caps
+cudaError_t launch_lod_update(const LodDev& L, int k, int highest, int decide, cudaStream_t s);
+// the last LOD again for those pairs (normally none)
+cudaError_t launch_lod_redo(const LodDev& L, int k, int decide, cudaStream_t s);
+
+}  // namespace tdp

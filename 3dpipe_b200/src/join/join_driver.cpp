@@ -29,6 +29,7 @@
 #include "../../csrc/cand_kernels.cuh"
 #include "../../csrc/exact_kernels.cuh"
 #include "../../csrc/fetch_kernels.cuh"
+#include "../../csrc/lod_kernels.cuh"
 #include "../../csrc/refine.cuh"
 #include "index/candidates.h"
 #include "storage/dev_tile.h"
@@ -48,6 +49,8 @@ enum Slot {
     kPexOut = 76, kOutD64,            // exact distances (64-75 and 78-81 are the exact stage's own)
     kQk = 82, kQtau,                  // per query object queries
     kPreset = 91,                     // the last LOD's item presets (within queries)
+    kLodExt = 101, kLodVox, kLodMg, kLodCaps, kLodFlags, kLodZero, kLodVres, kLodCl1, kLodCl2, kLodVb1, kLodVb2,
+    kLodLists, kLodTasks, kLodOver, kLodEvals, kLodBest,   // the LOD loop's task form
 };
 
 template <typename T>
@@ -83,7 +86,50 @@ struct LodLoop {
     LazyTile lz1, lz2;  // attached tiles: fetch each LOD's voxels before its refine
     cudaStream_t side;  // attached tiles: the next LOD's prefetch runs here
     cudaEvent_t pf[16];
+    // configuration 0 at every LOD (the default): the loop as task kernels
+    // (csrc/lod_kernels.cuh), 3 to 5 times as fast on kNN joins as the fastest
+    // of the other configurations, which stay for callers that pin one
+    int tasks;
+    LodDev t;
+    size_t caps_bytes, best_bytes, flags_bytes, zero_bytes;
 };
+
+// The loop as task kernels: per LOD the items, their refine in three or four
+// launches, the update; no count is reset in between.
+int enqueue_task_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool capturing) {
+#define CUL(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) return fail(ctx, TDP_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(_e)); } while (0)
+    auto rec = [&](cudaEvent_t e) {
+        return capturing ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
+    };
+    CUL(cudaMemsetAsync(L.counter + 8, 0, 26 * sizeof(unsigned), s));
+    CUL(cudaMemsetAsync(L.dstats, 0, 8, s));
+    CUL(cudaMemsetAsync(L.t.pcap, 0x7f, L.caps_bytes, s));     // 3.4e38: above any bound
+    CUL(cudaMemsetAsync(L.t.pbest, 0xff, L.best_bytes, s));
+    CUL(cudaMemsetAsync(L.t.flag1, 0xff, L.flags_bytes, s));
+    CUL(cudaMemsetAsync(L.t.ctr, 0, L.zero_bytes, s));
+    const bool prefetch = (L.lz1.on || L.lz2.on) && L.side;
+    for (int k = 0; k < L.nl; ++k) {
+        const int highest = k == L.highest_k;
+        CUL(launch_lod_items(L.t, k, s));
+        if (prefetch && k > 0) CUL(cudaStreamWaitEvent(s, L.pf[2 * (k - 1) + 1], 0));
+        CUL(launch_fetch_items(L.items, L.t.n_items + k, 0, L.li[k], L.lz1, L.lz2, L.num_sms, s));
+        if (prefetch && k + 1 < L.nl) {
+            CUL(cudaEventRecord(L.pf[2 * k], s));
+            CUL(cudaStreamWaitEvent(L.side, L.pf[2 * k], 0));
+            CUL(launch_prefetch_pairs(L.d.valive, L.d.vpair, L.d.pstat, L.d.vpa, L.d.vpb, L.V, L.li[k + 1], L.lz1,
+                                      L.lz2, L.num_sms, L.side));
+            CUL(cudaEventRecord(L.pf[2 * k + 1], L.side));
+        }
+        CUL(rec(L.ev[2 * k]));
+        CUL(launch_lod_refine(L.t, k, highest, s));
+        CUL(rec(L.ev[2 * k + 1]));
+        CUL(launch_lod_update(L.t, k, highest, L.any_within, s));
+        if (highest) CUL(launch_lod_redo(L.t, k, L.any_within, s));
+        if (L.any_knn) CUL(launch_knn_rank(L.d, L.K, 1, L.rankst, s));
+    }
+#undef CUL
+    return TDP_OK;
+}
 
 // Enqueue the loop on s.  While s is being captured, the per-LOD timing events
 // become event-record nodes of the graph (cudaEventRecordExternal), so that
@@ -97,6 +143,10 @@ int enqueue_lod_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captur
     unsigned* lod_counts = L.counter + 24;   // per-LOD item counts
     unsigned* cnt_recheck = L.counter + 32;  // pairs left for the FP64 recheck
     const int V = (int)L.V;
+    if (L.tasks) {
+        const int rc = enqueue_task_loop(ctx, L, s, capturing);
+        if (rc != TDP_OK) return rc;
+    } else {
     CUL(cudaMemsetAsync(L.counter + 8, 0, 26 * sizeof(unsigned), s));
     CUL(cudaMemsetAsync(L.dstats, 0, 8, s));
     // Attached tiles: once LOD k's own voxels are fetched, a second stream
@@ -128,6 +178,7 @@ int enqueue_lod_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captur
         // reads every candidate of a query and stays its own launch
         CUL(launch_pair_update(L.d, k, 1, s, L.any_within ? 1 : 0, L.tau));
         if (L.any_knn) CUL(launch_knn_rank(L.d, L.K, 1, L.rankst, s));
+    }
     }
     if (L.recheck) {
         CUL(launch_count_status(L.d, cnt_recheck, s));
@@ -473,12 +524,59 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         L.preset = presets ? buf<float>(ctx, kPreset) : nullptr;
         L.side = ctx->side;
         for (int k = 0; k < 16; ++k) L.pf[k] = ctx->pf_ev[k];
+        L.tasks = 1;
+        for (int k = 0; k < L.nl; ++k) L.tasks = L.tasks && L.cfg[k] == 0;
+        if (L.tasks) {
+            LodDev& t = L.t;
+            size_t c1 = 0, c2 = 0;  // cluster records of a LOD: at most one per 8 triangles and one more per voxel
+            for (int k = 0; k < L.nl; ++k) {
+                c1 = std::max<size_t>(c1, t1->host.n_tris[L.li[k]] / 8 + t1->n_vox + 1);
+                c2 = std::max<size_t>(c2, t2->host.n_tris[L.li[k]] / 8 + t2->n_vox + 1);
+            }
+            const size_t nv1 = (size_t)std::max<long>(t1->n_vox, 1), nv2 = self ? 0 : (size_t)std::max<long>(t2->n_vox, 1);
+            const size_t ctr_bytes = kLodCtrWords * kMaxPasses * sizeof(unsigned);
+            t.task_cap = (unsigned)std::min<int64_t>(std::max<int64_t>(16 * V, 1 << 17), 1 << 23);
+            t.eval_cap = (unsigned)std::min<int64_t>(std::max<int64_t>(8 * V, 1 << 17), 1 << 22);
+            L.caps_bytes = 2 * Pz * 4;
+            L.best_bytes = Pz * 8;
+            L.flags_bytes = (nv1 + nv2) * 4;
+            L.zero_bytes = ctr_bytes + 2 * Pz;
+            ENS(kLodExt, Vz * sizeof(int4)); ENS(kLodVox, Vz * sizeof(int2)); ENS(kLodMg, Vz * sizeof(float4));
+            ENS(kLodCaps, L.caps_bytes); ENS(kLodBest, L.best_bytes); ENS(kLodFlags, L.flags_bytes); ENS(kLodZero, L.zero_bytes);
+            ENS(kLodVres, Vz * 4); ENS(kLodCl1, c1 * 3 * sizeof(float4)); ENS(kLodVb1, nv1 * 2 * sizeof(float4));
+            if (!self) { ENS(kLodCl2, c2 * 3 * sizeof(float4)); ENS(kLodVb2, nv2 * 2 * sizeof(float4)); }
+            ENS(kLodLists, (nv1 + nv2) * 4); ENS(kLodTasks, (size_t)t.task_cap * sizeof(LodTask)); ENS(kLodOver, Vz * 4);
+            ENS(kLodEvals, (size_t)t.eval_cap * sizeof(LodEval));
+            t.d = d;
+            t.box1 = t1->d_boxes; t.box2 = t2->d_boxes;
+            t.self = self ? 1 : 0; t.level = prm->hausdorff_level; t.nl = L.nl;
+            for (int k = 0; k < L.nl; ++k) {
+                t.vt1[k] = L.vt1[k]; t.vt2[k] = L.vt2[k]; t.tri1[k] = L.tri1[k]; t.tri2[k] = L.tri2[k]; t.li[k] = L.li[k];
+            }
+            t.items = items; t.ext = buf<int4>(ctx, kLodExt); t.vox = buf<int2>(ctx, kLodVox); t.mg = buf<float4>(ctx, kLodMg);
+            t.pbest = buf<unsigned long long>(ctx, kLodBest); t.evals = buf<LodEval>(ctx, kLodEvals);
+            t.pcap = buf<float>(ctx, kLodCaps); t.pd = t.pcap + Pz;
+            t.ctr = buf<unsigned>(ctx, kLodZero);
+            t.pown = (uint8_t*)t.ctr + ctr_bytes; t.pmiss = t.pown + Pz;
+            t.vres = buf<float>(ctx, kLodVres);
+            t.cl1 = buf<float4>(ctx, kLodCl1); t.vb1 = buf<float4>(ctx, kLodVb1);
+            t.cl2 = self ? t.cl1 : buf<float4>(ctx, kLodCl2); t.vb2 = self ? t.vb1 : buf<float4>(ctx, kLodVb2);
+            t.flag1 = buf<int>(ctx, kLodFlags); t.flag2 = self ? t.flag1 : t.flag1 + nv1;
+            t.list1 = buf<int>(ctx, kLodLists); t.list2 = self ? t.list1 : t.list1 + nv1;
+            t.nvox1 = (long)nv1; t.nvox2 = (long)nv2;
+            t.tasks = buf<LodTask>(ctx, kLodTasks); t.over = buf<unsigned>(ctx, kLodOver);
+            t.n_items = ctx->d_counter + 24;
+            t.tri_pairs = (unsigned long long*)(ctx->d_counter + 10);
+            t.n_full = ctx->d_stats;
+            t.use_preset = presets ? 1 : 0; t.tau = within_dist; t.num_sms = ctx->num_sms;
+        }
         if ((rc = run_lod_loop(ctx, L, s, &st.lod_graph))) return rc;
         {   // per LOD: items, refine, apply, pair update (with the within decision),
             // the kNN rank; on attached tiles the fetch and the next LOD's prefetch
             const bool attached = L.lz1.on || L.lz2.on;
             // (a fetch or a prefetch is a mark launch and a copy launch)
-            launches += (4 + (L.any_knn ? 1 : 0) + (attached ? 2 : 0)) * L.nl +
+            // (task form: six a LOD, the seeds of the first and four of the redo)
+            launches += ((L.tasks ? 6 : 4) + (L.any_knn ? 1 : 0) + (attached ? 2 : 0)) * L.nl + (L.tasks ? 5 : 0) +
                         (attached && L.side ? 2 * (L.nl - 1) : 0) +
                         (L.recheck ? (knn ? 5 : 4) + (attached ? 2 : 0) : 0);
         }
@@ -636,6 +734,7 @@ int tdp_autotune(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp
     double lod_best[kNumLods];
     int lod_arg[kNumLods];
     for (int l = 0; l < kNumLods; ++l) { lod_best[l] = 1e300; lod_arg[l] = -1; }
+    double ms0 = 0;  // configuration 0: all LODs as task kernels, or none
     for (int cfg = 0; cfg < kTunedConfigs; ++cfg) {
         ctx->tuned_cfg = cfg;
         double ms = 0;
@@ -655,11 +754,19 @@ int tdp_autotune(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp
             best_ms = ms;
             best_cfg = cfg;
         }
-        // the fastest configuration at each LOD the join refined
-        for (int l = 0; l < kNumLods; ++l) {
+        if (cfg == 0) ms0 = ms;
+        // the fastest of the other configurations at each LOD the join refined
+        for (int l = 0; l < kNumLods && cfg > 0; ++l) {
             const double m = ctx->stats.refine_ms_lod[l];
             if (m > 0 && m < lod_best[l]) { lod_best[l] = m; lod_arg[l] = cfg; }
         }
+    }
+    double mixed_ms = 0;
+    for (int l = 0; l < kNumLods; ++l) mixed_ms += lod_arg[l] >= 0 ? lod_best[l] : 0;
+    if (best_cfg == 0 && mixed_ms > 0 && mixed_ms < ms0) {
+        best_cfg = lod_arg[kNumLods - 1] >= 0 ? lod_arg[kNumLods - 1] : 1;
+    } else if (best_cfg == 0) {
+        for (int& l : lod_arg) l = 0;
     }
     ctx->tuned_cfg = best_cfg;
     for (int l = 0; l < kNumLods; ++l) ctx->lod_cfg[l] = lod_arg[l];
