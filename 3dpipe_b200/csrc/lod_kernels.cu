@@ -21,12 +21,12 @@
 //                   and the exact box of the voxel's triangles
 //   k_lod_seed      first LOD only: the most promising cluster pair of each
 //                   item lowers its pair's cap to near its final value
-//   k_lod_cull      one warp per item: the cluster pairs that can matter go to
-//                   a queue in device memory
-//   k_lod_eval      persistent: half a warp tests a queued cluster pair's 64
-//                   triangle pairs by their exact extents along the line of
-//                   the two centres; what is left is evaluated 32 at a time,
-//                   one triangle pair a lane, whichever items they belong to
+//   k_lod_cull      the cluster pairs that can matter go to a queue in device
+//                   memory
+//   k_lod_test      half a warp tests a queued cluster pair's 64 triangle pairs
+//                   by their exact extents along the line of the two centres
+//   k_lod_eval      what is left is evaluated 32 at a time, one triangle pair a
+//                   lane, whichever items they belong to
 //   k_lod_update    the pair's bounds, evictions, the within decision
 //
 // One warp per voxel pair spent half of its issue slots on staging bounds and
@@ -34,10 +34,10 @@
 // long as its slowest one.  Here most items end after one pass over cluster
 // pairs and the rest of the work is spread over the chip.  Whole joins on one
 // B200, before (configuration 0, or autotuned where noted) and with this file:
-//   10-NN, 20,000 nuclei x 100 vessels   35.4 -> 6.8 ms
-//       (137 M full triangle evaluations -> 3.4 M)
-//   10-NN self-join, 3,000 nuclei        23.9 (autotuned) -> 5.5 ms
-//   within 60 self-join, 4,181 nuclei    3.5 -> 1.1 ms
+//   10-NN, 20,000 nuclei x 100 vessels   35.4 -> 6.0 ms
+//       (137 M full triangle evaluations -> 1.9 M)
+//   10-NN self-join, 3,000 nuclei        23.9 (autotuned) -> 4.6 ms
+//   within 60 self-join, 4,181 nuclei    3.5 -> 1.0 ms
 //   within 150, 2,000 x 100              1.87 -> 0.74 ms
 //   within 400, 20,000 x 100             1.14 (autotuned) -> 0.86 ms
 // Evaluating inside the kernel that tests the triangle pairs (128 registers,
@@ -173,6 +173,7 @@ __device__ __forceinline__ float grp8_sum(float v) {
     return v;
 }
 
+// One warp per voxel in use.
 __global__ void __launch_bounds__(256) k_lod_clusters(LodDev L, int k) {
     const int lane = threadIdx.x & 31;
     const unsigned* ctr = L.ctr + k * kLodCtrWords;
@@ -266,12 +267,10 @@ __device__ __forceinline__ float cluster_gap(const Cluster& a, const Cluster& b)
     return d2 * inv - ra - rb;
 }
 
+// a gap widened by triangles' own Hausdorff values: (upper bound's, lower bound's)
 template <int MODE>
-__device__ __forceinline__ float2 widen(float gap, float mg, const Cluster& a, const Cluster& b, float3 oh) {
-    // (z, y): below the cap, below the voxel pair's own lower bound
-    if (MODE == kTriH) return make_float2(gap + a.h + b.h - mg, gap - a.ph - b.ph - mg);
-    if (MODE == kObjH) return make_float2(gap + oh.x + oh.y - mg, gap - oh.z - mg);
-    return make_float2(gap - mg, INFINITY);
+__device__ __forceinline__ float2 widen(float gap, const Cluster& a, const Cluster& b) {
+    return MODE == kTriH ? make_float2(gap + a.h + b.h, gap - a.ph - b.ph) : make_float2(gap, gap);
 }
 
 // kObjH: what is added for the upper bound (x, y, one after the other) and
@@ -294,11 +293,28 @@ __device__ __forceinline__ float2 thresholds(const LodDev& L, int v, int p, floa
     const float* cap = L.pown[p] ? L.d.vmx + v : L.pcap + p;
     return make_float2(__ldcg(cap), MODE == kObjH && L.level == 0 ? -INFINITY : __ldcg(L.d.vmn + v));
 }
-// NaN bounds keep the pair
-__device__ __forceinline__ bool matters(float2 zy, float2 t) { return !(zy.x >= t.x) || !(zy.y >= t.y); }
+// the same, with the item's margin, on the scale of a widened gap; a bound that
+// is not at or above its limit (NaN too) matters
+template <int MODE>
+__device__ __forceinline__ float2 gap_limits(const LodDev& L, int k, int p, float2 th, float mg) {
+    float zt = th.x + mg, yt = th.y + mg;
+    if (MODE == kObjH) {
+        const float3 oh = object_h(L, p, k);
+        zt -= oh.x + oh.y;
+        yt += oh.z;
+    }
+    return make_float2(zt, yt);
+}
+__device__ __forceinline__ bool lower_to(float* at, float x) {
+    if (!(x < __ldcg(at))) return false;
+    return atomicMin((unsigned*)at, __float_as_uint(x)) > __float_as_uint(x);
+}
 
-__device__ __forceinline__ void lower_to(float* at, float x) {
-    if (x < __ldcg(at)) atomicMin((unsigned*)at, __float_as_uint(x));
+// from the middle of triangle A to the middle of triangle B
+__device__ __forceinline__ float4 tri_to_tri(const PreTri<float>& A, const PreTri<float>& B) {
+    return make_float4(B.v[0].x + B.v[1].x + B.v[2].x - A.v[0].x - A.v[1].x - A.v[2].x,
+                       B.v[0].y + B.v[1].y + B.v[2].y - A.v[0].y - A.v[1].y - A.v[2].y,
+                       B.v[0].z + B.v[1].z + B.v[2].z - A.v[0].z - A.v[1].z - A.v[2].z, 0.f);
 }
 
 // largest |coordinate| of both voxels relative to o: rounding x - o is
@@ -380,7 +396,7 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_seed(LodDev L, int k) {
         for (unsigned long long t = lane; t < tot; t += 32) {
             const Cluster a = load_cluster(L.cl1 + kClF4 * ((size_t)x.z + i)),
                           b = load_cluster(cl2 + kClF4 * ((size_t)x.w + j));
-            const float z = widen<MODE>(cluster_gap(a, b), mg, a, b, oh).x;
+            const float z = widen<MODE>(cluster_gap(a, b), a, b).x;
             if (z < best) {
                 best = z;
                 bi = i;
@@ -397,11 +413,12 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_seed(LodDev L, int k) {
         for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(kFull, m, o));
         // every voxel pair's core distance is one of its upper bounds
         if (lane == 0 && !L.pown[p]) L.pcap[p] = core;
-        if (!(m < (MODE == kLast ? core + slack : core))) continue;
+        if (!(m < core + mg + slack)) continue;
         const int src = __ffs(__ballot_sync(kFull, best == m)) - 1;
         bi = __shfl_sync(kFull, bi, src);
         bj = __shfl_sync(kFull, bj, src);
         // each lane takes the nearer of its two triangle pairs by their centres
+        float4 along = make_float4(0.f, 0.f, 0.f, 0.f);
         const unsigned ia = bi * kCl + (lane & 7);
         const unsigned b0 = bj * kCl + (lane >> 3), b1 = b0 + 4;
         if (ia < it.a_cnt && b0 < it.b_cnt) {
@@ -413,7 +430,9 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_seed(LodDev L, int k) {
                         uz = tb0[0].z + tb0[1].z + tb0[2].z - az;
             const float vx2 = tb1[0].x + tb1[1].x + tb1[2].x - ax, vy = tb1[0].y + tb1[1].y + tb1[2].y - ay,
                         vz = tb1[0].z + tb1[1].z + tb1[2].z - az;
-            const float4* tb = vx2 * vx2 + vy * vy + vz * vz < ux * ux + uy * uy + uz * uz ? tb1 : tb0;
+            const bool second = vx2 * vx2 + vy * vy + vz * vz < ux * ux + uy * uy + uz * uz;
+            const float4* tb = second ? tb1 : tb0;
+            along = second ? make_float4(vx2, vy, vz, 0.f) : make_float4(ux, uy, uz, 0.f);
             const float4 o4 = L.tri1[k][(size_t)it.a_off * kTriF4];
             PreTri<float> A, B;
             float pa, ha, pb, hb;
@@ -425,6 +444,7 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_seed(LodDev L, int k) {
             best = FLT_MAX;
         }
         const float up = __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(best >= 0.f ? best : FLT_MAX)));
+        if (up < FLT_MAX && lane == __ffs(__ballot_sync(kFull, best == up)) - 1) L.dir[p] = along;
         if (lane == 0) {
             if (MODE == kLast) L.pd[p] = up;
             else if (!L.pown[p]) L.pcap[p] = fminf(core, up);
@@ -433,146 +453,225 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_seed(LodDev L, int k) {
     }
 }
 
+// One side's share of a pair's two bounds (the pair's are the sums of two).
+struct TriSide {
+    float z, y;
+};
+
 // ---------------------------------------------------------------- cull
 constexpr int kCullWarps = 8;
-constexpr int kCullBuf = 96;  // tasks a warp collects before it claims queue slots (>= 64 + 32)
+constexpr int kCullBuf = 96;  // tasks a warp collects before it claims queue slots (>= 63 + 32)
+constexpr int kSide = 16;     // clusters of one side that are looked at together
 
 // Queue `cnt` of the warp's collected tasks.  Items whose tasks find the
 // queue full go to the list of items that are evaluated whole, once each.
 __device__ __forceinline__ void flush_tasks(const LodDev& L, unsigned* ctr, const LodTask* buf, int cnt, int lane) {
-    int* done = reinterpret_cast<int*>(&L.mg[0].w);
+    __syncwarp();
     unsigned base = 0;
     if (lane == 0) base = atomicAdd(ctr + cTasks, (unsigned)cnt);
     base = __shfl_sync(kFull, base, 0);
     for (int i = lane; i < cnt; i += 32) {
         const LodTask t = buf[i];
         if (base + i < L.task_cap) L.tasks[base + i] = t;
-        else if (atomicExch(done + 4 * (size_t)t.w, 1) == 0) L.over[atomicAdd(ctr + cOver, 1u)] = t.w;
+        else if (atomicExch((int*)&L.mg[t.w].w, 1) == 0) L.over[atomicAdd(ctr + cOver, 1u)] = t.w;
     }
+    __syncwarp();
 }
 
-// One warp per item, lanes over (A, B) cluster pairs: a lane keeps its B
-// cluster and steps through the A clusters of its group.
+// An item as the cull reads it: the pair's direction, where projections on it
+// start (the item's origin), the thresholds on the scale of a widened gap.
+struct alignas(16) CullItem {
+    float ux, uy, uz, ox;
+    float oy, oz, zt, yt;
+    uint32_t ca, cb, n, w;  // first clusters, cluster counts (A | B << 16), item
+};
+
+// What a cluster adds to a pair's two bounds along direction u: A clusters
+// reach up to their largest projection, B clusters down to their smallest.
+template <int MODE>
+__device__ __forceinline__ TriSide cluster_side(const Cluster& c, const CullItem& T, bool isA) {
+    const float x = c.s.x - T.ox, y = c.s.y - T.oy, z = c.s.z - T.oz;
+    const float pr = x * T.ux + y * T.uy + z * T.uz;
+    const float cu = c.n.x * T.ux + c.n.y * T.uy + c.n.z * T.uz;
+    const float reach = c.s.w * sqrt_up(1.000002f - cu * cu) + c.n.w * fabsf(cu);
+    const float g = (isA ? -pr : pr) - reach;
+    return MODE == kTriH ? TriSide{g + c.h, g - c.ph} : TriSide{g, g};
+}
+
+// the smaller of two shares; NaN wins, so that what cannot be bounded goes on
+__device__ __forceinline__ float least_of(float a, float b) { return b < a || b != b ? b : a; }
+
+// Batches of up to 32 items per warp, in three steps:
+// 1. one item a lane: margins, thresholds, what the update reads of the item;
+// 2. side by side (4, 8 or 16 lanes a side, so 4, 2 or 1 items at a time) every
+//    cluster's share of the bounds along the pair's direction: an item ends
+//    here when the least shares of both sides together do not matter, and of
+//    the others only the clusters that do with the other side's least go on
+//    (voxels of more than 16 clusters skip this);
+// 3. those in pairs, one a lane, along the line of their own centres.
+// One item a warp and every cluster pair of it took twice as long (10-NN
+// self-join of 3,000 nuclei, five LODs: 1.95 -> 1.11 ms): each item waited for
+// its own chain of loads.  Going on to the triangles in this kernel (each
+// loaded once per item) was faster by a fifth where items keep 15 cluster
+// pairs and slower everywhere else, most where a LOD has few items.
 template <int MODE>
 __global__ void __launch_bounds__(kCullWarps * 32) k_lod_cull(LodDev L, int k, int pass, const unsigned* n_items,
-                                                              int stamp) {
+                                                                int stamp) {
     __shared__ LodTask bufs[kCullWarps][kCullBuf];
+    __shared__ CullItem recs[kCullWarps][32];
+    __shared__ uint8_t lists[kCullWarps][4][2][kSide];  // clusters that go on, per item of a step and side
     const JoinDev& d = L.d;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     LodTask* buf = bufs[wid];
+    CullItem* rec = recs[wid];
     int bn = 0;
     unsigned* ctr = L.ctr + pass * kLodCtrWords;
     const unsigned n = *n_items;
-    const unsigned nw = gridDim.x * kCullWarps;
+    const unsigned nw = gridDim.x * kCullWarps, gw = blockIdx.x * kCullWarps + wid;
+    const unsigned batch = max(1u, min(32u, (n + nw - 1) / nw));
     const float4* cl2 = L.self ? L.cl1 : L.cl2;
-    for (unsigned w = blockIdx.x * kCullWarps + wid; w < n; w += nw) {
-        const RefineItem it = L.items[w];
-        const int4 x = L.ext[w];
-        const int2 vx = L.vox[w];
-        float rmax, mg, slack, preset;
-        item_margins<MODE>(L, it, x, vx, k, rmax, mg, slack, preset);
-        const float3 oh = MODE == kObjH ? object_h(L, x.y, k) : make_float3(0.f, 0.f, 0.f);
-        const float2 th = thresholds<MODE>(L, x.x, x.y, slack, preset);
-        const unsigned nA = (it.a_cnt + kCl - 1) / kCl, nB = (it.b_cnt + kCl - 1) / kCl;
-        if (lane == 0) L.mg[w] = make_float4(mg, slack, preset, __int_as_float(0));
-        __syncwarp();
-        int lg = 0;  // lanes of a group: the power of two that holds nB, up to 32
-        while ((1u << lg) < nB && lg < 5) ++lg;
-        const unsigned g = 1u << lg, ng = 32u >> lg;
-        float zmin = INFINITY;
-        if (nA > 0xffffu || nB > 0xffffu) {  // indices do not fit a task
-            if (lane == 0 && atomicExch((int*)&L.mg[w].w, 1) == 0) L.over[atomicAdd(ctr + cOver, 1u)] = w;
-        } else {
-            for (unsigned j0 = 0; j0 < nB; j0 += g) {
-                const unsigned j = j0 + (lane & (g - 1));
-                const bool jv = j < nB;
-                const Cluster b = load_cluster(cl2 + kClF4 * ((size_t)x.w + (jv ? j : nB - 1)));
-                for (unsigned i0 = 0; i0 < nA; i0 += ng) {
-                    const unsigned i = i0 + (lane >> lg);
-                    const bool ok = jv && i < nA;
-                    const Cluster a = load_cluster(L.cl1 + kClF4 * ((size_t)x.z + (ok ? i : 0)));
-                    const float2 zy = widen<MODE>(cluster_gap(a, b), mg, a, b, oh);
-                    zmin = fminf(zmin, zy.x);
-                    const bool keep = ok && matters(zy, th);
-                    const unsigned m = __ballot_sync(kFull, keep);
-                    if (!m) continue;
-                    if (keep) buf[bn + __popc(m & lt)] = LodTask{w, (i << 16) | j, zy.x, zy.y};
-                    bn += __popc(m);
-                    if (bn >= 64) {
-                        __syncwarp();
-                        flush_tasks(L, ctr, buf, bn, lane);
-                        __syncwarp();
-                        bn = 0;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) zmin = fminf(zmin, __shfl_xor_sync(kFull, zmin, o));
-        if (lane == 0) {
-            const float e = err_bound(rmax);
+    for (unsigned w0 = gw * batch; w0 < n; w0 += nw * batch) {
+        const unsigned cnt = min(batch, n - w0);
+        unsigned most = 0;
+        if (lane < cnt) {
+            const unsigned w = w0 + lane;
+            const RefineItem it = L.items[w];
+            const int4 x = L.ext[w];
+            const int2 vx = L.vox[w];
+            float rmax, mg, slack, preset;
+            item_margins<MODE>(L, it, x, vx, k, rmax, mg, slack, preset);
+            const float2 th = thresholds<MODE>(L, x.x, x.y, slack, preset);
+            const float4 o4 = L.tri1[k][(size_t)it.a_off * kTriF4];
+            const float4 u = __ldcg(L.dir + x.y);
+            const float u2 = u.x * u.x + u.y * u.y + u.z * u.z;
+            const float inv = u2 > 1e-30f && u2 < 1e30f ? rsqrtf(u2) : 0.f;
+            const unsigned nA = (it.a_cnt + kCl - 1) / kCl, nB = (it.b_cnt + kCl - 1) / kCl;
+            const float2 lim = gap_limits<MODE>(L, k, x.y, th, mg);
+            const bool big = nA > 0xffffu || nB > 0xffffu;  // indices do not fit a task
+            rec[lane] = CullItem{u.x * inv, u.y * inv, u.z * inv, o4.x, o4.y, o4.z, lim.x, lim.y,
+                                 (unsigned)x.z, (unsigned)x.w, big ? 0u : nA | (nB << 16), w};
+            most = big ? 0u : max(nA, nB);
+            L.mg[w] = make_float4(mg, slack, preset, __int_as_float(big ? 1 : 0));
+            if (big) L.over[atomicAdd(ctr + cOver, 1u)] = w;
             const int v = x.x;
+            const float e = err_bound(rmax);
             d.vupd[v] = stamp;
             if (MODE == kLast) {
                 L.vres[v] = FLT_MAX;
                 d.vmx[v] = e;  // read by the update, which then sets both bounds
             } else {
                 if (MODE == kObjH) L.vres[v] = FLT_MAX;
-                float mx;
-                if (L.pown[x.y]) mx = __ldcg(d.vmx + v);
-                else {
-                    // The voxel pair's own upper bound enters only its error
-                    // term (4 u of it): its least possible value stands in.
-                    mx = fminf(d.vmx[v], fmaxf(zmin, __ldcg(L.pcap + x.y)));
-                    d.vmx[v] = mx;
-                }
-                d.verr[v] = fmaxf(d.verr[v], e + 4.f * kUnitRoundoff * fmaxf(fabsf(d.vmn[v]), fabsf(mx)));
+                // The voxel pair's own upper bound enters only its error term
+                // (4 u of it); where it is not kept, the middle between the
+                // least it can be and its core distance stands in.
+                const float mn = d.vmn[v], core = __ldcg(d.vmx + v);
+                const float mx = L.pown[x.y] ? core : 0.5f * (core + fminf(core, fmaxf(mn, th.x)));
+                d.verr[v] = fmaxf(d.verr[v], e + 4.f * kUnitRoundoff * fmaxf(fabsf(mn), fabsf(mx)));
             }
         }
-    }
-    if (bn > 0) {
+        most = __reduce_max_sync(kFull, most);
+        const int lg = most <= 4 ? 2 : most <= 8 ? 3 : 4;  // lanes a side
+        const int g = 1 << lg, per = kSide >> lg;          // items a step
         __syncwarp();
-        flush_tasks(L, ctr, buf, bn, lane);
+        for (unsigned s0 = 0; s0 < cnt; s0 += per) {
+            const int slot = lane >> (lg + 1);
+            const bool isA = !((lane >> lg) & 1);
+            const int idx = lane & (g - 1);
+            const bool live = s0 + slot < cnt;
+            const CullItem& T = rec[live ? s0 + slot : s0];
+            const unsigned nA = T.n & 0xffffu, nB = T.n >> 16;
+            const unsigned cn = live ? (isA ? nA : nB) : 0u;
+            const bool wide = live && max(nA, nB) > (unsigned)kSide;
+            TriSide s{INFINITY, INFINITY};
+            if ((unsigned)idx < cn)
+                s = cluster_side<MODE>(load_cluster((isA ? L.cl1 + kClF4 * (size_t)T.ca : cl2 + kClF4 * (size_t)T.cb) +
+                                                    kClF4 * (size_t)idx), T, isA);
+            TriSide least = s;
+#pragma unroll
+            for (int o = 1; o < kSide; o <<= 1) {
+                if (o < g) {
+                    least.z = least_of(least.z, __shfl_xor_sync(kFull, least.z, o));
+                    if (MODE != kLast) least.y = least_of(least.y, __shfl_xor_sync(kFull, least.y, o));
+                }
+            }
+            const float oz = __shfl_xor_sync(kFull, least.z, g);
+            const float oy = MODE == kLast ? 0.f : __shfl_xor_sync(kFull, least.y, g);
+            const bool item_on = wide || (live && cn > 0 && (!(least.z + oz >= T.zt) || (MODE != kLast && !(least.y + oy >= T.yt))));
+            const bool keep = item_on && (unsigned)idx < cn && (!(s.z + oz >= T.zt) || (MODE != kLast && !(s.y + oy >= T.yt)));
+            const unsigned on = __ballot_sync(kFull, item_on);
+            if (!on) continue;
+            const unsigned km = __ballot_sync(kFull, keep);
+            const unsigned sm = (km >> (lane & ~(g - 1))) & ((1u << g) - 1u);
+            if (keep) lists[wid][slot][isA ? 0 : 1][__popc(sm & ((1u << idx) - 1u))] = (uint8_t)idx;
+            __syncwarp();
+            for (int sl = 0; sl < per; ++sl) {
+                if (!((on >> (sl * 2 * g)) & 1u)) continue;
+                const CullItem I = rec[s0 + sl];
+                const unsigned iA = I.n & 0xffffu, iB = I.n >> 16;
+                const bool all = max(iA, iB) > (unsigned)kSide;
+                const unsigned rows = all ? iA : __popc((km >> (sl * 2 * g)) & ((1u << g) - 1u));
+                const unsigned cols = all ? iB : __popc((km >> (sl * 2 * g + g)) & ((1u << g) - 1u));
+                const unsigned total = rows * cols;
+                unsigned r = lane / max(cols, 1u), c = lane - r * max(cols, 1u);
+                for (unsigned t0 = 0; t0 < total; t0 += 32) {
+                    bool go = t0 + lane < total;
+                    LodTask t{I.w, 0, 0.f, 0.f};
+                    if (go) {
+                        const unsigned i = all ? r : lists[wid][sl][0][r], j = all ? c : lists[wid][sl][1][c];
+                        const Cluster a = load_cluster(L.cl1 + kClF4 * ((size_t)I.ca + i)),
+                                      b = load_cluster(cl2 + kClF4 * ((size_t)I.cb + j));
+                        const float2 zy = widen<MODE>(cluster_gap(a, b), a, b);
+                        t = LodTask{I.w, (i << 16) | j, zy.x, zy.y};
+                        go = !(t.z >= I.zt) || (MODE != kLast && !(t.y >= I.yt));
+                    }
+                    const unsigned m = __ballot_sync(kFull, go);
+                    if (go) buf[bn + __popc(m & lt)] = t;
+                    bn += __popc(m);
+                    if (bn >= 64) {
+                        flush_tasks(L, ctr, buf, bn, lane);
+                        bn = 0;
+                    }
+                    c += 32;
+                    while (c >= cols) {
+                        c -= cols;
+                        ++r;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        __syncwarp();
     }
+    if (bn > 0) flush_tasks(L, ctr, buf, bn, lane);
 }
 
 // ---------------------------------------------------------------- triangle tests
 // A cluster pair on a half warp: lanes 0-7 hold the A triangles, lanes 8-15
-// the B triangles, each its least contribution to the two bounds of a
-// triangle pair: A's largest and B's smallest projection on the line of the
-// two centres (taken relative to the A cluster's centre), with the triangle's
-// own Hausdorff values.  A pair's bound is the sum of its two sides.  Any
-// direction gives a lower bound of the distance; along this one it is off
-// only by the square of the angle to the closest points' direction.
+// the B triangles, each its share of the two bounds of a triangle pair: A's
+// largest and B's smallest projection on the line of the two centres (taken
+// relative to the A cluster's centre), with the triangle's own Hausdorff
+// values.  A pair's bound is the sum of its two sides.  Any direction gives a
+// lower bound of the distance; along this one it is off only by the square of
+// the angle to the closest points' direction.
 struct alignas(16) TaskDir {
     float ux, uy, uz, ax;
-    float ay, az, zt, yt;  // a pair matters when its z is below zt or its y below yt
-    uint32_t a0, b0, n, w; // first triangles, counts (A | B << 8), item
+    float ay, az, zt, yt;   // a pair matters when its z is below zt or its y below yt
+    uint32_t a0, b0, n, w;  // first triangles, counts (A | B << 8), item
 };
 
 template <int MODE>
-__device__ __forceinline__ TaskDir task_dir(const LodDev& L, int k, const float4* cl2, unsigned w, unsigned ci,
-                                            unsigned cj, float2 th, const int4& x, float mg) {
+__device__ __forceinline__ TaskDir task_dir(const LodDev& L, const float4* cl2, unsigned w, unsigned ci, unsigned cj,
+                                            float2 lim, const int4& x) {
     const RefineItem it = L.items[w];
     const float4 ca = L.cl1[kClF4 * ((size_t)x.z + ci)], cb = cl2[kClF4 * ((size_t)x.w + cj)];
     const float ux = cb.x - ca.x, uy = cb.y - ca.y, uz = cb.z - ca.z;
     const float u2 = ux * ux + uy * uy + uz * uz;
     const float inv = u2 > 0.f ? rsqrtf(u2) : 0.f;
-    float zt = th.x + mg, yt = th.y + mg;
-    if (MODE == kObjH) {
-        const float3 oh = object_h(L, x.y, k);
-        zt -= oh.x + oh.y;
-        yt += oh.z;
-    }
     const unsigned na = min(8u, it.a_cnt - ci * kCl), nb = min(8u, it.b_cnt - cj * kCl);
-    return TaskDir{ux * inv, uy * inv, uz * inv, ca.x, ca.y, ca.z, zt, yt,
+    return TaskDir{ux * inv, uy * inv, uz * inv, ca.x, ca.y, ca.z, lim.x, lim.y,
                    it.a_off + ci * kCl, it.b_off + cj * kCl, na | (nb << 8), w};
 }
-
-struct TriSide {
-    float z, y;
-};
 
 template <int MODE>
 __device__ __forceinline__ TriSide tri_side(const TaskDir& T, const float4* __restrict__ tri1,
@@ -591,7 +690,8 @@ __device__ __forceinline__ TriSide tri_side(const TaskDir& T, const float4* __re
 
 // the least sum over a half warp's (A, B) triangle pairs
 __device__ __forceinline__ float least_sum(float v) {
-    v = grp8_min(v);
+#pragma unroll
+    for (int o = 1; o < kCl; o <<= 1) v = least_of(v, __shfl_xor_sync(kFull, v, o));
     return v + __shfl_xor_sync(kFull, v, 8);
 }
 
@@ -600,8 +700,8 @@ constexpr int kTestBuf = 96;  // triangle pairs a warp collects before it claims
 
 template <int MODE>
 __global__ void __launch_bounds__(kTestWarps * 32, 5) k_lod_test(LodDev L, int k, int pass) {
-    __shared__ __align__(16) TaskDir dirs[kTestWarps][32];
-    __shared__ __align__(16) LodEval bufs[kTestWarps][kTestBuf];
+    __shared__ TaskDir dirs[kTestWarps][32];
+    __shared__ LodEval bufs[kTestWarps][kTestBuf];
     const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15, wid = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     TaskDir* dir = dirs[wid];
@@ -633,19 +733,18 @@ __global__ void __launch_bounds__(kTestWarps * 32, 5) k_lod_test(LodDev L, int k
         bool have = lane < batch && t0 + lane < n;
         LodTask t{0, 0, 0.f, 0.f};
         int4 x = make_int4(0, 0, 0, 0);
-        float2 th = make_float2(0.f, 0.f);
-        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 lim = make_float2(0.f, 0.f);
         if (have) {
             t = L.tasks[t0 + lane];
             x = L.ext[t.w];
-            g = L.mg[t.w];
-            th = thresholds<MODE>(L, x.x, x.y, g.y, g.z);
-            have = matters(make_float2(t.z, t.y), th);
+            const float4 g = L.mg[t.w];
+            lim = gap_limits<MODE>(L, k, x.y, thresholds<MODE>(L, x.x, x.y, g.y, g.z), g.x);
+            have = !(t.z >= lim.x) || (MODE != kLast && !(t.y >= lim.y));
         }
         const unsigned m = __ballot_sync(kFull, have);
         if (!m) continue;
         __syncwarp();
-        if (have) dir[__popc(m & lt)] = task_dir<MODE>(L, k, cl2, t.w, t.ij >> 16, t.ij & 0xffffu, th, x, g.x);
+        if (have) dir[__popc(m & lt)] = task_dir<MODE>(L, cl2, t.w, t.ij >> 16, t.ij & 0xffffu, lim, x);
         __syncwarp();
         const int cnt = __popc(m);
         for (int c = 0; c < cnt; c += 2) {
@@ -711,12 +810,7 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_eval(LodDev L, int k, int
                 if (e.z > -INFINITY) {  // the caps may have come down since its test
                     const int4 x = L.ext[e.w];
                     const float4 g = L.mg[e.w];
-                    float zt = thresholds<MODE>(L, x.x, x.y, g.y, g.z).x + g.x;
-                    if (MODE == kObjH) {
-                        const float3 oh = object_h(L, x.y, k);
-                        zt -= oh.x + oh.y;
-                    }
-                    have = !(e.z >= zt);
+                    have = !(e.z >= gap_limits<MODE>(L, k, x.y, thresholds<MODE>(L, x.x, x.y, g.y, g.z), g.x).x);
                 }
             }
             const unsigned km = __ballot_sync(kFull, have);
@@ -738,7 +832,7 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_eval(LodDev L, int k, int
             if (over_left) {
                 const int4 x = L.ext[ow];
                 const float4 g = L.mg[ow];
-                const float2 th = thresholds<MODE>(L, x.x, x.y, g.y, g.z);
+                const float2 lim = gap_limits<MODE>(L, k, x.y, thresholds<MODE>(L, x.x, x.y, g.y, g.z), g.x);
                 if (!todo) {
                     bool have = false;
                     if (opos + lane < otot) {
@@ -746,8 +840,8 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_eval(LodDev L, int k, int
                         const unsigned cj = (unsigned)((opos + lane) - (unsigned long long)ci * onB);
                         const Cluster a = load_cluster(L.cl1 + kClF4 * ((size_t)x.z + ci)),
                                       b = load_cluster(cl2 + kClF4 * ((size_t)x.w + cj));
-                        const float3 oh = MODE == kObjH ? object_h(L, x.y, k) : make_float3(0.f, 0.f, 0.f);
-                        have = matters(widen<MODE>(cluster_gap(a, b), g.x, a, b, oh), th);
+                        const float2 zy = widen<MODE>(cluster_gap(a, b), a, b);
+                        have = !(zy.x >= lim.x) || (MODE != kLast && !(zy.y >= lim.y));
                     }
                     todo = __ballot_sync(kFull, have);
                     obase = opos;
@@ -757,7 +851,7 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_eval(LodDev L, int k, int
                     const unsigned long long t = obase + (__ffs(todo) - 1);
                     todo &= todo - 1;
                     const unsigned ci = (unsigned)(t / onB), cj = (unsigned)(t - (unsigned long long)ci * onB);
-                    const TaskDir T = task_dir<MODE>(L, k, cl2, ow, ci, cj, th, x, g.x);
+                    const TaskDir T = task_dir<MODE>(L, cl2, ow, ci, cj, lim, x);
                     const TriSide s = tri_side<MODE>(T, tri1, tri2, lane & 15);
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
@@ -786,12 +880,15 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_eval(LodDev L, int k, int
                 pre_rel(tri2 + (size_t)e.z * kTriF4, o4, B, pb, hb);
                 const float dd = sqrtf(tri_dist2(A, B));
                 const int4 x = L.ext[e.x];
+                // a pair's new best also gives it its direction (racing writers may
+                // mix theirs: the reader normalises, and any direction is valid)
+                bool best = false;
                 if (MODE == kTriH) {
-                    lower_to(L.pown[x.y] ? d.vmx + x.x : L.pcap + x.y, dd + ha + hb);
+                    best = lower_to(L.pown[x.y] ? d.vmx + x.x : L.pcap + x.y, dd + ha + hb);
                     lower_to(d.vmn + x.x, fmaxf(dd - pa - pb, 0.f));
                 } else if (MODE == kObjH) {
                     const float3 o = object_h(L, x.y, k);
-                    lower_to(L.pown[x.y] ? d.vmx + x.x : L.pcap + x.y, dd + o.x + o.y);
+                    best = lower_to(L.pown[x.y] ? d.vmx + x.x : L.pcap + x.y, dd + o.x + o.y);
                     lower_to(L.vres + x.x, dd);
                 } else {
                     // what is not below the threshold does not count as found:
@@ -802,6 +899,7 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_eval(LodDev L, int k, int
                         lower_to(L.vres + x.x, dd);
                     }
                 }
+                if (best) L.dir[x.y] = tri_to_tri(A, B);
                 ++evals;
             }
             // up to 95 pairs: two moves to the front
@@ -951,7 +1049,7 @@ int blocks_for(int64_t n, int per_block, int cap) {
 
 template <int MODE>
 cudaError_t refine_pass(const LodDev& L, int k, int pass, const unsigned* n_items, int stamp, cudaStream_t s) {
-    k_lod_cull<MODE><<<blocks_for(L.d.V, kCullWarps, L.num_sms * 8), kCullWarps * 32, 0, s>>>(L, k, pass, n_items,
+    k_lod_cull<MODE><<<blocks_for(L.d.V, kCullWarps, L.num_sms * 4), kCullWarps * 32, 0, s>>>(L, k, pass, n_items,
                                                                                             stamp);
     k_lod_test<MODE><<<L.num_sms * 5, kTestWarps * 32, 0, s>>>(L, k, pass);
     k_lod_eval<MODE><<<L.num_sms * 4, kEvalBlock, 0, s>>>(L, k, pass);

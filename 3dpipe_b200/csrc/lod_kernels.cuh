@@ -13,16 +13,16 @@ namespace tdp {
 constexpr int kLodCtrWords = 8;   // counters of one pass over the items
 constexpr int kMaxPasses = 10;    // up to 8 LODs, the redo pass, one spare
 
-// A queued cluster pair of item w: z and y are its lower bounds of the
-// Hausdorff-widened upper and lower bound (less the item's FP32 margin), so
-// that a later look at the running caps can drop it without its clusters.
+// A queued cluster pair of item w: z and y are its gap widened for the upper
+// and the lower bound, so that a later look at the running caps can drop it
+// without its clusters.
 struct alignas(16) LodTask {
     uint32_t w, ij;
     float z, y;
 };
 
-// A queued triangle pair: item, triangles, lower bound (less the margin) of
-// its upper bound; -inf where its lower bound matters too.
+// A queued triangle pair: item, triangles, gap widened for the upper bound;
+// -inf where its lower bound matters too.
 struct alignas(16) LodEval {
     uint32_t w, a, b;
     float z;
@@ -51,6 +51,7 @@ struct LodDev {
     float* pd;     // per pair: the last LOD's running distance
     uint8_t* pown; // per pair: 1 = caps per voxel pair (vmx) instead of pcap
     uint8_t* pmiss;  // per pair: 1 = nothing of its last LOD came below its cap: done again without it
+    float4* dir;   // per pair: about the direction of its closest points (any vector, or 0)
     float* vres;   // per voxel pair: distance minimum (last LOD; levels 0 and 1)
     // cluster records of the voxels in use at the current LOD
     float4* cl1;
@@ -62,8 +63,7 @@ struct LodDev {
     int* list1;    // voxels whose records are built at this LOD
     int* list2;
     long nvox1, nvox2;
-    // cluster pairs that survive the cull
-    LodTask* tasks;
+    LodTask* tasks;  // cluster pairs that survive the cull
     unsigned task_cap;
     LodEval* evals;  // triangle pairs that survive their tests
     unsigned eval_cap;
@@ -78,7 +78,7 @@ struct LodDev {
 };
 
 cudaError_t launch_lod_items(const LodDev& L, int k, cudaStream_t s);
-// clusters, (first LOD) seeds, cull, evaluation of LOD k's items
+// clusters, (first LOD) seeds, cull, tests and evaluation of LOD k's items
 cudaError_t launch_lod_refine(const LodDev& L, int k, int highest, cudaStream_t s);
 // the pairs' bounds, evictions and the within decision; at the last LOD also
 // the items of the pairs that have to be done again without their caps

@@ -50,7 +50,7 @@ enum Slot {
     kQk = 82, kQtau,                  // per query object queries
     kPreset = 91,                     // the last LOD's item presets (within queries)
     kLodExt = 101, kLodVox, kLodMg, kLodCaps, kLodFlags, kLodZero, kLodVres, kLodCl1, kLodCl2, kLodVb1, kLodVb2,
-    kLodLists, kLodTasks, kLodOver, kLodEvals, kLodBest,   // the LOD loop's task form
+    kLodLists, kLodTasks, kLodOver, kLodEvals, kLodBest, kLodDir,   // the LOD loop's task form
 };
 
 template <typename T>
@@ -104,6 +104,7 @@ int enqueue_task_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captu
     CUL(cudaMemsetAsync(L.counter + 8, 0, 26 * sizeof(unsigned), s));
     CUL(cudaMemsetAsync(L.dstats, 0, 8, s));
     CUL(cudaMemsetAsync(L.t.pcap, 0x7f, L.caps_bytes, s));     // 3.4e38: above any bound
+    CUL(cudaMemsetAsync(L.t.dir, 0, L.best_bytes * 2, s));
     CUL(cudaMemsetAsync(L.t.pbest, 0xff, L.best_bytes, s));
     CUL(cudaMemsetAsync(L.t.flag1, 0xff, L.flags_bytes, s));
     CUL(cudaMemsetAsync(L.t.ctr, 0, L.zero_bytes, s));
@@ -542,10 +543,11 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             L.flags_bytes = (nv1 + nv2) * 4;
             L.zero_bytes = ctr_bytes + 2 * Pz;
             ENS(kLodExt, Vz * sizeof(int4)); ENS(kLodVox, Vz * sizeof(int2)); ENS(kLodMg, Vz * sizeof(float4));
-            ENS(kLodCaps, L.caps_bytes); ENS(kLodBest, L.best_bytes); ENS(kLodFlags, L.flags_bytes); ENS(kLodZero, L.zero_bytes);
+            ENS(kLodCaps, L.caps_bytes); ENS(kLodBest, L.best_bytes); ENS(kLodDir, 2 * L.best_bytes); ENS(kLodFlags, L.flags_bytes); ENS(kLodZero, L.zero_bytes);
             ENS(kLodVres, Vz * 4); ENS(kLodCl1, c1 * 3 * sizeof(float4)); ENS(kLodVb1, nv1 * 2 * sizeof(float4));
             if (!self) { ENS(kLodCl2, c2 * 3 * sizeof(float4)); ENS(kLodVb2, nv2 * 2 * sizeof(float4)); }
-            ENS(kLodLists, (nv1 + nv2) * 4); ENS(kLodTasks, (size_t)t.task_cap * sizeof(LodTask)); ENS(kLodOver, Vz * 4);
+            ENS(kLodLists, (nv1 + nv2) * 4); ENS(kLodOver, Vz * 4);
+            ENS(kLodTasks, (size_t)t.task_cap * sizeof(LodTask));
             ENS(kLodEvals, (size_t)t.eval_cap * sizeof(LodEval));
             t.d = d;
             t.box1 = t1->d_boxes; t.box2 = t2->d_boxes;
@@ -555,6 +557,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             }
             t.items = items; t.ext = buf<int4>(ctx, kLodExt); t.vox = buf<int2>(ctx, kLodVox); t.mg = buf<float4>(ctx, kLodMg);
             t.pbest = buf<unsigned long long>(ctx, kLodBest); t.evals = buf<LodEval>(ctx, kLodEvals);
+            t.dir = buf<float4>(ctx, kLodDir);
             t.pcap = buf<float>(ctx, kLodCaps); t.pd = t.pcap + Pz;
             t.ctr = buf<unsigned>(ctx, kLodZero);
             t.pown = (uint8_t*)t.ctr + ctr_bytes; t.pmiss = t.pown + Pz;
@@ -564,7 +567,8 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             t.flag1 = buf<int>(ctx, kLodFlags); t.flag2 = self ? t.flag1 : t.flag1 + nv1;
             t.list1 = buf<int>(ctx, kLodLists); t.list2 = self ? t.list1 : t.list1 + nv1;
             t.nvox1 = (long)nv1; t.nvox2 = (long)nv2;
-            t.tasks = buf<LodTask>(ctx, kLodTasks); t.over = buf<unsigned>(ctx, kLodOver);
+            t.tasks = buf<LodTask>(ctx, kLodTasks);
+            t.over = buf<unsigned>(ctx, kLodOver);
             t.n_items = ctx->d_counter + 24;
             t.tri_pairs = (unsigned long long*)(ctx->d_counter + 10);
             t.n_full = ctx->d_stats;
