@@ -62,9 +62,10 @@ struct JoinDev {
     unsigned long long* stat_vp;  // voxel pairs evaluated by the filter (statistic)
 };
 
-// filter: per object pair, min box gap and min core distance over all voxel pairs
-cudaError_t launch_pair_bounds(const JoinDev& d, cudaStream_t s);
-// within: classify pairs at the filter (min > tau drop, max <= tau report)
+// filter: per object pair, min box gap and min core distance over all voxel
+// pairs; decide != 0 also classifies within pairs (as launch_within_decide)
+cudaError_t launch_pair_bounds(const JoinDev& d, cudaStream_t s, int decide, float tau, int tuned);
+// within: classify undecided pairs (min > tau drop, max <= tau report)
 cudaError_t launch_within_decide(const JoinDev& d, float tau, int tuned, cudaStream_t s);
 // kNN: the bulk rank rule per query object, then the confirm cap at K
 cudaError_t launch_knn_rank(const JoinDev& d, int K, int tuned, int* scratch_status, cudaStream_t s);

@@ -409,10 +409,8 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     long launches = 0;
 
     // ---- 2. filter ----
-    CU(launch_pair_bounds(d, s)); ++launches;
-    if (any_knn) { CU(launch_knn_rank(d, prm->knn, tuned, buf<int>(ctx, kRankSt), s)); }
-    if (any_within) { CU(launch_within_decide(d, within_dist, tuned, s)); }
-    ++launches;
+    CU(launch_pair_bounds(d, s, any_within, within_dist, tuned)); ++launches;
+    if (any_knn) { CU(launch_knn_rank(d, prm->knn, tuned, buf<int>(ctx, kRankSt), s)); ++launches; }
     int64_t* cnt = buf<int64_t>(ctx, kCnt);
     CU(cudaMemsetAsync(cnt + P, 0, 8, s));
     CU(launch_count_vps(d, !knn, within_dist, tuned, cnt, s)); ++launches;
