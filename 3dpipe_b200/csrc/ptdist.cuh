@@ -74,6 +74,40 @@ __host__ __device__ inline double tri2(D3 p, D3 a, D3 b, D3 c) {
     return dist2(p, D3{a.x + ab.x * v + ac.x * w, a.y + ab.y * v + ac.y * w, a.z + ab.z * v + ac.z * w});
 }
 
+#ifdef __CUDACC__
+// tri2 with the same values on the device: the region picks the operands of one
+// division (two inside the triangle) instead of a branch with its own, so that
+// lanes in different regions run one instruction stream and the code stays
+// small.  Adding the zero products changes no coordinate.
+__device__ __noinline__ double tri2_degenerate(D3 p, D3 a, D3 b, D3 c) {
+    return dmin(seg2(p, a, b), dmin(seg2(p, b, c), seg2(p, c, a)));
+}
+__device__ inline double tri2_dev(D3 p, D3 a, D3 b, D3 c) {
+    const D3 ab = sub(b, a), ac = sub(c, a), ap = sub(p, a), bp = sub(p, b), cp = sub(p, c);
+    const double d1 = dot(ab, ap), d2 = dot(ac, ap), d3 = dot(ab, bp), d4 = dot(ac, bp), d5 = dot(ab, cp), d6 = dot(ac, cp);
+    const double vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
+    const double e = d4 - d3, f = d5 - d6;
+    const bool at_a = d1 <= 0 && d2 <= 0;
+    const bool at_b = !at_a && d3 >= 0 && d4 <= d3;
+    const bool on_ab = !at_a && !at_b && vc <= 0 && d1 >= 0 && d3 <= 0;
+    const bool at_c = !at_a && !at_b && !on_ab && d6 >= 0 && d5 <= d6;
+    const bool r4 = !at_a && !at_b && !on_ab && !at_c;
+    const bool on_ac = r4 && vb <= 0 && d2 >= 0 && d6 <= 0;
+    const bool on_bc = r4 && !on_ac && va <= 0 && e >= 0 && f >= 0;
+    const bool inside = r4 && !on_ac && !on_bc;
+    const double s = va + vb + vc;
+    if (inside && !(s > 0)) return tri2_degenerate(p, a, b, c);
+    const double num = on_ab ? d1 : on_ac ? d2 : on_bc ? e : vb;
+    const double den = on_ab ? d1 - d3 : on_ac ? d2 - d6 : on_bc ? e + f : s;
+    const bool vertex = at_a || at_b || at_c;
+    const double t = !vertex && den > 0 ? num / den : 0.0;
+    const double w = inside ? vc / s : 0.0;
+    const D3 o = at_b || on_bc ? b : at_c ? c : a;
+    const D3 u = on_ac ? ac : on_bc ? sub(c, b) : ab;
+    return dist2(p, D3{o.x + u.x * t + ac.x * w, o.y + u.y * t + ac.y * w, o.z + u.z * t + ac.z * w});
+}
+#endif
+
 // distance from q to the box [lo, hi] (0 inside; +inf for an empty box lo > hi)
 __host__ __device__ inline double box_gap(D3 q, float4 lo, float4 hi) {
     const double gx = dmax(dmax((double)lo.x - q.x, q.x - (double)hi.x), 0.0);
