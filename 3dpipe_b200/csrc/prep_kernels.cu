@@ -30,13 +30,21 @@
 //     assigned the same way to the voxels kept, triangles keeping LOD order.
 //  4. Transform = the vertex nearest the centre of the float bounding box.
 // Ties go to the lowest index everywhere.  Work layout: one CTA per object.
-// Decimation keeps the object's facets (16- or 32-bit vertex ids), flags and
-// four vertex bitmasks in shared memory (global memory for objects too large
-// for it); each thread owns the facets tid + k T, caches the smallest key of
-// its own candidate edges and recomputes it only after one of its facets
-// changed; a round is a block argmin, one scan of the facets around the edge
-// (links, neighbour masks, normals) and one applying scan.  This file is built
-// with -fmad=false: every product and sum is rounded on its own, as on the host.
+// Decimation keeps the object's facets (16- or 32-bit vertex ids), flags, four
+// vertex bitmasks and the smallest key of every 32 facets in shared memory
+// (global memory for objects too large for it), every facet's smallest key and
+// every vertex's facets in global memory.  Collapses only ever join two
+// vertices' facets, so a vertex's live facets are those of the vertices merged
+// into it, a chain of the first lists.  A round is a block argmin over the
+// groups of 32, the facets around the edge (a warp for each end: links,
+// neighbour masks, normals), those around the two third vertices, the change
+// itself, and the groups that it touched; it costs what the neighbourhood
+// costs, not the mesh.  The rounds of one object are a serial chain of FP64
+// and memory latencies, which bounds it: vessels of 20,160 facets and 8,068
+// rounds took 23.7 us a round with three scans over all facets, 4.2 here (6
+// vessels 191 -> 34 ms, 1,000 nuclei of 1,280 facets 7.7 -> 4.6 ms).  This file
+// is built with -fmad=false: every product and sum is rounded on its own, as on
+// the host.
 #include <cuda_runtime.h>
 
 #include <cub/device/device_scan.cuh>
@@ -59,7 +67,7 @@ namespace {
 constexpr int kDecLods = kNumLods - 1;  // LODs made by decimation (20..80)
 constexpr int kPrepThreads = 256;       // voxel and writer kernels
 constexpr size_t kSmemSmall = 40 << 10;  // decimation in shared memory, 128 threads
-constexpr size_t kSmemLarge = 200 << 10; // decimation in shared memory, 1024 threads
+constexpr size_t kSmemLarge = 220 << 10; // decimation in shared memory, 256 threads
 
 struct Meshes {  // one batch on the device; object o: vertices V[3 voff[o]..), facets F[3 foff[o]..)
     const float* V;
@@ -100,16 +108,10 @@ __device__ __forceinline__ double3 cross3(double3 a, double3 b) {
     return make_double3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
 
-__device__ __forceinline__ bool key_less(double l1, uint32_t a1, uint32_t b1, double l2, uint32_t a2, uint32_t b2) {
-    if (l1 != l2) return l1 < l2;
-    if (a1 != a2) return a1 < a2;
-    return b1 < b2;
-}
-
-// true when replacing u by v turns facet (x, y, z) (which holds u, not v)
-__device__ bool turns(const float* P, uint32_t x, uint32_t y, uint32_t z, uint32_t u, uint32_t v) {
-    const double3 p0 = vtx(P, x), p1 = vtx(P, y), p2 = vtx(P, z);
-    const double3 q0 = vtx(P, x == u ? v : x), q1 = vtx(P, y == u ? v : y), q2 = vtx(P, z == u ? v : z);
+// true when moving corner u of facet (x, y, z) (corners p0, p1, p2) to point q turns it
+__device__ bool turns(uint32_t x, uint32_t y, double3 p0, double3 p1, double3 p2, uint32_t u, double3 q) {
+    const bool at0 = x == u, at1 = !at0 && y == u;
+    const double3 q0 = at0 ? q : p0, q1 = at1 ? q : p1, q2 = at0 || at1 ? p2 : q;
     const double3 n0 = cross3(sub3(p1, p0), sub3(p2, p0)), n1 = cross3(sub3(q1, q0), sub3(q2, q0));
     const double a0 = sqrt(dot3(n0, n0)), a1 = sqrt(dot3(n1, n1));
     return a1 < 1e-12 * (a0 + 1e-300) || dot3(n0, n1) < 0.3 * a0 * a1;
@@ -121,25 +123,66 @@ __device__ __forceinline__ void mark(uint32_t* M, uint32_t x, uint32_t y, uint32
     if (z != c) atomicOr(M + (z >> 5), 1u << (z & 31));
 }
 
-// smallest key (|P_a - P_b|^2, a, b) over the candidate slots of facet f with
-// flags fla, folded into (bl, ba, bb, bf)
-template <typename VI>
-__device__ __forceinline__ void fold_facet(const float* P, const VI* fv, uint32_t f, uint32_t fla, double& bl,
-                                           uint32_t& ba, uint32_t& bb, uint32_t& bf) {
+// An edge's key: the bits of |P_a - P_b|^2 (lengths are not negative, so the
+// bits order like the values, without the latency of FP64 compares), then
+// a << 32 | b (a < b).
+struct alignas(16) Key {
+    uint64_t l, ab;
+};
+constexpr uint64_t kNoLength = 0x7ff0000000000000ull;  // +inf: no candidate
+__device__ __forceinline__ bool key_less(const Key& x, const Key& y) { return x.l != y.l ? x.l < y.l : x.ab < y.ab; }
+__device__ __forceinline__ Key no_key() { return Key{kNoLength, ~0ull}; }
+// the warp's least key: a word at a time among the lanes that still tie
+__device__ __forceinline__ Key warp_least(Key k) {
+    const uint32_t word[4] = {(uint32_t)(k.l >> 32), (uint32_t)k.l, (uint32_t)(k.ab >> 32), (uint32_t)k.ab};
+    unsigned tie = 0xffffffffu;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        if (fla & (2u << j)) continue;
-        const uint32_t x = fv[3 * f + j], y = fv[3 * f + (j == 2 ? 0 : j + 1)];
-        const uint32_t a = min(x, y), b = max(x, y);
-        const double L = dist2(vtx(P, a), vtx(P, b));
-        if (key_less(L, a, b, bl, ba, bb)) { bl = L; ba = a; bb = b; bf = f; }
+    for (int w = 0; w < 4; ++w) {
+        const bool in = (tie >> (threadIdx.x & 31)) & 1u;
+        const uint32_t least = __reduce_min_sync(0xffffffffu, in ? word[w] : UINT_MAX);
+        tie = __ballot_sync(0xffffffffu, in && word[w] == least);
+        if (!(tie & (tie - 1))) break;
     }
+    const int src = __ffs(tie) - 1;
+    return Key{__shfl_sync(0xffffffffu, k.l, src), __shfl_sync(0xffffffffu, k.ab, src)};
 }
 
-// bytes of decimation storage for an object (facets, flags, 4 masks)
-__host__ __device__ inline size_t dec_bytes(int64_t n, int64_t m, size_t vi) {
-    return round16(3 * (size_t)m * vi) + round16((size_t)m) + 16 * (size_t)((n + 31) / 32);
+// smallest key over the candidate edges of facet (x, y, z) with corners p, q, r
+// and flags fla
+__device__ __forceinline__ Key facet_key(double3 p, double3 q, double3 r, uint32_t x, uint32_t y, uint32_t z,
+                                         uint32_t fla) {
+    const uint32_t t[3] = {x, y, z};
+    const double len[3] = {dist2(p, q), dist2(q, r), dist2(r, p)};
+    Key k = no_key();
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const uint32_t c = t[j], d = t[j == 2 ? 0 : j + 1];
+        const Key e{(uint64_t)__double_as_longlong(len[j]), (uint64_t)min(c, d) << 32 | max(c, d)};
+        if (!(fla & (2u << j)) && key_less(e, k)) k = e;
+    }
+    return k;
 }
+
+constexpr int kGroup = 32;     // facets whose smallest key is kept
+constexpr int kTouched = 128;  // touched groups listed a round (more: all are redone)
+
+// bytes of an object's own storage: facets, flags, 4 masks, merge chains, group
+// keys
+__host__ __device__ inline size_t dec_bytes(int64_t n, int64_t m, size_t vi) {
+    const size_t g = ((size_t)m + kGroup - 1) / kGroup;
+    return round16(3 * (size_t)m * vi) + round16((size_t)m) + round16(16 * (size_t)((n + 31) / 32)) +
+           2 * round16((size_t)n * vi) + sizeof(Key) * g;
+}
+
+// Per batch in global memory: every facet's smallest key, every vertex's facets
+// as the mesh has them (csr[start[v] .. start[v + 1]), start with one entry more
+// per object), fill cursors.
+struct DecLists {
+    Key* keys;
+    uint32_t* csr;
+    uint32_t* start;
+    uint32_t* cur;
+};
 
 // ------------------------------------------------------------------ validation
 // first object (lowest index) without vertices or facets, with a vertex index
@@ -155,205 +198,6 @@ __global__ void k_validate(Meshes M, int* first_bad) {
         }
         for (int64_t i = 3 * v0 + threadIdx.x; !bad && i < 3 * v1; i += blockDim.x) bad = !isfinite(M.V[i]);
         if (__syncthreads_or(bad) && threadIdx.x == 0) atomicMin(first_bad, o);
-    }
-}
-
-// ------------------------------------------------------------------ decimation
-template <typename VI, int T>
-__global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict__ objs, int n_objs, uint8_t* gstore,
-                                                const int64_t* __restrict__ gstore_off, uint32_t* __restrict__ lodF,
-                                                int64_t Ftot, uint32_t* __restrict__ lodCnt) {
-    constexpr int NW = T / 32;
-    extern __shared__ __align__(16) uint8_t dsm[];
-    __shared__ double s_len[NW];
-    __shared__ uint32_t s_a[NW], s_b[NW], s_red[3][NW], s_third[2];
-    __shared__ int s_nsh, s_fuv, s_fvu, s_alive;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int i = blockIdx.x; i < n_objs; i += gridDim.x) {
-        const int o = objs[i];
-        const int64_t v0 = M.voff[o], f0 = M.foff[o];
-        const uint32_t n = (uint32_t)(M.voff[o + 1] - v0), m = (uint32_t)(M.foff[o + 1] - f0);
-        const float* P = M.V + 3 * v0;
-        uint8_t* base = gstore ? gstore + gstore_off[i] : dsm;
-        VI* fv = reinterpret_cast<VI*>(base);
-        uint8_t* fl = base + round16(3 * (size_t)m * sizeof(VI));
-        uint32_t* Mu = reinterpret_cast<uint32_t*>(fl + round16(m));
-        const uint32_t W = (n + 31) / 32;
-        uint32_t *Mv = Mu + W, *M1 = Mu + 2 * W, *M2 = Mu + 3 * W;
-        for (uint32_t f = tid; f < m; f += T) {
-            for (int k = 0; k < 3; ++k) fv[3 * f + k] = (VI)M.F[3 * (f0 + f) + k];
-            fl[f] = 1;  // bit 0 live, bit 1 + j: edge (j, j + 1) refused
-        }
-        for (uint32_t w = tid; w < 4 * W; w += T) Mu[w] = 0;
-        if (tid == 0) s_alive = (int)m;
-        __syncthreads();
-        // this thread's smallest candidate key and the facet holding it; a full
-        // rescan (dirty) is needed only when that facet changes, any other
-        // changed facet is folded in
-        bool dirty = true;
-        double bl = INFINITY;
-        uint32_t ba = UINT_MAX, bb = UINT_MAX, bf = UINT_MAX;
-        int li = kDecLods - 1;
-        while (li >= 0) {
-            const uint32_t target = (uint32_t)((uint64_t)m * (uint64_t)(20 * (li + 1)) / 100);  // LOD 20 (li + 1)
-            bool snap = (uint32_t)s_alive <= target;
-            uint32_t u = 0, v = 0;
-            if (!snap) {
-                if (dirty) {  // smallest key among this thread's candidate edges
-                    bl = INFINITY;
-                    ba = bb = bf = UINT_MAX;
-                    for (uint32_t f = tid; f < m; f += T) {
-                        const uint32_t fla = fl[f];
-                        if (fla & 1) fold_facet(P, fv, f, fla, bl, ba, bb, bf);
-                    }
-                    dirty = false;
-                }
-                double L = bl;
-                uint32_t A = ba, B = bb;
-#pragma unroll
-                for (int s = 16; s > 0; s >>= 1) {
-                    const double L2 = __shfl_xor_sync(0xffffffffu, L, s);
-                    const uint32_t A2 = __shfl_xor_sync(0xffffffffu, A, s), B2 = __shfl_xor_sync(0xffffffffu, B, s);
-                    if (key_less(L2, A2, B2, L, A, B)) { L = L2; A = A2; B = B2; }
-                }
-                if (lane == 0) { s_len[wid] = L; s_a[wid] = A; s_b[wid] = B; }
-                __syncthreads();
-                if (wid == 0) {
-                    L = lane < NW ? s_len[lane] : INFINITY;
-                    A = lane < NW ? s_a[lane] : UINT_MAX;
-                    B = lane < NW ? s_b[lane] : UINT_MAX;
-#pragma unroll
-                    for (int s = 16; s > 0; s >>= 1) {
-                        const double L2 = __shfl_xor_sync(0xffffffffu, L, s);
-                        const uint32_t A2 = __shfl_xor_sync(0xffffffffu, A, s), B2 = __shfl_xor_sync(0xffffffffu, B, s);
-                        if (key_less(L2, A2, B2, L, A, B)) { L = L2; A = A2; B = B2; }
-                    }
-                    if (lane == 0) {
-                        s_len[0] = L; s_a[0] = A; s_b[0] = B;
-                        s_nsh = 0; s_fuv = 0; s_fvu = 0;
-                    }
-                }
-                __syncthreads();
-                snap = !(s_len[0] < INFINITY);  // no candidate edge left
-                u = s_a[0];
-                v = s_b[0];
-            }
-            if (snap) {  // LOD li: the live facets in index order
-                uint32_t pos = 0;
-                uint32_t* out = lodF + (size_t)li * 3 * Ftot + 3 * f0;
-                for (uint32_t c = 0; c < m; c += T) {
-                    const uint32_t f = c + tid;
-                    const bool al = f < m && (fl[f] & 1);
-                    const unsigned bal = __ballot_sync(0xffffffffu, al);
-                    if (lane == 0) s_red[0][wid] = __popc(bal);
-                    __syncthreads();
-                    uint32_t before = 0, total = 0;
-                    for (int w = 0; w < NW; ++w) {
-                        const uint32_t x = s_red[0][w];
-                        total += x;
-                        if (w < wid) before += x;
-                    }
-                    if (al) {
-                        const uint32_t at = pos + before + __popc(bal & ((1u << lane) - 1u));
-                        for (int k = 0; k < 3; ++k) out[3 * (size_t)at + k] = fv[3 * f + k];
-                    }
-                    pos += total;
-                    __syncthreads();
-                }
-                if (tid == 0) lodCnt[(size_t)o * kDecLods + li] = pos;
-                --li;
-                continue;
-            }
-            // scan 1: facets around u and v -- shared facets, neighbour masks, normals
-            for (uint32_t f = tid; f < m; f += T) {
-                if (!(fl[f] & 1)) continue;
-                const uint32_t x = fv[3 * f], y = fv[3 * f + 1], z = fv[3 * f + 2];
-                const bool hu = x == u || y == u || z == u, hv = x == v || y == v || z == v;
-                if (!hu && !hv) continue;
-                if (hu && hv) {
-                    const int k = atomicAdd(&s_nsh, 1);
-                    if (k < 2) s_third[k] = (x != u && x != v) ? x : (y != u && y != v) ? y : z;
-                }
-                if (hu) mark(Mu, x, y, z, u);
-                if (hv) mark(Mv, x, y, z, v);
-                if (hu && !hv && turns(P, x, y, z, u, v)) s_fuv = 1;
-                if (hv && !hu && turns(P, x, y, z, v, u)) s_fvu = 1;
-            }
-            __syncthreads();
-            const bool cand = s_nsh == 2 && s_third[0] != s_third[1];
-            const uint32_t w1 = s_third[0], w2 = s_third[1];
-            if (cand) {  // scan 2: neighbours of the two third vertices
-                for (uint32_t f = tid; f < m; f += T) {
-                    if (!(fl[f] & 1)) continue;
-                    const uint32_t x = fv[3 * f], y = fv[3 * f + 1], z = fv[3 * f + 2];
-                    if (x == w1 || y == w1 || z == w1) mark(M1, x, y, z, w1);
-                    if (x == w2 || y == w2 || z == w2) mark(M2, x, y, z, w2);
-                }
-                __syncthreads();
-            }
-            // mask counts (and clear)
-            uint32_t c0 = 0, c1 = 0, c2 = 0;
-            for (uint32_t w = tid; w < W; w += T) {
-                c0 += __popc(Mu[w] & Mv[w]);
-                c1 += __popc(M1[w]);
-                c2 += __popc(M2[w]);
-                Mu[w] = Mv[w] = M1[w] = M2[w] = 0;
-            }
-#pragma unroll
-            for (int s = 16; s > 0; s >>= 1) {
-                c0 += __shfl_xor_sync(0xffffffffu, c0, s);
-                c1 += __shfl_xor_sync(0xffffffffu, c1, s);
-                c2 += __shfl_xor_sync(0xffffffffu, c2, s);
-            }
-            if (lane == 0) { s_red[0][wid] = c0; s_red[1][wid] = c1; s_red[2][wid] = c2; }
-            __syncthreads();
-            c0 = c1 = c2 = 0;
-            for (int w = 0; w < NW; ++w) { c0 += s_red[0][w]; c1 += s_red[1][w]; c2 += s_red[2][w]; }
-            const bool link = cand && c0 == 2 && c1 > 3 && c2 > 3;
-            int mode = 0;  // 0: refuse the edge, 1: collapse r into k
-            uint32_t r = 0, k = 0;
-            if (link && !s_fuv) { mode = 1; r = u; k = v; }
-            else if (link && !s_fvu) { mode = 1; r = v; k = u; }
-            // scan 3: apply
-            int kills = 0;
-            for (uint32_t f = tid; f < m; f += T) {
-                const uint32_t fla = fl[f];
-                if (!(fla & 1)) continue;
-                VI* t = fv + 3 * f;
-                const uint32_t x = t[0], y = t[1], z = t[2];
-                if (mode) {
-                    const bool hr = x == r || y == r || z == r, hk = x == k || y == k || z == k;
-                    if (hr && hk) { fl[f] = 0; ++kills; dirty |= f == bf; continue; }
-                    if (!hr && !hk) continue;
-                    if (hr) {
-                        if (x == r) t[0] = (VI)k;
-                        if (y == r) t[1] = (VI)k;
-                        if (z == r) t[2] = (VI)k;
-                    }
-                    uint32_t nf = fla;  // every edge at k is a candidate again
-#pragma unroll
-                    for (int j = 0; j < 3; ++j)
-                        if ((uint32_t)t[j] == k || (uint32_t)t[j == 2 ? 0 : j + 1] == k) nf &= ~(2u << j);
-                    fl[f] = (uint8_t)nf;
-                    if (f == bf) dirty = true;  // its old keys may have been the minimum
-                    else fold_facet(P, fv, f, nf, bl, ba, bb, bf);
-                } else {
-                    const bool hu = x == u || y == u || z == u, hv = x == v || y == v || z == v;
-                    if (!(hu && hv)) continue;
-                    uint32_t nf = fla;
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        const uint32_t a = t[j], b = t[j == 2 ? 0 : j + 1];
-                        if ((a == u && b == v) || (a == v && b == u)) nf |= 2u << j;
-                    }
-                    fl[f] = (uint8_t)nf;
-                    dirty |= f == bf;  // slots only left the candidates
-                }
-            }
-            if (kills) atomicSub(&s_alive, kills);
-            __syncthreads();
-        }
-        __syncthreads();  // the next object reuses the storage
     }
 }
 
@@ -398,6 +242,327 @@ __device__ __forceinline__ uint32_t block_excl_sum(uint32_t x, uint32_t* red, ui
     }
     __syncthreads();
     return before + incl - x;
+}
+
+// ------------------------------------------------------------------ decimation
+// The live facets of vertex x, 32 at a time, one a lane: fn(facet, valid) is
+// called by the whole warp.  x's chain of merged vertices is followed 32 at a
+// time, their lists taken as one row.  Returns the rows' number; `last` is the
+// lane's facet in the last one (UINT_MAX: none).
+template <typename VI, typename Fn>
+__device__ __forceinline__ int each_facet(uint32_t x, const VI* next, const uint32_t* start, const uint32_t* csr,
+                                          const uint8_t* fl, int lane, uint32_t& last, Fn fn) {
+    constexpr uint32_t kEnd = (uint32_t)(VI)~0u;
+    uint32_t s = x;
+    int rows = 0;
+    while (s != kEnd) {
+        uint32_t mine = kEnd;
+        int k = 0;
+        for (; k < 32 && s != kEnd; ++k) {
+            if (lane == k) mine = s;
+            s = next[s];
+        }
+        const uint32_t b = lane < k ? start[mine] : 0u, c = lane < k ? start[mine + 1] - b : 0u;
+        uint32_t end = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            if (o >= k) break;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, end, k - 1);
+        for (uint32_t e0 = 0; e0 < total; e0 += 32) {
+            const uint32_t at = min(e0 + lane, total - 1);
+            int src = 0;  // the first list that ends after `at`
+            if (k > 1) {
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, end, src + step - 1) <= at && src + step < k) src += step;
+            }
+            const uint32_t lb = __shfl_sync(0xffffffffu, b, src), lc = __shfl_sync(0xffffffffu, c, src),
+                           le = __shfl_sync(0xffffffffu, end, src);
+            const uint32_t f = csr[lb + (at - (le - lc))];
+            const bool on = e0 + lane < total && (fl[f] & 1);
+            last = on ? f : UINT_MAX;
+            ++rows;
+            fn(f, on);
+        }
+    }
+    return rows;
+}
+
+template <typename VI, int T>
+__global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict__ objs, int n_objs, DecLists D,
+                                                uint8_t* gstore, const int64_t* __restrict__ gstore_off,
+                                                uint32_t* __restrict__ lodF, int64_t Ftot, uint32_t* __restrict__ lodCnt) {
+    constexpr int NW = T / 32;
+    static_assert(NW >= 4, "a round uses four warps beside each other");
+    extern __shared__ __align__(16) uint8_t dsm[];
+    __shared__ Key s_key[NW];
+    __shared__ uint32_t s_red[NW], s_third[2], s_cnt[3], s_list[kTouched];
+    __shared__ int s_nsh, s_turn[2], s_alive, s_ng;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int i = blockIdx.x; i < n_objs; i += gridDim.x) {
+        const int o = objs[i];
+        const int64_t v0 = M.voff[o], f0 = M.foff[o];
+        const uint32_t n = (uint32_t)(M.voff[o + 1] - v0), m = (uint32_t)(M.foff[o + 1] - f0);
+        const float* P = M.V + 3 * v0;
+        uint8_t* base = gstore ? gstore + gstore_off[i] : dsm;
+        const uint32_t W = (n + 31) / 32, G = (m + kGroup - 1) / kGroup;
+        VI* fv = reinterpret_cast<VI*>(base);
+        uint8_t* fl = base + round16(3 * (size_t)m * sizeof(VI));
+        uint32_t* Mu = reinterpret_cast<uint32_t*>(fl + round16(m));
+        uint32_t *Mv = Mu + W, *M1 = Mu + 2 * W, *M2 = Mu + 3 * W;
+        VI* next = reinterpret_cast<VI*>(reinterpret_cast<uint8_t*>(Mu) + round16(16 * (size_t)W));
+        VI* tail = reinterpret_cast<VI*>(reinterpret_cast<uint8_t*>(next) + round16((size_t)n * sizeof(VI)));
+        Key* gk = reinterpret_cast<Key*>(reinterpret_cast<uint8_t*>(tail) + round16((size_t)n * sizeof(VI)));
+        Key* keys = D.keys + f0;
+        uint32_t* csr = D.csr + 3 * f0;
+        uint32_t* start = D.start + v0 + o;
+        uint32_t* cur = D.cur + v0;
+        for (uint32_t f = tid; f < m; f += T) {
+            uint32_t t[3];
+            for (int k = 0; k < 3; ++k) {
+                t[k] = M.F[3 * (f0 + f) + k];
+                fv[3 * f + k] = (VI)t[k];
+            }
+            fl[f] = 1;  // bit 0 live, bit 1 + j: edge (j, j + 1) refused
+            keys[f] = facet_key(vtx(P, t[0]), vtx(P, t[1]), vtx(P, t[2]), t[0], t[1], t[2], 1);
+        }
+        for (uint32_t w = tid; w < 4 * W; w += T) Mu[w] = 0;
+        for (uint32_t v = tid; v < n; v += T) {
+            next[v] = (VI)~0u;
+            tail[v] = (VI)v;
+            cur[v] = 0;
+        }
+        if (tid == 0) {
+            s_alive = (int)m;
+            s_nsh = s_turn[0] = s_turn[1] = s_ng = 0;
+        }
+        __syncthreads();
+        // every vertex's facets
+        for (uint32_t c = tid; c < 3 * m; c += T) atomicAdd(cur + fv[c], 1u);
+        __syncthreads();
+        uint32_t run = 0;
+        for (uint32_t c0 = 0; c0 < n; c0 += T) {
+            const uint32_t v = c0 + tid, x = v < n ? cur[v] : 0u;
+            uint32_t total;
+            const uint32_t at = run + block_excl_sum<T>(x, s_red, total);
+            if (v < n) {
+                start[v] = at;
+                cur[v] = at;
+            }
+            run += total;
+        }
+        if (tid == 0) start[n] = run;
+        __syncthreads();
+        for (uint32_t c = tid; c < 3 * m; c += T) csr[atomicAdd(cur + fv[c], 1u)] = c / 3;
+        auto redo_group = [&](uint32_t g) {
+            const uint32_t f = g * kGroup + lane;
+            const Key k = warp_least(f < m ? keys[f] : no_key());
+            if (lane == 0) gk[g] = k;
+        };
+        for (uint32_t g = wid; g < G; g += NW) redo_group(g);
+        __syncthreads();
+        // the whole warp: the groups of its changed facets f to the list, each once
+        auto touched = [&](uint32_t f, bool changed) {
+            const uint32_t g = changed ? f / kGroup : UINT_MAX - lane;
+            const unsigned same = __match_any_sync(0xffffffffu, g);
+            const bool first = changed && lane == __ffs(same) - 1;
+            const unsigned all = __ballot_sync(0xffffffffu, first);
+            if (!all) return;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&s_ng, __popc(all));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(all & ((1u << lane) - 1u));
+            if (first && at < kTouched) s_list[at] = g;
+        };
+        int li = kDecLods - 1;
+        auto target_of = [&](int l) { return (uint32_t)((uint64_t)m * (uint64_t)(20 * (l + 1)) / 100); };  // LOD 20 (l + 1)
+        uint32_t target = target_of(li);
+        while (li >= 0) {
+            bool snap = (uint32_t)s_alive <= target;
+            uint32_t u = 0, v = 0;
+            if (!snap) {
+                Key k = no_key();
+                for (uint32_t g = tid; g < G; g += 4 * T) {  // the loads of four at a time beside each other
+                    Key x[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) x[j] = g + j * T < G ? gk[g + j * T] : no_key();
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (key_less(x[j], k)) k = x[j];
+                }
+                k = warp_least(k);
+                if (lane == 0) s_key[wid] = k;
+                __syncthreads();
+                k = warp_least(lane < NW ? s_key[lane] : no_key());
+                snap = k.l >= kNoLength;  // no candidate edge left
+                u = (uint32_t)(k.ab >> 32);
+                v = (uint32_t)k.ab;
+            }
+            if (snap) {  // LOD li: the live facets in index order
+                __syncthreads();
+                uint32_t pos = 0;
+                uint32_t* out = lodF + (size_t)li * 3 * Ftot + 3 * f0;
+                for (uint32_t c = 0; c < m; c += T) {
+                    const uint32_t f = c + tid;
+                    const bool al = f < m && (fl[f] & 1);
+                    uint32_t total;
+                    const uint32_t at = pos + block_count_before<T>(al, s_red, total);
+                    if (al)
+                        for (int k = 0; k < 3; ++k) out[3 * (size_t)at + k] = fv[3 * f + k];
+                    pos += total;
+                }
+                if (tid == 0) lodCnt[(size_t)o * kDecLods + li] = pos;
+                target = target_of(--li);
+                continue;
+            }
+            // the facets around u (warp 0) and v (warp 1): shared ones, neighbours
+            const uint32_t own = wid ? v : u, other = wid ? u : v;  // of warps 0 and 1
+            uint32_t row = UINT_MAX;  // the lane's facet around its warp's end of the edge
+            int rows = 0, nsh = 0;
+            if (wid < 2) {
+                uint32_t* mask = wid ? Mv : Mu;
+                rows = each_facet<VI>(own, next, start, csr, fl, lane, row, [&](uint32_t f, bool on) {
+                    uint32_t a = 0, b = 0, c = 0;
+                    if (on) {
+                        a = fv[3 * f];
+                        b = fv[3 * f + 1];
+                        c = fv[3 * f + 2];
+                        mark(mask, a, b, c, own);
+                    }
+                    if (wid) return;
+                    const bool both = on && (a == v || b == v || c == v);
+                    const unsigned sh = __ballot_sync(0xffffffffu, both);
+                    const int at = nsh + __popc(sh & ((1u << lane) - 1u));
+                    if (both && at < 2) s_third[at] = (a != u && a != v) ? a : (b != u && b != v) ? b : c;
+                    nsh += __popc(sh);
+                });
+                if (tid == 0) s_nsh = nsh;
+            }
+            __syncthreads();
+            const bool cand = s_nsh == 2 && s_third[0] != s_third[1];
+            // A facet around the edge with its corners' points: kept from the normals
+            // to the change where the row is one.
+            struct Facet {
+                uint32_t f, a, b, c;
+                double3 p, q, r;
+            };
+            Facet held;
+            auto load = [&](uint32_t f) {
+                const uint32_t a = fv[3 * f], b = fv[3 * f + 1], c = fv[3 * f + 2];
+                return Facet{f, a, b, c, vtx(P, a), vtx(P, b), vtx(P, c)};
+            };
+            auto around = [&](auto fn) {  // fn(facet, on) by the whole warp
+                uint32_t unused;
+                if (rows == 1) fn(held, row != UINT_MAX);
+                else
+                    each_facet<VI>(own, next, start, csr, fl, lane, unused, [&](uint32_t f, bool on) {
+                        Facet t{};
+                        if (on) t = load(f);
+                        fn(t, on);
+                    });
+            };
+            double3 to = make_double3(0.0, 0.0, 0.0);  // the other end
+            if (wid < 2) {
+                to = vtx(P, other);
+                if (rows == 1 && row != UINT_MAX) held = load(row);
+            }
+            if (cand) {
+                if (wid < 2) {  // does a facet turn when its end moves to the other?
+                    bool turn = false;
+                    around([&](const Facet& t, bool on) {
+                        if (on && t.a != other && t.b != other && t.c != other && turns(t.a, t.b, t.p, t.q, t.r, own, to)) turn = true;
+                    });
+                    if (turn) s_turn[wid] = 1;
+                } else if (wid < 4) {  // neighbours of the two third vertices
+                    const uint32_t x = s_third[wid - 2];
+                    uint32_t* mask = wid == 2 ? M1 : M2;
+                    uint32_t cnt = 0, unused;
+                    auto add = [&](uint32_t a) {
+                        if (a != x && !(atomicOr(mask + (a >> 5), 1u << (a & 31)) & (1u << (a & 31)))) ++cnt;
+                    };
+                    each_facet<VI>(x, next, start, csr, fl, lane, unused, [&](uint32_t f, bool on) {
+                        if (!on) return;
+                        add(fv[3 * f]);
+                        add(fv[3 * f + 1]);
+                        add(fv[3 * f + 2]);
+                    });
+                    cnt = __reduce_add_sync(0xffffffffu, cnt);
+                    if (lane == 0) s_cnt[wid - 2] = cnt;
+                }
+                if (wid == (NW > 4 ? 4 : 3)) {  // neighbours that u and v share
+                    uint32_t cnt = 0;
+                    for (uint32_t w = lane; w < W; w += 32) cnt += __popc(Mu[w] & Mv[w]);
+                    cnt = __reduce_add_sync(0xffffffffu, cnt);
+                    if (lane == 0) s_cnt[2] = cnt;
+                }
+            }
+            __syncthreads();
+            const bool link = cand && s_cnt[2] == 2 && s_cnt[0] > 3 && s_cnt[1] > 3;
+            // collapse r into k, or refuse the edge
+            const bool uv = link && !s_turn[0], vu = link && !uv && !s_turn[1], go = uv || vu;
+            const uint32_t r = uv ? u : v, k = uv ? v : u;
+            if (go && wid < 2) {
+                const bool moves = own == r;  // this warp's end goes to the other
+                around([&](const Facet& t, bool on) {
+                    const bool both = on && (t.a == other || t.b == other || t.c == other);
+                    const bool dies = both && moves, stays = on && !both;  // (a shared one is in both rows)
+                    if (dies) {
+                        fl[t.f] = 0;
+                        keys[t.f] = no_key();
+                    }
+                    if (stays) {
+                        const uint32_t a = t.a == r ? k : t.a, b = t.b == r ? k : t.b, c = t.c == r ? k : t.c;
+                        if (moves) {
+                            VI* w = fv + 3 * t.f;
+                            w[0] = (VI)a;
+                            w[1] = (VI)b;
+                            w[2] = (VI)c;
+                        }
+                        uint32_t nf = fl[t.f];  // every edge at k is a candidate again
+                        if (a == k || b == k) nf &= ~2u;
+                        if (b == k || c == k) nf &= ~4u;
+                        if (c == k || a == k) nf &= ~8u;
+                        fl[t.f] = (uint8_t)nf;
+                        keys[t.f] = facet_key(t.a == r ? to : t.p, t.b == r ? to : t.q, t.c == r ? to : t.r, a, b, c, nf);
+                    }
+                    const unsigned dead = __ballot_sync(0xffffffffu, dies);
+                    if (dead && lane == 0) atomicSub(&s_alive, __popc(dead));
+                    touched(t.f, dies || stays);
+                });
+            } else if (!go && wid == 0) {
+                around([&](const Facet& t, bool on) {
+                    const bool both = on && (t.a == v || t.b == v || t.c == v);
+                    if (both) {
+                        uint32_t nf = fl[t.f];
+                        if ((t.a == u && t.b == v) || (t.a == v && t.b == u)) nf |= 2u;
+                        if ((t.b == u && t.c == v) || (t.b == v && t.c == u)) nf |= 4u;
+                        if ((t.c == u && t.a == v) || (t.c == v && t.a == u)) nf |= 8u;
+                        fl[t.f] = (uint8_t)nf;
+                        keys[t.f] = facet_key(t.p, t.q, t.r, t.a, t.b, t.c, nf);
+                    }
+                    touched(t.f, both);
+                });
+            } else {
+                for (uint32_t w = tid - 64; w < 4 * W; w += T - 64) Mu[w] = 0;
+            }
+            __syncthreads();
+            // the touched groups; k's chain goes on with r's
+            const int ng = s_ng;
+            if (ng <= kTouched)
+                for (int q = wid; q < ng; q += NW) redo_group(s_list[q]);
+            else
+                for (uint32_t g = wid; g < G; g += NW) redo_group(g);
+            if (tid == 0 && go) {
+                next[tail[k]] = (VI)r;
+                tail[k] = tail[r];
+            }
+            __syncthreads();
+            if (tid == 0) s_turn[0] = s_turn[1] = s_ng = 0;  // read again after the next barrier
+        }
+        __syncthreads();  // the next object reuses the storage
+    }
 }
 
 // nearest of the points c[0..k) (double triples) to p; ties to the lowest index
@@ -776,7 +941,7 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
         size_t acc = 0;
         for (long o = 0; o < n_objects; ++o) {
             const int64_t n = vert_off[o + 1] - vert_off[o], m = face_off[o + 1] - face_off[o];
-            const size_t need = 24 * (size_t)n + (12 + 48 + 40) * (size_t)m + 80 * ((size_t)m / voxel_size + 1) +
+            const size_t need = 32 * (size_t)n + (12 + 48 + 40 + 28) * (size_t)m + 80 * ((size_t)m / voxel_size + 1) +
                                 upper_bytes(m, voxel_size) + dec_bytes(n, m, 4) + 64;
             if (acc > 0 && acc + need > budget) {
                 cuts.push_back(o);
@@ -850,6 +1015,11 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
             else if (n <= 65535 && b16 <= kSmemLarge) { large.push_back((int)i); s_large = std::max(s_large, b16); }
             else { huge.push_back((int)i); hoff.push_back(hoff.back() + (int64_t)dec_bytes(n, m, 4)); }
         }
+        DecLists dls{};
+        CU(dm.get(&dls.keys, (size_t)Ftot));
+        CU(dm.get(&dls.csr, 3 * (size_t)Ftot));
+        CU(dm.get(&dls.start, (size_t)(Vtot + nb)));
+        CU(dm.get(&dls.cur, (size_t)Vtot));
         int* dl;
         CU(dm.get(&dl, small.size() + large.size() + huge.size()));
         std::vector<int> all(small);
@@ -859,15 +1029,15 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
         if (!small.empty()) {
             auto kern = k_decimate<uint16_t, 128>;
             CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_small));
-            kern<<<(int)std::min<size_t>(small.size(), 1u << 30), 128, s_small, s>>>(Mh, dl, (int)small.size(), nullptr,
-                                                                                    nullptr, lodF, Ftot, lodCnt);
+            kern<<<(int)std::min<size_t>(small.size(), 1u << 30), 128, s_small, s>>>(Mh, dl, (int)small.size(), dls,
+                                                                                    nullptr, nullptr, lodF, Ftot, lodCnt);
             CU(cudaGetLastError());
         }
         if (!large.empty()) {
-            auto kern = k_decimate<uint16_t, 1024>;
+            auto kern = k_decimate<uint16_t, 256>;
             CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_large));
-            kern<<<(int)large.size(), 1024, s_large, s>>>(Mh, dl + small.size(), (int)large.size(), nullptr, nullptr,
-                                                         lodF, Ftot, lodCnt);
+            kern<<<(int)large.size(), 256, s_large, s>>>(Mh, dl + small.size(), (int)large.size(), dls, nullptr, nullptr,
+                                                        lodF, Ftot, lodCnt);
             CU(cudaGetLastError());
         }
         if (!huge.empty()) {
@@ -877,7 +1047,8 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
             CU(dm.get(&dho, hoff.size()));
             CU(cudaMemcpyAsync(dho, hoff.data(), 8 * hoff.size(), cudaMemcpyHostToDevice, s));
             k_decimate<uint32_t, 1024><<<(int)huge.size(), 1024, 0, s>>>(Mh, dl + small.size() + large.size(),
-                                                                      (int)huge.size(), gst, dho, lodF, Ftot, lodCnt);
+                                                                      (int)huge.size(), dls, gst, dho, lodF, Ftot,
+                                                                      lodCnt);
             CU(cudaGetLastError());
         }
         CU(cudaEventRecord(ev[1], s));
