@@ -565,6 +565,57 @@ cudaError_t launch_gather_bounds(const float4* tri, size_t n, float* out, cudaSt
     return cudaGetLastError();
 }
 
+int bounds_scratch(tdp_ctx* ctx, const BoundRecords& r) {
+    int rc;
+    if ((rc = ensure(ctx, ctx->scratch[kBoxes], (size_t)kNumLods * r.n_vox * 2 * sizeof(float4)))) return rc;
+    if ((rc = ensure(ctx, ctx->scratch[kVobj], (size_t)r.n_vox * sizeof(int)))) return rc;
+    if ((rc = ensure(ctx, ctx->scratch[kMeanEdge], (size_t)r.n_obj * sizeof(double)))) return rc;
+    return ensure(ctx, ctx->scratch[kBoundCounters], 4 * sizeof(unsigned long long));
+}
+
+void bounds_scratch_free(tdp_ctx* ctx) {
+    for (int k = kBoxes; k <= kBoundCounters; ++k) {
+        Buf& b = ctx->scratch[k];
+        if (b.p) dfree(ctx, b.p);
+        b = Buf{};
+    }
+}
+
+const unsigned long long* bounds_counters(const tdp_ctx* ctx) {
+    return (const unsigned long long*)ctx->scratch[kBoundCounters].p;
+}
+
+cudaError_t launch_bounds(tdp_ctx* ctx, const BoundRecords& r) {
+    cudaStream_t s = ctx->stream;
+    BoundsDev b{};
+    float4* boxes = (float4*)ctx->scratch[kBoxes].p;
+    for (int l = 0; l < kNumLods; ++l) {
+        b.tri[l] = r.tri[l];
+        b.vtri[l] = r.vtri[l];
+        b.box[l] = boxes + (size_t)l * r.n_vox * 2;
+    }
+    b.obj_vox = r.obj_vox;
+    b.vobj = (const int*)ctx->scratch[kVobj].p;
+    b.e0 = (const double*)ctx->scratch[kMeanEdge].p;
+    b.n_vox = r.n_vox;
+    b.n_obj = r.n_obj;
+    b.counters = (unsigned long long*)ctx->scratch[kBoundCounters].p;
+    cudaError_t e = cudaMemsetAsync(b.counters, 0, 4 * sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    const int small_grid = ctx->num_sms * 8;
+    for (int l = 0; l < kNumLods; ++l) {
+        if (r.n_tris[l]) k_zero_bounds<<<small_grid, 256, 0, s>>>(r.tri[l], r.n_tris[l]);
+        k_voxel_boxes<<<small_grid, 128, 0, s>>>(r.tri[l], r.vtri[l], r.n_vox, boxes + (size_t)l * r.n_vox * 2);
+    }
+    k_objects<<<(int)std::min<long>((r.n_obj + 3) / 4, (long)ctx->num_sms * 16), 128, 0, s>>>(
+        b, (int*)ctx->scratch[kVobj].p, (double*)ctx->scratch[kMeanEdge].p);
+    const int grid = ctx->num_sms * kBoundsBlocksPerSm;
+    k_proxy<<<grid, kBoundsThreads, 0, s>>>(b);
+    k_hausdorff<<<grid, kBoundsThreads, 0, s>>>(b);
+    k_object_bounds<<<small_grid, 256, 0, s>>>(b, r.obj_hd, r.obj_phd);
+    return cudaGetLastError();
+}
+
 }  // namespace tdp
 
 using namespace tdp;
@@ -577,45 +628,27 @@ extern "C" int tdp_tile_compute_bounds(tdp_ctx* ctx, tdp_tile* tile, tdp_bounds_
     cudaStream_t s = ctx->stream;
     const long nv = tile->n_vox, no = tile->n_obj;
     if (no == 0 || nv == 0) return TDP_OK;
-    int rc;
-    if ((rc = ensure(ctx, ctx->scratch[kBoxes], (size_t)kNumLods * nv * 2 * sizeof(float4)))) return rc;
-    if ((rc = ensure(ctx, ctx->scratch[kVobj], (size_t)nv * sizeof(int)))) return rc;
-    if ((rc = ensure(ctx, ctx->scratch[kMeanEdge], (size_t)no * sizeof(double)))) return rc;
-    if ((rc = ensure(ctx, ctx->scratch[kBoundCounters], 4 * sizeof(unsigned long long)))) return rc;
-    BoundsDev b{};
-    float4* boxes = (float4*)ctx->scratch[kBoxes].p;
+    BoundRecords r{};
     for (int l = 0; l < kNumLods; ++l) {
-        b.tri[l] = tile->tri[l];
-        b.vtri[l] = tile->vtri[l];
-        b.box[l] = boxes + (size_t)l * nv * 2;
+        r.tri[l] = tile->tri[l];
+        r.vtri[l] = tile->vtri[l];
+        r.n_tris[l] = tile->host.n_tris[l];
     }
-    b.obj_vox = tile->obj_vox;
-    b.vobj = (const int*)ctx->scratch[kVobj].p;
-    b.e0 = (const double*)ctx->scratch[kMeanEdge].p;
-    b.n_vox = nv;
-    b.n_obj = no;
-    b.counters = (unsigned long long*)ctx->scratch[kBoundCounters].p;
+    r.obj_vox = tile->obj_vox;
+    r.n_vox = nv;
+    r.n_obj = no;
+    r.obj_hd = tile->obj_hd;
+    r.obj_phd = tile->obj_phd;
+    if (const int rc = bounds_scratch(ctx, r)) return rc;
 #define CU(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) return fail(ctx, TDP_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(_e)); } while (0)
     // an attached tile first fetches every voxel: the bounds are written into
     // the device records, which later fetches must not overwrite
     CU(launch_fetch_all(lazy_view(tile), ctx->num_sms, s));
     CU(cudaEventRecord(ctx->ev[0], s));
-    CU(cudaMemsetAsync(b.counters, 0, 4 * sizeof(unsigned long long), s));
-    const int small_grid = ctx->num_sms * 8;
-    for (int l = 0; l < kNumLods; ++l) {
-        const size_t n = tile->host.n_tris[l];
-        if (n) k_zero_bounds<<<small_grid, 256, 0, s>>>(tile->tri[l], n);
-        k_voxel_boxes<<<small_grid, 128, 0, s>>>(tile->tri[l], tile->vtri[l], nv, boxes + (size_t)l * nv * 2);
-    }
-    k_objects<<<(int)std::min<long>((no + 3) / 4, (long)ctx->num_sms * 16), 128, 0, s>>>(b, (int*)ctx->scratch[kVobj].p, (double*)ctx->scratch[kMeanEdge].p);
-    const int grid = ctx->num_sms * kBoundsBlocksPerSm;
-    k_proxy<<<grid, kBoundsThreads, 0, s>>>(b);
-    k_hausdorff<<<grid, kBoundsThreads, 0, s>>>(b);
-    k_object_bounds<<<small_grid, 256, 0, s>>>(b, tile->obj_hd, tile->obj_phd);
-    CU(cudaGetLastError());
+    CU(launch_bounds(ctx, r));
     CU(cudaEventRecord(ctx->ev[1], s));
     unsigned long long cnt[4] = {0, 0, 0, 0};
-    CU(cudaMemcpyAsync(cnt, b.counters, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(cnt, bounds_counters(ctx), sizeof(cnt), cudaMemcpyDeviceToHost, s));
     tile->host.obj_hd.resize((size_t)no * kNumLods);
     tile->host.obj_phd.resize((size_t)no * kNumLods);
     CU(cudaMemcpyAsync(tile->host.obj_hd.data(), tile->obj_hd, (size_t)no * kNumLods * 4, cudaMemcpyDeviceToHost, s));

@@ -5,7 +5,7 @@
 // decimation into LODs (src/spatial/himesh_comp.cpp:28-190), skeleton voxels
 // (src/spatial/himesh_skeleton.cpp:17-168), LOD triangles to voxels
 // (src/spatial/himesh_retrieve.cpp:183-200), the per-triangle Hausdorff bounds
-// (src/spatial/himesh_hausdorff.cpp:197-296, done here by
+// (src/spatial/himesh_hausdorff.cpp:197-296, done here with the kernels of
 // tdp_tile_compute_bounds) and the RAW writer (src/storage/tile_IO.cpp:79-172).
 // The rule, per object with vertices P (float, evaluated in double) and
 // LOD-100 facets F[0..m):
@@ -58,6 +58,7 @@
 #include <string>
 #include <vector>
 
+#include "bounds_kernels.cuh"
 #include "ctx.cuh"
 #include "storage/dt_format.h"
 
@@ -749,12 +750,43 @@ __global__ void __launch_bounds__(T) k_voxels(Meshes M, int voxel_size, const ui
     }
 }
 
+// ------------------------------------------------------------------ records
+// The batch's triangle records for the bound preparation, as a resident tile of
+// its RAW bytes would hold them: block (o, l) places LOD l of object o, grouped
+// by voxel, from record t0[l][o] on.  (Through the host, that tile took 30 of
+// the 48 ms of bounds of 1,000 nuclei: 169 MB down, parsed, up and unpacked.)
+struct RecordsDev {
+    float4* tri[kNumLods];
+    uint32_t* vtri[kNumLods];
+    const uint32_t* t0[kNumLods];  // n + 1: an object's first record at the LOD
+    const uint32_t* vox0;          // n + 1: an object's first voxel
+    const float *hd, *phd;         // kNumLods object-level values an object, once computed
+};
+
+__global__ void __launch_bounds__(kPrepThreads) k_records(Meshes M, const uint32_t* __restrict__ lodF, VoxScratch S, RecordsDev R) {
+    const int l = blockIdx.y;
+    for (int o = blockIdx.x; o < M.n; o += gridDim.x) {
+        const int64_t f0 = M.foff[o], s0 = S.soff[o];
+        const float* P = M.V + 3 * M.voff[o];
+        const uint32_t* LF = l < kNumLods - 1 ? lodF + (size_t)l * 3 * S.Ftot + 3 * f0 : M.F + 3 * f0;
+        const uint32_t* od = S.ord + (size_t)l * S.Ftot + f0;
+        const uint32_t t0 = R.t0[l][o], n = R.t0[l][o + 1] - t0, v0 = R.vox0[o], nv = R.vox0[o + 1] - v0;
+        for (uint32_t i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+            const float* q = P + 3 * (size_t)LF[3 * od[i / 3] + i % 3];
+            R.tri[l][3 * (size_t)t0 + i] = make_float4(q[0], q[1], q[2], 0.f);
+        }
+        for (uint32_t v = threadIdx.x; v < nv; v += blockDim.x) R.vtri[l][v0 + v] = t0 + S.vst[(size_t)l * S.Stot + s0 + v];
+        if (threadIdx.x == 0 && o == M.n - 1) R.vtri[l][v0 + nv] = t0 + n;
+    }
+}
+
 // ------------------------------------------------------------------ RAW writer
 // Object o's bytes start at word pos[o] / 4 of `out` (every object is a
-// multiple of 4 bytes long and the batch starts on an object).
+// multiple of 4 bytes long and the batch starts on an object).  The bounds are
+// those of R's records, 0 without records.
 template <int T>
 __global__ void __launch_bounds__(T) k_write(Meshes M, const uint32_t* __restrict__ lodF, const uint32_t* __restrict__ lodCnt,
-                                             VoxScratch S, const unsigned long long* __restrict__ pos,
+                                             VoxScratch S, const unsigned long long* __restrict__ pos, RecordsDev R,
                                              uint32_t* __restrict__ out) {
     constexpr int NW = T / 32;
     __shared__ float s_f[6][NW];
@@ -794,13 +826,15 @@ __global__ void __launch_bounds__(T) k_write(Meshes M, const uint32_t* __restric
                     c[3 * k + 1] = __float_as_uint(q[1]);
                     c[3 * k + 2] = __float_as_uint(q[2]);
                 }
-                grp[9 * cv + 2 * j] = 0u;
-                grp[9 * cv + 2 * j + 1] = 0u;
+                const float4* r = R.tri[l] ? R.tri[l] + 3 * ((size_t)R.t0[l][o] + g) : nullptr;
+                grp[9 * cv + 2 * j] = r ? __float_as_uint(r[0].w) : 0u;
+                grp[9 * cv + 2 * j + 1] = r ? __float_as_uint(r[1].w) : 0u;
             }
         }
         uint32_t* H = D + 11 * (size_t)ntri;
         if (tid == 0) { H[0] = nvox; H[1] = 0u; }
-        if (tid < 2 * kNumLods) H[2 + tid] = 0u;  // object-level bounds
+        if (tid < 2 * kNumLods)  // object-level bounds: (hausdorff, proxy) of every LOD
+            H[2 + tid] = R.hd ? __float_as_uint((tid & 1 ? R.phd : R.hd)[(size_t)o * kNumLods + tid / 2]) : 0u;
         for (uint32_t v = tid; v < nvox; v += T) {
             float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
             for (int l = 0; l < kNumLods; ++l) {
@@ -816,16 +850,16 @@ __global__ void __launch_bounds__(T) k_write(Meshes M, const uint32_t* __restric
                         }
                     }
             }
-            uint32_t* R = H + 12 + 29 * (size_t)v;
-            for (int d = 0; d < 3; ++d) { R[d] = __float_as_uint(lo[d]); R[3 + d] = __float_as_uint(hi[d]); }
-            for (int d = 0; d < 3; ++d) R[6 + d] = __float_as_uint(P[3 * (size_t)core[v] + d]);
+            uint32_t* X = H + 12 + 29 * (size_t)v;
+            for (int d = 0; d < 3; ++d) { X[d] = __float_as_uint(lo[d]); X[3 + d] = __float_as_uint(hi[d]); }
+            for (int d = 0; d < 3; ++d) X[6 + d] = __float_as_uint(P[3 * (size_t)core[v] + d]);
             for (int l = 0; l < kNumLods; ++l) {
                 const uint64_t off = 44ull * (lstart[l] + S.vst[(size_t)l * S.Stot + s0 + v]);
                 const uint32_t cv = S.vcnt[(size_t)l * S.Stot + s0 + v];
-                R[9 + 4 * l] = (uint32_t)off;
-                R[10 + 4 * l] = (uint32_t)(off >> 32);
-                R[11 + 4 * l] = cv;
-                R[12 + 4 * l] = 0u;
+                X[9 + 4 * l] = (uint32_t)off;
+                X[10 + 4 * l] = (uint32_t)(off >> 32);
+                X[11 + 4 * l] = cv;
+                X[12 + 4 * l] = 0u;
             }
         }
         // 4. transform: the vertex nearest the centre of the float bounding box
@@ -883,9 +917,12 @@ namespace {
 struct DevMem {  // allocations of one batch, back to the context's block cache on every return
     tdp_ctx* ctx;
     std::vector<void*> ps;
-    ~DevMem() {
+    ~DevMem() { release(); }
+    void release() {
+        if (ps.empty()) return;
         cudaStreamSynchronize(ctx->stream);  // nothing queued may still use a block
         for (void* p : ps) block_release(ctx, p);
+        ps.clear();
     }
     template <typename X>
     cudaError_t get(X** p, size_t count) {
@@ -952,6 +989,10 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
         cuts.push_back(n_objects);
     }
     size_t pos_out = 1;  // the tile's type byte
+    // bounds batch by batch; an object beyond the limits of a resident tile is
+    // left to the upload of the finished tile, which names the limit
+    bool dev_bounds = true;
+    for (long o = 0; o < n_objects; ++o) dev_bounds = dev_bounds && face_off[o + 1] - face_off[o] <= (1 << 24);
     std::vector<unsigned long long> bytes;
     cudaEvent_t ev[4];
     for (auto& e : ev) CU(cudaEventCreate(&e));
@@ -1097,13 +1138,62 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
             inf.n_triangles[kNumLods - 1] += foff[i + 1] - foff[i];
             inf.n_voxels += hnvox[i];
         }
-        // 4. RAW bytes of the batch, then to the caller's buffer
         if (out && pos_out + run <= cap) {
             uint32_t* dout;
             CU(dm.get(&dout, (size_t)(run / 4)));
+            // 4. the bounds of the batch's triangles and objects
+            DevMem bm{ctx, {}};
+            RecordsDev R{};
+            BoundRecords br{};
+            std::vector<uint32_t> at((size_t)(kNumLods + 1) * (nb + 1));  // t0 of every LOD, then vox0
+            if (dev_bounds) {
+                for (int l = 0; l <= kNumLods; ++l) {
+                    uint64_t sum = 0;
+                    for (long i = 0; i <= nb; ++i) {
+                        at[(size_t)l * (nb + 1) + i] = (uint32_t)sum;
+                        if (i < nb) sum += l == kNumLods ? hnvox[i] : l == kNumLods - 1 ? (uint64_t)(foff[i + 1] - foff[i]) : hcnt[(size_t)i * kDecLods + l];
+                    }
+                    if (l < kNumLods) br.n_tris[l] = (size_t)sum;
+                    else br.n_vox = (long)sum;
+                    if (sum >= UINT_MAX) dev_bounds = false;
+                }
+                br.n_obj = nb;
+            }
+            if (dev_bounds) {
+                uint32_t* dat;
+                float* obj;
+                bool ok = bm.get(&dat, at.size()) == cudaSuccess && bm.get(&obj, 2 * (size_t)kNumLods * nb) == cudaSuccess;
+                for (int l = 0; ok && l < kNumLods; ++l) {
+                    uint32_t* vt;
+                    ok = bm.get(&br.tri[l], 3 * br.n_tris[l]) == cudaSuccess && bm.get(&vt, (size_t)br.n_vox + 1) == cudaSuccess;
+                    R.tri[l] = br.tri[l];
+                    R.vtri[l] = vt;
+                    br.vtri[l] = vt;
+                    R.t0[l] = dat + (size_t)l * (nb + 1);
+                }
+                ok = ok && bounds_scratch(ctx, br) == TDP_OK;
+                if (ok) {
+                    R.vox0 = br.obj_vox = dat + (size_t)kNumLods * (nb + 1);
+                    R.hd = br.obj_hd = obj;
+                    R.phd = br.obj_phd = obj + (size_t)kNumLods * nb;
+                    CU(cudaMemcpyAsync(dat, at.data(), 4 * at.size(), cudaMemcpyHostToDevice, s));
+                    CU(cudaEventRecord(ev[0], s));
+                    k_records<<<dim3((unsigned)nb, kNumLods), kPrepThreads, 0, s>>>(Mh, lodF, S, R);
+                    CU(cudaGetLastError());
+                    CU(launch_bounds(ctx, br));
+                    CU(cudaEventRecord(ev[1], s));
+                } else {  // no room beside the batch: the finished tile's bounds, below
+                    cudaGetLastError();
+                    bm.release();
+                    bounds_scratch_free(ctx);
+                    R = RecordsDev{};
+                    dev_bounds = false;
+                }
+            }
+            // 5. RAW bytes of the batch, then to the caller's buffer
             CU(cudaMemcpyAsync(dpos, hpos.data(), 8 * nb, cudaMemcpyHostToDevice, s));
             CU(cudaEventRecord(ev[2], s));  // the writer alone (the host's allocation above is not timed)
-            k_write<kPrepThreads><<<(int)nb, kPrepThreads, 0, s>>>(Mh, lodF, lodCnt, S, dpos, dout);
+            k_write<kPrepThreads><<<(int)nb, kPrepThreads, 0, s>>>(Mh, lodF, lodCnt, S, dpos, R, dout);
             CU(cudaGetLastError());
             CU(cudaEventRecord(ev[3], s));
             CU(cudaMemcpyAsync((uint8_t*)out + pos_out, dout, (size_t)run, cudaMemcpyDeviceToHost, s));
@@ -1111,6 +1201,11 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
             float ms = 0;
             cudaEventElapsedTime(&ms, ev[2], ev[3]);
             inf.write_ms += ms;
+            if (R.hd) {
+                cudaEventElapsedTime(&ms, ev[0], ev[1]);
+                inf.bounds_ms += ms;
+                if (ctx->budget) bounds_scratch_free(ctx);  // the next batch's room is what it was
+            }
         }
         pos_out += (size_t)run;
         inf.batches += 1;
@@ -1123,13 +1218,14 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
     }
     if (cap < pos_out) return fail(ctx, TDP_ERR_ARG, "tdp_raw_from_meshes: output buffer too small");
     ((uint8_t*)out)[0] = kRawType;
-    // per-triangle and object-level bounds, on the device
     const auto t_b = std::chrono::steady_clock::now();
-    tdp_bounds_info bi{};
-    int rc = TDP_OK;
-    if (n_objects > 0 && (rc = tdp_raw_compute_bounds(ctx, out, pos_out, out, &bi)) != TDP_OK) return rc;
+    if (n_objects > 0 && !dev_bounds) {
+        if (ctx->budget) cache_trim(ctx);  // blocks of just the sizes asked for
+        tdp_bounds_info bi{};
+        if (const int rc = tdp_raw_compute_bounds(ctx, out, pos_out, out, &bi)) return rc;
+    }
     const auto t_end = std::chrono::steady_clock::now();
-    inf.bounds_ms = std::chrono::duration<double, std::milli>(t_end - t_b).count();
+    if (!dev_bounds) inf.bounds_ms = std::chrono::duration<double, std::milli>(t_end - t_b).count();
     inf.total_ms = std::chrono::duration<double, std::milli>(t_end - t_start).count();
     if (info) *info = inf;
     return TDP_OK;

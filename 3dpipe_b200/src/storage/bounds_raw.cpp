@@ -47,6 +47,12 @@ extern "C" int tdp_raw_compute_bounds(tdp_ctx* ctx, const void* raw, size_t len,
         tdp_tile* t;
         ~Release() { tdp_tile_free(c, t); }
     } release{ctx, T};
+    if (ctx->budget)  // under a cap the upload's staging (scratch 12, 13) makes room
+        for (int k = 12; k <= 13; ++k) {
+            cudaStreamSynchronize(ctx->stream);
+            if (ctx->scratch[k].p) dfree(ctx, ctx->scratch[k].p);
+            ctx->scratch[k] = Buf{};
+        }
     if ((rc = tdp_tile_compute_bounds(ctx, T, info))) return rc;
     const TileHost& H = T->host;
     // the (proxy, hausdorff) pairs of every LOD, in the tile's voxel order

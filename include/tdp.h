@@ -260,7 +260,9 @@ typedef struct {
     double decimate_ms;   /* device time of the decimation kernels */
     double voxel_ms;      /* device time of the voxel kernel */
     double write_ms;      /* device time of the RAW writer */
-    double bounds_ms;     /* host wall time of the bound preparation */
+    double bounds_ms;     /* device time of the bound preparation (host wall time of
+                             it where it took the finished tile: no room for its
+                             records beside a batch) */
     long n_objects;
     long n_triangles[5];  /* per LOD 20..100 */
     long n_voxels;

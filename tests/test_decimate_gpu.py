@@ -56,3 +56,16 @@ def test_meshes_equal_the_oracle(pkg, ctx, name, mesh):
     want = oracle_bounds(oracle_prep(meshes, voxel_size=40))
     np.testing.assert_array_equal(raw, want)
     assert info["n_objects"] == 3
+
+
+@pytest.mark.parametrize("mb", [13, 15, 18, 24])
+def test_bounds_of_a_batch_with_and_without_room_for_its_records(pkg, mb):
+    """Under a small cap the bounds come from the finished tile instead of the
+    batch's own records; the bytes are the same."""
+    V, vo, F, fo = pkg.tdp.gen_meshes(2, 1, seed=3, which="vessels")
+    meshes = [(V[vo[i]:vo[i + 1]], F[fo[i]:fo[i + 1]]) for i in range(2)]
+    with pkg.Context(0, budget_bytes=mb << 20) as small:
+        raw, info = small.raw_from_meshes(V, vo, F, fo, voxel_size=100)
+        raw = np.array(raw)
+    np.testing.assert_array_equal(raw, oracle_bounds(oracle_prep(meshes)))
+    assert info["batches"] == 1
