@@ -14,15 +14,17 @@
 // boundary is decided exactly as on the host.
 //
 // Per query, one warp:
-//   k_cand_kth   ring search over a grid of transform points; after each ring
-//                the K-th smallest (distance, id) key of the points seen so far
-//                is found by bisection, and the search stops once it is inside
-//                the ring's radius by more than the grid's rounding slack;
+//   k_cand_kth   ring search over a grid of transform points, which stops once
+//                K of the points seen so far are inside the ring's radius by
+//                more than the grid's rounding slack; the K-th smallest
+//                (distance, id) key is then found by bisection;
 //   k_cand_pass  scans the box-grid cells that the query box, grown by tau or
 //                by the K-th distance, overlaps; an object spanning several
 //                cells is counted only in its first cell inside the scan
-//                range; a count pass sizes the CSR, a write pass emits keys;
-// then a CUB segmented sort orders each query's keys.
+//                range; a count pass sizes the CSR, a write pass emits keys and
+//                orders its query's by rank (a key is preceded by those below
+//                it) while no query has more than kRankMost; beyond that a CUB
+//                segmented sort and k_cand_finish order them.
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_segmented_sort.cuh>
 #include <float.h>
@@ -86,19 +88,34 @@ __device__ __forceinline__ unsigned long long key_of(float d, int id) {
 constexpr int kWarps = 4;
 constexpr int kCap = 1024;  // transform points a warp keeps during one ring search
 
-// smallest key T with count(key <= T) >= K among n keys (n >= K), by bisection
+// the K-th smallest of n distinct keys (n >= K): its distance by bisection on
+// the keys' high words between their least and largest, then its id likewise
+// among the keys at that distance
 __device__ unsigned long long kth_key(const unsigned long long* keys, int n, int K, int lane) {
-    unsigned long long lo = 0, hi = ~0ull;
-    while (lo < hi) {
-        const unsigned long long mid = lo + (hi - lo) / 2;
-        int c = 0;
-        for (int i = lane; i < n; i += 32) c += keys[i] <= mid;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if (c >= K) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo;
+    constexpr unsigned kFull = 0xffffffffu;
+    auto select = [&](auto&& word, auto&& in, int k) {
+        unsigned lo = UINT_MAX, hi = 0;
+        for (int i = lane; i < n; i += 32)
+            if (in(keys[i])) { lo = min(lo, word(keys[i])); hi = max(hi, word(keys[i])); }
+        lo = __reduce_min_sync(kFull, lo);
+        hi = __reduce_max_sync(kFull, hi);
+        while (lo < hi) {
+            const unsigned mid = lo + (hi - lo) / 2;
+            unsigned c = 0;
+            for (int i = lane; i < n; i += 32) c += in(keys[i]) && word(keys[i]) <= mid;
+            if ((int)__reduce_add_sync(kFull, c) >= k) hi = mid;
+            else lo = mid + 1;
+        }
+        return lo;
+    };
+    auto high = [](unsigned long long k) { return (unsigned)(k >> 32); };
+    auto low = [](unsigned long long k) { return (unsigned)k; };
+    const unsigned d = select(high, [](unsigned long long) { return true; }, K);
+    unsigned before = 0;
+    for (int i = lane; i < n; i += 32) before += high(keys[i]) < d;
+    before = __reduce_add_sync(kFull, before);
+    const unsigned id = select(low, [=](unsigned long long k) { return high(k) == d; }, K - (int)before);
+    return ((unsigned long long)d << 32) | id;
 }
 
 // Ring search of one query (one warp): the K-th smallest (transform
@@ -107,47 +124,88 @@ __device__ unsigned long long kth_key(const unsigned long long* keys, int n, int
 // brought more than cap points (the result is then unusable).  Every point of
 // tile 2 lies in exactly one grid cell and every cell is visited by exactly
 // one ring, so cap >= n2 can never overflow.
+//
+// Latency bounds it (a few hundred points a query): a ring is taken as runs of
+// cells along z, whose points are one range, 32 runs at a time and their points
+// one a lane; rings 0 and 1 go together (the search cannot end at ring 0), a
+// ring only counts the keys inside its radius, and the K-th key is selected
+// once, at the end.  10-NN of 200 / 20,000 queries: 54 / 275 us with a cell a
+// lane and a 64-step bisection on the keys at every ring, 15 / 70 us here.
 __device__ bool kth_search(const DG& pg, const float* xq, const float* __restrict__ xf2, int q, int K, int self,
-                           unsigned long long* keys, int cap, int* cnt, int lane, unsigned long long& result) {
+                           unsigned long long* keys, int cap, int lane, unsigned long long& result) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const unsigned lt = (1u << lane) - 1u;
     const int cx = dci(xq[0], pg.lo0, pg.cell, pg.n0), cy = dci(xq[1], pg.lo1, pg.cell, pg.n1);
     const int cz = dci(xq[2], pg.lo2, pg.cell, pg.n2);
-    if (lane == 0) *cnt = 0;
-    __syncwarp();
+    const float x0 = xq[0], x1 = xq[1], x2 = xq[2];
     const int maxr = max(pg.n0, max(pg.n1, pg.n2));
     result = ~0ull;  // fewer than K objects: every object is a candidate
-    bool over = false;
-    for (int r = 0; r <= maxr; ++r) {
+    int seen = 0;
+    for (int r = 1; r <= maxr; ++r) {
         const int side = 2 * r + 1;
-        const int total = side * side * side;
-        for (int t = lane; t < total; t += 32) {
-            const int dx = t % side - r, dy = (t / side) % side - r, dz = t / (side * side) - r;
-            if (max(abs(dx), max(abs(dy), abs(dz))) != r) continue;
-            const int x = cx + dx, y = cy + dy, z = cz + dz;
-            if (x < 0 || y < 0 || z < 0 || x >= pg.n0 || y >= pg.n1 || z >= pg.n2) continue;
-            const size_t c = ((size_t)x * pg.n1 + y) * pg.n2 + z;
-            for (int64_t k = pg.start[c]; k < pg.start[c + 1]; ++k) {
-                const int o = pg.items[k];
-                if (self && o == q) continue;
-                const int pos = atomicAdd(cnt, 1);
-                if (pos < cap) keys[pos] = key_of(d_point_dist(xq, xf2 + 3 * (size_t)o), o);
+        const int runs = r == 1 ? side * side : 2 * side * side;
+        for (int s0 = 0; s0 < runs; s0 += 32) {
+            const int s = s0 + lane;
+            const int row = r == 1 ? s : s >> 1, half = r == 1 ? 0 : s & 1;
+            const int dy = row % side - r, dx = row / side - r;
+            const int x = cx + dx, y = cy + dy;
+            int64_t b = 0;
+            int n = 0;
+            if (s < runs && x >= 0 && y >= 0 && x < pg.n0 && y < pg.n1) {
+                int z0 = cz - r, z1 = cz + r;  // a row on the ring's sides is whole, others end in two cells
+                bool on = true;
+                if (r > 1 && max(abs(dx), abs(dy)) < r) {
+                    if (half) z0 = z1;
+                    else z1 = z0;
+                } else {
+                    on = !half;
+                }
+                z0 = max(z0, 0);
+                z1 = min(z1, pg.n2 - 1);
+                if (on && z0 <= z1) {
+                    const size_t c = ((size_t)x * pg.n1 + y) * pg.n2;
+                    b = pg.start[c + z0];
+                    n = (int)(pg.start[c + z1 + 1] - b);
+                }
             }
+            int inc = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(kFull, inc, o);
+                if (lane >= o) inc += t;
+            }
+            const int ex = inc - n, tot = __shfl_sync(kFull, inc, 31);
+            for (int j0 = 0; j0 < tot; j0 += 32) {
+                const int j = j0 + lane;
+                int k = 0;  // the last lane whose run starts at or before point j
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(kFull, ex, k + step) <= j) k += step;
+                const int64_t bk = __shfl_sync(kFull, b, k);
+                const int ek = __shfl_sync(kFull, ex, k);
+                const int o = j < tot ? pg.items[bk + (j - ek)] : q;
+                const bool keep = j < tot && !(self && o == q);
+                const unsigned m = __ballot_sync(kFull, keep);
+                const int pos = seen + __popc(m & lt);
+                if (keep && pos < cap) {
+                    const float p[3] = {x0, x1, x2};
+                    keys[pos] = key_of(d_point_dist(p, xf2 + 3 * (size_t)o), o);
+                }
+                seen += __popc(m);
+            }
+            if (seen > cap) return false;
         }
         __syncwarp();
-        const int seen = *cnt;
-        if (seen > cap) {
-            over = true;
-            break;
-        }
         if (seen >= K) {
-            const unsigned long long kk = kth_key(keys, seen, K, lane);
-            const float kd = __uint_as_float((unsigned)(kk >> 32));
-            result = kk;  // best so far; the loop ends after the last ring anyway
-            if (kd < __fsub_rn(__fmul_rn((float)r, pg.cell), pg.slack)) break;
+            const float radius = __fsub_rn(__fmul_rn((float)r, pg.cell), pg.slack);
+            int c = 0;
+            for (int i = lane; i < seen; i += 32) c += __uint_as_float((unsigned)(keys[i] >> 32)) < radius;
+            if (__reduce_add_sync(kFull, c) >= K) break;  // the K-th is inside
         }
-        __syncwarp();
     }
+    if (seen >= K) result = kth_key(keys, seen, K, lane);
     __syncwarp();
-    return !over;
+    return true;
 }
 
 // Pass 1: every kNN query with its keys in shared memory (kCap per warp); a
@@ -160,14 +218,13 @@ __global__ void __launch_bounds__(kWarps * 32) k_cand_kth(DG pg, const float* __
                                                          int* __restrict__ n_over, int* __restrict__ ovlist,
                                                          int qb0) {
     __shared__ unsigned long long keys[kWarps][kCap];
-    __shared__ int cnt[kWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nw = gridDim.x * kWarps;
     for (int q = qb0 + blockIdx.x * kWarps + w; q < n1; q += nw) {
         const int K = qk ? qk[q] : K_all;
         if (K <= 0) continue;  // a within object of a mixed batch (warp-uniform)
         unsigned long long result;
-        const bool ok = kth_search(pg, xf1 + 3 * (size_t)q, xf2, q, K, self, keys[w], kCap, &cnt[w], lane, result);
+        const bool ok = kth_search(pg, xf1 + 3 * (size_t)q, xf2, q, K, self, keys[w], kCap, lane, result);
         if (lane == 0) {
             kth[q] = result;
             if (!ok) ovlist[atomicAdd(n_over, 1)] = q;
@@ -185,15 +242,14 @@ __global__ void __launch_bounds__(kWarps * 32) k_cand_kth_global(DG pg, const fl
                                                                 const int* __restrict__ n_over,
                                                                 const int* __restrict__ ovlist,
                                                                 unsigned long long* __restrict__ gkeys, int cap) {
-    __shared__ int cnt[kWarps];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int gw = blockIdx.x * kWarps + w, nw = gridDim.x * kWarps;
+    const int lane = threadIdx.x & 31;
+    const int gw = blockIdx.x * kWarps + (threadIdx.x >> 5), nw = gridDim.x * kWarps;
     unsigned long long* keys = gkeys + (size_t)gw * cap;
     for (int i = gw; i < *n_over; i += nw) {
         const int q = ovlist[i];
         const int K = qk ? qk[q] : K_all;
         unsigned long long result;
-        kth_search(pg, xf1 + 3 * (size_t)q, xf2, q, K, self, keys, cap, &cnt[w], lane, result);
+        kth_search(pg, xf1 + 3 * (size_t)q, xf2, q, K, self, keys, cap, lane, result);
         if (lane == 0) kth[q] = result;
         __syncwarp();
     }
@@ -208,6 +264,11 @@ __global__ void k_first_cells(DG bg, const float* __restrict__ box2, int n2, int
     }
 }
 
+// Most keys of a query that its warp orders itself: ranking n keys takes n^2 / 32
+// broadcast loads.  The segmented sort is three launches, a host synchronisation
+// between them, and k_cand_finish.
+constexpr int kRankMost = 512;
+
 // The cells of the scan range are taken 32 at a time, one per lane; their
 // item counts are prefix-summed across the warp and the lanes then stride
 // over the items of all 32 cells together (each lane finds its item's cell by
@@ -221,7 +282,8 @@ __global__ void __launch_bounds__(256) k_cand_pass(DG bg, const float* __restric
                                                    const float* __restrict__ qtau, int isect,
                                                    const unsigned long long* __restrict__ kth,
                                                    int64_t* __restrict__ cnt, const int64_t* __restrict__ off,
-                                                   unsigned long long* __restrict__ keys, int qb0, int qe0) {
+                                                   unsigned long long* __restrict__ keys, int qb0, int qe0,
+                                                   int* __restrict__ most, int* __restrict__ pq, int* __restrict__ pt) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -302,7 +364,23 @@ __global__ void __launch_bounds__(256) k_cand_pass(DG bg, const float* __restric
                 count += __popc(m);
             }
         }
-        if (!WRITE && lane == 0) cnt[q] = count;
+        if (!WRITE && lane == 0) {
+            cnt[q] = count;
+            if (count > *most) atomicMax(most, (int)min(count, (int64_t)INT_MAX));
+        }
+        if (WRITE && pq) {  // order the keys: they are distinct
+            __syncwarp();
+            const unsigned long long* k = keys + off[q];
+            for (int i = lane; i < (int)count; i += 32) {
+                const unsigned long long key = k[i];
+                int rank = 0;
+#pragma unroll 4
+                for (int j = 0; j < (int)count; ++j) rank += k[j] < key;
+                pq[off[q] + rank] = q;
+                pt[off[q] + rank] = (int)(key & 0xffffffffull);
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -390,7 +468,7 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
     int* d_over = (int*)(ctx->d_counter + 40);
     Buf& ovb = ctx->scratch[89];
     if ((rc = ensure(ctx, ovb, (size_t)(n1 + 1) * 4))) return rc;
-    CU(cudaMemsetAsync(d_over, 0, 4, s));
+    CU(cudaMemsetAsync(d_over, 0, 8, s));  // [0] ring searches to redo, [1] most candidates of a query
     const DG bg = dg(t2->box_grid), pg = dg(t2->point_grid);
     unsigned long long* kth = (unsigned long long*)kthb.p;
     const bool any_knn = knn || qk;
@@ -412,19 +490,20 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
     int64_t* qoff = (int64_t*)qoff_buf.p;
     const int pblocks = (int)std::min<long>((n1 + 7) / 8, (long)ctx->num_sms * 32);
     int64_t total = 0;
-    int over = 0;
+    int found[2] = {0, 0};
+    const int& over = found[0];
     for (int pass = 0;; ++pass) {
         CU(cudaMemsetAsync(cnt + n1, 0, 8, s));
         k_cand_pass<false><<<std::max(pblocks, 1), 256, 0, s>>>(bg, box1, xf1, box2, xf2, fc, (int)n1, self, knn, tau,
                                                                qk, qtau, isect ? 1 : 0, kth, cnt, nullptr, nullptr,
-                                                               (int)qb0, (int)qe0);
+                                                               (int)qb0, (int)qe0, d_over + 1, nullptr, nullptr);
         CU(cudaGetLastError());
         size_t tb = 0;
         CU(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, qoff, (int)n1 + 1, s));
         if ((rc = ensure(ctx, tmp, tb + 16))) return rc;
         CU(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt, qoff, (int)n1 + 1, s));
         CU(cudaMemcpyAsync(&total, qoff + n1, 8, cudaMemcpyDeviceToHost, s));
-        CU(cudaMemcpyAsync(&over, d_over, 4, cudaMemcpyDeviceToHost, s));
+        CU(cudaMemcpyAsync(found, d_over, 8, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
         if (!over || pass > 0) break;
         // Some kNN ring searches saw more points than a warp's shared-memory
@@ -440,6 +519,7 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
             pg, xf1, xf2, K, self, qk, kth, d_over, (const int*)ovb.p, (unsigned long long*)gk.p, (int)cap);
         CU(cudaGetLastError());
         n_redone = over;
+        CU(cudaMemsetAsync(d_over + 1, 0, 4, s));  // counted again
     }
     if (total >= (1LL << 31) - 1) return fail(ctx, TDP_ERR_ARG, "too many candidate pairs");
     P = (long)total;
@@ -449,10 +529,13 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
     if ((rc = ensure(ctx, pq_buf, Pz * 4))) return rc;
     if ((rc = ensure(ctx, pt_buf, Pz * 4))) return rc;
     if (P > 0) {
+        const bool ranked = found[1] <= kRankMost;
         k_cand_pass<true><<<std::max(pblocks, 1), 256, 0, s>>>(bg, box1, xf1, box2, xf2, fc, (int)n1, self, knn, tau, qk, qtau, isect ? 1 : 0, kth,
                                                               nullptr, qoff, (unsigned long long*)keys.p, (int)qb0,
-                                                              (int)qe0);
+                                                              (int)qe0, nullptr, ranked ? (int*)pq_buf.p : nullptr,
+                                                              (int*)pt_buf.p);
         CU(cudaGetLastError());
+        if (ranked) return TDP_OK;
         size_t sb = 0;
         CU(cub::DeviceSegmentedSort::SortKeys(nullptr, sb, (const unsigned long long*)keys.p,
                                               (unsigned long long*)keys2.p, (int)P, (int)n1, qoff, qoff + 1, s));
