@@ -20,15 +20,35 @@ void cache_trim(tdp_ctx* ctx) {
     ctx->small_cached = 0;
 }
 
+bool lod_scratch_drop(tdp_ctx* ctx) {
+    if (ctx->lod_busy) return false;
+    bool any = false;
+    for (int k = kLodScratchFirst; k < kLodScratchEnd; ++k) {
+        Buf& b = ctx->scratch[k];
+        if (!b.p) continue;
+        if (!any) cudaStreamSynchronize(ctx->stream);
+        any = true;
+        dfree(ctx, b.p);
+        b = Buf{};
+    }
+    return any;
+}
+
 cudaError_t dmalloc(tdp_ctx* ctx, void** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
-    if (ctx->budget && ctx->in_use + bytes > ctx->budget) return cudaErrorMemoryAllocation;
+    if (ctx->budget && ctx->in_use + bytes > ctx->budget &&
+        (!lod_scratch_drop(ctx) || ctx->in_use + bytes > ctx->budget))
+        return cudaErrorMemoryAllocation;
     if (ctx->budget && ctx->in_use + ctx->cached_bytes + bytes > ctx->budget) cache_trim(ctx);
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess && !ctx->block_cache.empty()) {  // the cache holds the memory: give it back, retry
         cudaGetLastError();
         cache_trim(ctx);
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess && lod_scratch_drop(ctx)) {
+        cudaGetLastError();
         e = cudaMalloc(p, bytes);
     }
     if (e != cudaSuccess) { *p = nullptr; return e; }

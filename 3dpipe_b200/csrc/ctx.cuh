@@ -65,6 +65,7 @@ struct tdp_ctx {
     std::unordered_map<void*, size_t> allocs;
     tdp::Buf scratch[120];  // slots: refine-batch 0-4, tile upload 12-13, join 20-48, candidates 50-59 and 88-90, result sort 60-63, exact distances 64-81 and 84-86, per-object queries 82-83, last-LOD presets 91, GPU attach pass 96-100, LOD task form 101-117
     unsigned* d_counter = nullptr;            // work counters (device)
+    bool lod_busy = false;                    // the LOD task scratch is in use (LodScratchUse)
     unsigned long long* d_stats = nullptr;    // device-side statistics
     tdp::LastStats stats;
     int tuned_cfg = 0;  // tuned refine kernel configuration (tdp_set_refine_config / tdp_autotune)
@@ -116,6 +117,17 @@ constexpr size_t kSmallCached = 512;
 cudaError_t block_alloc(tdp_ctx* ctx, void** p, size_t bytes);
 void block_release(tdp_ctx* ctx, void* p);
 void cache_trim(tdp_ctx* ctx);
+
+// Scratch of the LOD loop's task form (and of the exact stage's).  Its queues
+// are large, and only a speed-up: an allocation that would fail otherwise takes
+// them back while no join is between their set-up and its last use of them.
+constexpr int kLodScratchFirst = 101, kLodScratchEnd = 118;
+bool lod_scratch_drop(tdp_ctx* ctx);
+struct LodScratchUse {
+    tdp_ctx* ctx;
+    explicit LodScratchUse(tdp_ctx* c) : ctx(c) { c->lod_busy = true; }
+    ~LodScratchUse() { ctx->lod_busy = false; }
+};
 
 enum ScratchSlot {
     kSlotRawData = 0, kSlotRawHd, kSlotTris, kSlotItems, kSlotOut,

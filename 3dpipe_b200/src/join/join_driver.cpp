@@ -49,7 +49,7 @@ enum Slot {
     kPexOut = 76, kOutD64,            // exact distances (64-75 and 78-81 are the exact stage's own)
     kQk = 82, kQtau,                  // per query object queries
     kPreset = 91,                     // the last LOD's item presets (within queries)
-    kLodExt = 101, kLodVox, kLodMg, kLodCaps, kLodFlags, kLodZero, kLodVres, kLodCl1, kLodCl2, kLodVb1, kLodVb2,
+    kLodExt = kLodScratchFirst, kLodVox, kLodMg, kLodCaps, kLodFlags, kLodZero, kLodVres, kLodCl1, kLodCl2, kLodVb1, kLodVb2,
     kLodLists, kLodTasks, kLodOver, kLodEvals, kLodBest, kLodDir,   // the LOD loop's task form
 };
 
@@ -525,6 +525,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         for (int k = 0; k < 16; ++k) L.pf[k] = ctx->pf_ev[k];
         L.tasks = 1;
         for (int k = 0; k < L.nl; ++k) L.tasks = L.tasks && L.cfg[k] == 0;
+        LodScratchUse in_use(ctx);
         if (L.tasks) {
             LodDev& t = L.t;
             size_t c1 = 0, c2 = 0;  // cluster records of a LOD: at most one per 8 triangles and one more per voxel
@@ -540,13 +541,25 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             L.best_bytes = Pz * 8;
             L.flags_bytes = (nv1 + nv2) * 4;
             L.zero_bytes = ctr_bytes + 2 * Pz;
-            ENS(kLodExt, Vz * sizeof(int4)); ENS(kLodVox, Vz * sizeof(int2)); ENS(kLodMg, Vz * sizeof(float4));
-            ENS(kLodCaps, L.caps_bytes); ENS(kLodBest, L.best_bytes); ENS(kLodDir, 2 * L.best_bytes); ENS(kLodFlags, L.flags_bytes); ENS(kLodZero, L.zero_bytes);
-            ENS(kLodVres, Vz * 4); ENS(kLodCl1, c1 * 3 * sizeof(float4)); ENS(kLodVb1, nv1 * 2 * sizeof(float4));
-            if (!self) { ENS(kLodCl2, c2 * 3 * sizeof(float4)); ENS(kLodVb2, nv2 * 2 * sizeof(float4)); }
-            ENS(kLodLists, (nv1 + nv2) * 4); ENS(kLodOver, Vz * 4);
-            ENS(kLodTasks, (size_t)t.task_cap * sizeof(LodTask));
-            ENS(kLodEvals, (size_t)t.eval_cap * sizeof(LodEval));
+            const struct { int slot; size_t bytes; } need[] = {
+                {kLodExt, Vz * sizeof(int4)}, {kLodVox, Vz * sizeof(int2)}, {kLodMg, Vz * sizeof(float4)},
+                {kLodCaps, L.caps_bytes}, {kLodBest, L.best_bytes}, {kLodDir, 2 * L.best_bytes},
+                {kLodFlags, L.flags_bytes}, {kLodZero, L.zero_bytes}, {kLodVres, Vz * 4},
+                {kLodCl1, c1 * 3 * sizeof(float4)}, {kLodVb1, nv1 * 2 * sizeof(float4)},
+                {kLodCl2, self ? 0 : c2 * 3 * sizeof(float4)}, {kLodVb2, self ? 0 : nv2 * 2 * sizeof(float4)},
+                {kLodLists, (nv1 + nv2) * 4}, {kLodOver, Vz * 4}, {kLodTasks, (size_t)t.task_cap * sizeof(LodTask)},
+                {kLodEvals, (size_t)t.eval_cap * sizeof(LodEval)}};
+            for (const auto& n : need)
+                if (n.bytes && L.tasks && ensure(ctx, ctx->scratch[n.slot], n.bytes) != TDP_OK) L.tasks = 0;
+        }
+        if (!L.tasks) {  // no room for the queues: the refine of one warp per voxel pair
+            cudaGetLastError();
+            std::memset(&L.t, 0, sizeof L.t);
+            L.caps_bytes = L.best_bytes = L.flags_bytes = L.zero_bytes = 0;
+        } else {
+            LodDev& t = L.t;
+            const size_t nv1 = (size_t)std::max<long>(t1->n_vox, 1), nv2 = self ? 0 : (size_t)std::max<long>(t2->n_vox, 1);
+            const size_t ctr_bytes = kLodCtrWords * kMaxPasses * sizeof(unsigned);
             t.d = d;
             t.box1 = t1->d_boxes; t.box2 = t2->d_boxes;
             t.self = self ? 1 : 0; t.level = prm->hausdorff_level; t.nl = L.nl;
