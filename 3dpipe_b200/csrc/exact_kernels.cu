@@ -9,25 +9,36 @@
 //      LOD-100 surface), and, at Hausdorff level 2, also the pair's upper
 //      bound pmx when it was decided (d + h1 + h2 at a lower LOD bounds D);
 //      each widened by its FP32 error, max(perr, 1e-4 (value + 1));
-//      U is then tightened by refining, in FP32, the voxel pair with the
-//      closest cores (kExK per object pair): its minimum d32 + err_bound(R)
-//      is a distance between two surface points, hence also >= D;
+//      U is then tightened by the FP32 distances of some triangle pairs of the
+//      voxel pair with the closest cores (k_exact_seed): d32 + err_bound(R) is
+//      a distance between two surface points, hence also >= D;
 //   2. every LOD-100 voxel pair whose box gap is <= U is a candidate (the
 //      voxel pair holding the closest points has gap <= D <= U);
-//   3. the tuned FP32 refine, its minimum preset to U plus the candidate's
+//   3. the candidates go through the task kernels of the LOD loop's last LOD
+//      (lod_kernels.cu) with U as the pair's first cap: cluster pairs, then
+//      triangle pairs, whose FP32 gap is not below the pair's running minimum
+//      by more than its error are left out, the others are evaluated in FP32;
+//   4. of those, again a triangle pair a lane, the ones whose FP32 distance less
+//      its error is within the pair's final minimum and error are evaluated in
+//      FP64 (candidates that found a queue full: all their triangle pairs that
+//      pass the same tests);
+//   5. D = the smallest of them.
+// 905 reported pairs, 52,584 candidates: 1.59 -> 0.42 ms against one warp per
+// candidate with its own FP32 minimum (the lazy refine: 406 us for 905
+// closest-core voxel pairs, 520 for the candidates left by an item-level test
+// of 77, and 343 for FP64 over those voxel pairs again).  That form remains for
+// contexts without room for the queues: there
+//   3'. the lazy FP32 refine, its minimum preset to U plus the candidate's
 //      largest possible FP32 error, gives each candidate that has a triangle
-//      pair below that preset its minimum d32 (error e = err_bound(R)) and
-//      skips the rest after a few cluster tests (sphere and cylinder bounds);
-//      per object pair best32 =
-//      min d32 and E = max e;
-//   4. a candidate can hold the minimum only if d32 - E <= best32 + E (its
+//      pair below that preset its minimum d32 (error e = err_bound(R)); per
+//      object pair best32 = min d32 and E = max e;
+//   4'. a candidate can hold the minimum only if d32 - E <= best32 + E (its
 //      true minimum is >= d32 - e, and D <= best32 + E): those are evaluated
 //      again triangle pair by triangle pair, skipping pairs whose (inflated)
 //      bounding-sphere gap or cylinder bound exceeds best32 + 2E; a pair's
 //      FP32 distance d32'
 //      with its error e' comes first, and only a pair with d32' - e' <=
-//      best32 + E (one that can be the minimum) is evaluated in FP64;
-//   5. D = the smallest FP64 distance over the evaluated candidates.
+//      best32 + E (one that can be the minimum) is evaluated in FP64.
 // Every filter is conservative, so D is the exact minimum over the stored
 // float coordinates up to the FP64 rounding of one triangle distance.
 #include <cub/device/device_scan.cuh>
@@ -39,6 +50,7 @@
 
 #include "exact_kernels.cuh"
 #include "cull.cuh"
+#include "lod_kernels.cuh"
 #include "refine.cuh"
 #include "tridist.cuh"
 
@@ -47,14 +59,12 @@ namespace {
 
 constexpr int kBlk = 256;
 
-// Voxel pairs per object pair refined in FP32 to tighten U (the ones with
-// the closest cores).  On the within-400 join eight cost 8x the FP32 work of
-// one and left the candidate set 1.4 % smaller (28.0 M voxel pairs against
-// 28.4 M); the two with the smallest box gaps instead gave a looser U (29.6 M
-// candidates, 15 % more FP32 work); so one is refined.
+// Closest-core voxel pairs per object pair that tighten U.  On the within-400
+// join eight left the candidate set 1.4 % smaller (28.0 M voxel pairs against
+// 28.4 M) for eight times the work.
 constexpr int kExK = 1;
 
-// The FP32 passes run the lazy refine with the cylinder bound in its culls
+// The lazy form's FP32 pass runs the lazy refine with the cylinder bound in its culls
 // (configuration 16): a reported pair's closest points face each other across
 // a gap of up to tau, where the sphere gap keeps every triangle pair whose
 // centres are offset sideways by less than about sqrt(2 gap (r1 + r2)).
@@ -139,15 +149,82 @@ __global__ void __launch_bounds__(kBlk) k_exact_upper(JoinDev d, int pmx_valid, 
     }
 }
 
-// U = min(U, d32 + err) over the FP32 minima of the kExK closest-core voxel pairs
-__global__ void k_exact_tighten(const float4* __restrict__ res1, int64_t P, float* __restrict__ U) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < P; p += (int64_t)gridDim.x * blockDim.x) {
-        float u = U[p];
-        for (int k = 0; k < kExK; ++k) {
-            const float4 r = res1[(size_t)kExK * p + k];
-            if (r.x < FLT_MAX) u = fminf(u, r.x + err_bound(r.w) + 1e-5f * r.x + 1e-6f);
+// the FP32 operands as the refine forms them (translated to o), and the
+// largest |coordinate| after translation (the R of the error model)
+__device__ __forceinline__ float pre32(const float4* t, float4 o, PreTri<float>& P) {
+    const float4 a = t[0], b = t[1], c = t[2];
+    const V3<float> x = v3<float>(a.x - o.x, a.y - o.y, a.z - o.z), y = v3<float>(b.x - o.x, b.y - o.y, b.z - o.z),
+                    z = v3<float>(c.x - o.x, c.y - o.y, c.z - o.z);
+    pretri(P, x, y, z);
+    float r = 0.f;
+    r = fmaxf(r, fmaxf(fabsf(x.x), fmaxf(fabsf(x.y), fabsf(x.z))));
+    r = fmaxf(r, fmaxf(fabsf(y.x), fmaxf(fabsf(y.y), fabsf(y.z))));
+    return fmaxf(r, fmaxf(fabsf(z.x), fmaxf(fabsf(z.y), fabsf(z.z))));
+}
+
+// U = min(U, d32 + err) over some triangle pairs of the pair's closest-core
+// voxel pair, one warp a pair: the nearest triangles of A and of B to each
+// other by their middles, found by turns, and the 64 pairs of one of them with
+// every lane's nearest of the other side.  dir = from the best pair's A to its
+// B triangle.  Any triangle pair bounds the distance; the voxel pair's full
+// FP32 minimum instead (the lazy refine, one warp an item) gave a U hardly
+// smaller and took 406 us for 905 pairs of 100-triangle voxels; this takes 14.
+__global__ void __launch_bounds__(128) k_exact_seed(const float4* __restrict__ triA, const float4* __restrict__ triB,
+                                                    const RefineItem* __restrict__ item1, int64_t P,
+                                                    float* __restrict__ U, float4* __restrict__ dir) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < P; p += nw) {
+        const RefineItem it = item1[p];
+        if (it.a_cnt == 0 || it.b_cnt == 0) {
+            if (lane == 0) dir[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+            continue;
         }
-        U[p] = u;
+        const float4* tA = triA + (size_t)it.a_off * kTriF4;
+        const float4* tB = triB + (size_t)it.b_off * kTriF4;
+        const float4 o4 = tA[0];
+        // three times the middle of a triangle, relative to o4
+        auto mid = [&](const float4* t) {
+            const float4 a = t[0], b = t[1], c = t[2];
+            return make_float3((a.x - o4.x) + (b.x - o4.x) + (c.x - o4.x), (a.y - o4.y) + (b.y - o4.y) + (c.y - o4.y),
+                               (a.z - o4.z) + (b.z - o4.z) + (c.z - o4.z));
+        };
+        // the lane's and the warp's nearest triangle to m (no finite distance: the first)
+        auto nearest = [&](const float4* t, uint32_t n, float3 m, uint32_t& mine) {
+            float best = INFINITY;
+            mine = (uint32_t)lane < n ? lane : 0u;
+            for (uint32_t i = lane; i < n; i += 32) {
+                const float3 c = mid(t + (size_t)i * kTriF4);
+                const float dx = c.x - m.x, dy = c.y - m.y, dz = c.z - m.z, d2 = dx * dx + dy * dy + dz * dz;
+                if (d2 < best) { best = d2; mine = i; }
+            }
+            const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(best));
+            const unsigned who = __ballot_sync(0xffffffffu, __float_as_uint(best) == least);
+            return __shfl_sync(0xffffffffu, mine, __ffs(who) - 1);
+        };
+        uint32_t ia = 0, ib = 0, la = 0, lb = 0;
+        for (int turn = 0; turn < 2; ++turn) {
+            ia = nearest(tA, it.a_cnt, mid(tB + (size_t)ib * kTriF4), la);
+            ib = nearest(tB, it.b_cnt, mid(tA + (size_t)ia * kTriF4), lb);
+        }
+        float u = INFINITY;
+        uint32_t ba = ia, bb = ib;
+        for (int side = 0; side < 2; ++side) {
+            const uint32_t i = side ? ia : la, j = side ? lb : ib;
+            PreTri<float> A, B;
+            const float rA = pre32(tA + (size_t)i * kTriF4, o4, A);
+            const float rB = pre32(tB + (size_t)j * kTriF4, o4, B);
+            const float d = sqrtf(tri_dist2(A, B));
+            const float x = d + err_bound(fmaxf(rA, rB)) + 1e-5f * d + 1e-6f;
+            if (x < u) { u = x; ba = i; bb = j; }
+        }
+        const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(u));
+        const unsigned who = __ballot_sync(0xffffffffu, __float_as_uint(u) == least);
+        if (lane == __ffs(who) - 1) {
+            if (u < U[p]) U[p] = u;
+            const float3 a = mid(tA + (size_t)ba * kTriF4), b = mid(tB + (size_t)bb * kTriF4);
+            dir[p] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, 0.f);
+        }
     }
 }
 
@@ -160,21 +237,28 @@ __device__ __forceinline__ float box_gap2(const float4* a, const float4* b) {
     return gx * gx + gy * gy + gz * gz;
 }
 
-// count (WRITE = false) or write the candidate voxel pairs of every reported pair
-// The preset of a candidate is U plus the largest FP32 error its minimum can
-// carry: err_bound of a coordinate bound R <= gap + both voxel diagonals, as
-// every coordinate is taken relative to a vertex of the A voxel.
-template <bool WRITE>
+// Candidate voxel pairs of every reported pair (one warp a pair): counted, or
+// written as items of the lazy pass or of the task pass.  The B voxels are first
+// held against the box of all the A voxels, 32 at a time; of those near it every
+// pair with an A voxel is tested, one a lane.
+// An item of the lazy pass has a preset: U plus the largest FP32 error its
+// minimum can carry: err_bound of a coordinate bound R <= gap + both voxel
+// diagonals, as every coordinate is taken relative to a vertex of the A voxel.
+enum class Vp { kCount, kLazy, kTasks };
+
+template <Vp OUT>
 __global__ void __launch_bounds__(kBlk) k_exact_vp(JoinDev d, const float* __restrict__ Ub,
                                                    const uint32_t* __restrict__ vt1,
                                                    const uint32_t* __restrict__ vt2, int64_t* __restrict__ cnt,
                                                    const int64_t* __restrict__ off, RefineItem* __restrict__ items,
-                                                   int* __restrict__ item_pair, float* __restrict__ preset) {
+                                                   int* __restrict__ item_pair, float* __restrict__ preset, LodDev L) {
+    __shared__ uint32_t lists[kBlk / 32][32];
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
+    uint32_t* list = lists[threadIdx.x >> 5];
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < d.P; p += nw) {
         if (d.pstat[p] != kReported) {
-            if (!WRITE && lane == 0) cnt[p] = 0;
+            if (OUT == Vp::kCount && lane == 0) cnt[p] = 0;
             continue;
         }
         const int q = d.pq[p], t = d.pt[p];
@@ -183,35 +267,70 @@ __global__ void __launch_bounds__(kBlk) k_exact_vp(JoinDev d, const float* __res
         const float U = Ub[p];
         const float lim = U * (1.f + 1e-5f) + 1e-6f;
         const float lim2 = lim * lim;
-        const uint64_t total = (uint64_t)n1 * n2;
-        int64_t pos = WRITE ? off[p] : 0, count = 0;
-        for (uint64_t base = 0; base < total; base += 32) {
-            const uint64_t k = base + lane;
-            bool keep = false;
-            uint32_t a = 0, b = 0;
-            if (k < total) {
-                a = a0 + (uint32_t)(k / n2);
-                b = b0 + (uint32_t)(k % n2);
-                keep = box_gap2(d.vox1 + 3 * (size_t)a, d.vox2 + 3 * (size_t)b) <= lim2 && vt1[a + 1] > vt1[a] &&
-                       vt2[b + 1] > vt2[b];
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            if (WRITE && keep) {
-                const int64_t w = pos + __popc(bal & ((1u << lane) - 1u));
-                items[w] = RefineItem{vt1[a], vt1[a + 1] - vt1[a], vt2[b], vt2[b + 1] - vt2[b]};
-                item_pair[w] = p;
-                const float4* va = d.vox1 + 3 * (size_t)a;
-                const float4* vb = d.vox2 + 3 * (size_t)b;
-                const float4 alo = va[0], ahi = va[1], blo = vb[0], bhi = vb[1];
-                const float da = (ahi.x - alo.x) + (ahi.y - alo.y) + (ahi.z - alo.z);
-                const float db = (bhi.x - blo.x) + (bhi.y - blo.y) + (bhi.z - blo.z);
-                const float R = (U + da + db) * 1.001f + 1.f;
-                preset[w] = U + 2.f * err_bound(R) + 1e-6f;
-            }
-            pos += __popc(bal);
-            count += __popc(bal);
+        float4 all[2] = {make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f)};
+        for (uint32_t a = lane; a < n1; a += 32) {
+            const float4 lo = d.vox1[3 * (size_t)(a0 + a)], hi = d.vox1[3 * (size_t)(a0 + a) + 1];
+            all[0] = make_float4(fminf(all[0].x, lo.x), fminf(all[0].y, lo.y), fminf(all[0].z, lo.z), 0.f);
+            all[1] = make_float4(fmaxf(all[1].x, hi.x), fmaxf(all[1].y, hi.y), fmaxf(all[1].z, hi.z), 0.f);
         }
-        if (!WRITE && lane == 0) cnt[p] = count;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            all[0].x = fminf(all[0].x, __shfl_xor_sync(0xffffffffu, all[0].x, o));
+            all[0].y = fminf(all[0].y, __shfl_xor_sync(0xffffffffu, all[0].y, o));
+            all[0].z = fminf(all[0].z, __shfl_xor_sync(0xffffffffu, all[0].z, o));
+            all[1].x = fmaxf(all[1].x, __shfl_xor_sync(0xffffffffu, all[1].x, o));
+            all[1].y = fmaxf(all[1].y, __shfl_xor_sync(0xffffffffu, all[1].y, o));
+            all[1].z = fmaxf(all[1].z, __shfl_xor_sync(0xffffffffu, all[1].z, o));
+        }
+        int64_t pos = OUT != Vp::kCount ? off[p] : 0, count = 0;
+        for (uint32_t c0 = 0; c0 < n2; c0 += 32) {
+            // (the gap to the larger box rounds to no more than any A voxel's: every step of it is monotone)
+            const uint32_t bl = b0 + c0 + lane;
+            const bool near = c0 + lane < n2 && !(box_gap2(all, d.vox2 + 3 * (size_t)bl) > lim2) && vt2[bl + 1] > vt2[bl];
+            const unsigned nm = __ballot_sync(0xffffffffu, near);
+            if (!nm) continue;
+            __syncwarp();
+            if (near) list[__popc(nm & ((1u << lane) - 1u))] = bl;
+            __syncwarp();
+            const uint64_t total = (uint64_t)__popc(nm) * n1;
+            for (uint64_t base = 0; base < total; base += 32) {
+                const uint64_t k = base + lane;
+                bool keep = false;
+                uint32_t a = 0, b = 0;
+                if (k < total) {
+                    const uint32_t i = (uint32_t)(k / n1);
+                    a = a0 + (uint32_t)(k - (uint64_t)i * n1);
+                    b = list[i];
+                    keep = box_gap2(d.vox1 + 3 * (size_t)a, d.vox2 + 3 * (size_t)b) <= lim2 && vt1[a + 1] > vt1[a];
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, keep);
+                if (OUT != Vp::kCount && keep) {
+                    const int64_t w = pos + __popc(bal & ((1u << lane) - 1u));
+                    items[w] = RefineItem{vt1[a], vt1[a + 1] - vt1[a], vt2[b], vt2[b + 1] - vt2[b]};
+                    if (OUT == Vp::kTasks) {
+                        L.ext[w] = make_int4((int)w, p, (int)cluster_base(vt1[a], (int)a), (int)cluster_base(vt2[b], (int)b));
+                        L.vox[w] = make_int2((int)a, (int)b);
+                    } else {
+                        item_pair[w] = p;
+                        const float4* va = d.vox1 + 3 * (size_t)a;
+                        const float4* vb = d.vox2 + 3 * (size_t)b;
+                        const float4 alo = va[0], ahi = va[1], blo = vb[0], bhi = vb[1];
+                        const float da = (ahi.x - alo.x) + (ahi.y - alo.y) + (ahi.z - alo.z);
+                        const float db = (bhi.x - blo.x) + (bhi.y - blo.y) + (bhi.z - blo.z);
+                        const float R = (U + da + db) * 1.001f + 1.f;
+                        preset[w] = U + 2.f * err_bound(R) + 1e-6f;
+                    }
+                }
+                if (OUT == Vp::kTasks && bal) {
+                    lod_claim(keep, (int)a, 0, L.flag1, L.list1, L.ctr + cList1, lane);
+                    if (L.self) lod_claim(keep, (int)b, 0, L.flag1, L.list1, L.ctr + cList1, lane);
+                    else lod_claim(keep, (int)b, 0, L.flag2, L.list2, L.ctr + cList2, lane);
+                }
+                pos += __popc(bal);
+                count += __popc(bal);
+            }
+        }
+        if (OUT == Vp::kCount && lane == 0) cnt[p] = count;
     }
 }
 
@@ -369,19 +488,6 @@ __device__ __forceinline__ void pre64(const float4* t, double ox, double oy, dou
            v3<double>(c.x - ox, c.y - oy, c.z - oz));
 }
 
-// the FP32 operands as the refine forms them (translated to o), and the
-// largest |coordinate| after translation (the R of the error model)
-__device__ __forceinline__ float pre32(const float4* t, float4 o, PreTri<float>& P) {
-    const float4 a = t[0], b = t[1], c = t[2];
-    const V3<float> x = v3<float>(a.x - o.x, a.y - o.y, a.z - o.z), y = v3<float>(b.x - o.x, b.y - o.y, b.z - o.z),
-                    z = v3<float>(c.x - o.x, c.y - o.y, c.z - o.z);
-    pretri(P, x, y, z);
-    float r = 0.f;
-    r = fmaxf(r, fmaxf(fabsf(x.x), fmaxf(fabsf(x.y), fabsf(x.z))));
-    r = fmaxf(r, fmaxf(fabsf(y.x), fmaxf(fabsf(y.y), fabsf(y.z))));
-    return fmaxf(r, fmaxf(fabsf(z.x), fmaxf(fabsf(z.y), fabsf(z.z))));
-}
-
 constexpr int kExWarps = 4;
 constexpr int kExQueue = 64;  // queued triangle pairs per warp (>= 32 + 31)
 
@@ -409,23 +515,19 @@ __device__ __forceinline__ double exact_pair(const float4* ta, const float4* tb,
 // spheres (staged in shared memory); the pairs that pass are queued, and
 // every 32 queued pairs are evaluated one per lane, so the evaluations run
 // with the whole warp instead of with the few lanes whose test passed.
-__global__ void __launch_bounds__(kExWarps * 32) k_exact_f64(const float4* __restrict__ triA,
-                                                             const float4* __restrict__ triB,
-                                                             const RefineItem* __restrict__ sel,
-                                                             const int* __restrict__ sel_pair,
-                                                             const float2* __restrict__ sel_thr,
-                                                             const unsigned* __restrict__ n_sel,
-                                                             unsigned long long* __restrict__ pexact_bits) {
+template <typename Get>
+__device__ __forceinline__ void exact_items_f64(const float4* __restrict__ triA, const float4* __restrict__ triB,
+                                                unsigned n, unsigned long long* __restrict__ pexact_bits, Get get) {
     __shared__ float4 sphA[kExWarps][32];
     __shared__ float2 prjA[kExWarps][32];
     __shared__ uint2 queue[kExWarps][kExQueue];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    const unsigned n = *n_sel;
     uint2* q = queue[w];
     for (unsigned it = blockIdx.x * kExWarps + w; it < n; it += gridDim.x * kExWarps) {
-        const RefineItem r = sel[it];
-        const float2 tl = sel_thr[it];
+        RefineItem r;
+        float2 tl;
+        const int p = get(it, r, tl);
         const float thr = tl.x, lim = tl.y;
         const float4 o4 = triA[(size_t)r.a_off * kTriF4];
         const float4* tA = triA + (size_t)r.a_off * kTriF4;
@@ -496,8 +598,38 @@ __global__ void __launch_bounds__(kExWarps * 32) k_exact_f64(const float4* __res
         }
         // non-negative doubles order like their bit patterns
         if (lane == 0 && best < 1e300)
-            atomicMin(pexact_bits + sel_pair[it], (unsigned long long)__double_as_longlong(sqrt(best)));
+            atomicMin(pexact_bits + p, (unsigned long long)__double_as_longlong(sqrt(best)));
     }
+}
+
+__global__ void __launch_bounds__(kExWarps * 32) k_exact_f64(const float4* __restrict__ triA,
+                                                             const float4* __restrict__ triB,
+                                                             const RefineItem* __restrict__ sel,
+                                                             const int* __restrict__ sel_pair,
+                                                             const float2* __restrict__ sel_thr,
+                                                             const unsigned* __restrict__ n_sel,
+                                                             unsigned long long* __restrict__ pexact_bits) {
+    exact_items_f64(triA, triB, *n_sel, pexact_bits, [&](unsigned it, RefineItem& r, float2& tl) {
+        r = sel[it];
+        tl = sel_thr[it];
+        return sel_pair[it];
+    });
+}
+
+// the task pass's items that found a queue full
+__global__ void __launch_bounds__(kExWarps * 32) k_exact_over_f64(LodDev L, unsigned long long* __restrict__ pexact_bits,
+                                                                  unsigned* __restrict__ n_f64) {
+    exact_items_f64(L.tri1[0], L.tri2[0], L.ctr[cOver], pexact_bits, [&](unsigned it, RefineItem& r, float2& tl) {
+        const unsigned w = L.over[it];
+        const int p = L.ext[w].y;
+        const float4 g = L.mg[w];
+        r = L.items[w];
+        tl.y = fminf(L.pd[p], L.pcap[p]) + g.y;
+        tl.x = tl.y + g.x;
+        // counted once: the queued triangle pairs of the item may have been evaluated too
+        if ((threadIdx.x & 31) == 0 && !(atomicOr((int*)&L.mg[w].w, kExactFlag) & kExactFlag)) atomicAdd(n_f64, 1u);
+        return p;
+    });
 }
 
 // largest |best32 - D| / max(D, 1) over the reported pairs: the FP32 refine's
@@ -519,6 +651,84 @@ int grid(int64_t n, int per_block, int cap) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(g, cap));
 }
 
+// the counters of a finished stage (dropped: items that never reached the pass)
+int read_info(tdp_ctx* ctx, const unsigned* ctr, long dropped, ExactInfo& info) {
+    unsigned ns[12] = {0};
+    cudaError_t e = cudaMemcpyAsync(ns, ctr + 4, 48, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, TDP_ERR_CUDA, std::string("exact-distance stage: ") + cudaGetErrorString(e));
+    info.f64_items = ns[0];
+    float e32;
+    std::memcpy(&e32, &ns[4], 4);
+    info.max_rel_err32 = e32;
+    std::memcpy(&info.full_evals, &ns[8], 8);
+    info.dropped_items = dropped + (long)ns[10];
+    info.below_items = ns[11];
+    for (int k = 0; k < 4; ++k) {
+        float ms = 0;
+        cudaEventElapsedTime(&ms, ctx->xev[k], ctx->xev[k + 1]);
+        info.phase_ms[k] = ms;
+    }
+    return TDP_OK;
+}
+
+// Candidates that go through the task queues at a time: those hold 16 cluster
+// pairs and 8 triangle pairs a candidate (128 and 64 MB), about twice what the
+// joins measured here bring.
+constexpr int64_t kChunk = 1 << 19;
+
+// Scratch of the task pass over L.d.V candidates (the LOD loop's, and this
+// stage's own slots); false when it does not fit.
+bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t2, size_t Pz) {
+    if (!t1->d_boxes || !t2->d_boxes) return false;
+    enum { kCl1 = kLodScratchFirst + 7, kCl2, kVb1, kVb2, kLists, kTasks, kOver, kEvals, kFlags = kLodScratchFirst + 4,
+           kCtr = kLodScratchFirst + 5 };  // the LOD loop's slots
+    const size_t E = (size_t)L.d.V;
+    L.self = t1 == t2;
+    L.nl = 1;
+    L.li[0] = kNumLods - 1;
+    L.vt1[0] = t1->vtri[kNumLods - 1];
+    L.vt2[0] = t2->vtri[kNumLods - 1];
+    L.tri1[0] = t1->tri[kNumLods - 1];
+    L.tri2[0] = t2->tri[kNumLods - 1];
+    L.box1 = t1->d_boxes;
+    L.box2 = t2->d_boxes;
+    L.nvox1 = std::max<long>(t1->n_vox, 1);
+    L.nvox2 = L.self ? 0 : std::max<long>(t2->n_vox, 1);
+    L.num_sms = ctx->num_sms;
+    // most candidates end at their clusters; what finds a queue full is evaluated whole
+    const size_t C = std::min<size_t>(E, kChunk);
+    L.task_cap = (unsigned)std::max<size_t>(16 * C, 1 << 17);
+    L.eval_cap = (unsigned)std::max<size_t>(8 * C, 1 << 17);
+    const size_t c1 = t1->host.n_tris[kNumLods - 1] / 8 + (size_t)L.nvox1 + 1;
+    const size_t c2 = t2->host.n_tris[kNumLods - 1] / 8 + (size_t)std::max<long>(t2->n_vox, 1) + 1;
+    const size_t nv = (size_t)(L.nvox1 + L.nvox2);
+    auto get = [&](int slot, size_t bytes, auto** p) {
+        if (ensure(ctx, ctx->scratch[slot], bytes) != TDP_OK) return false;
+        *p = (std::remove_reference_t<decltype(**p)>*)ctx->scratch[slot].p;
+        return true;
+    };
+    const bool ok = get(67, E * sizeof(RefineItem), &L.items) && get(72, E * sizeof(int4), &L.ext) &&
+                    get(74, E * sizeof(int2), &L.vox) && get(69, E * sizeof(float4), &L.mg) && get(68, E * 4, &L.vres) &&
+                    get(73, E * 4, &L.d.vmx) && get(81, E * 4, &L.d.vupd) && get(kOver, C * 4, &L.over) &&
+                    get(70, Pz * 4, &L.pd) && get(71, 2 * Pz, &L.pown) && get(kFlags, nv * 4, &L.flag1) &&
+                    get(kLists, nv * 4, &L.list1) && get(kCtr, (E / kChunk + 1) * kLodCtrWords * sizeof(unsigned), &L.ctr) &&
+                    get(kCl1, c1 * 3 * sizeof(float4), &L.cl1) && get(kVb1, (size_t)L.nvox1 * 2 * sizeof(float4), &L.vb1) &&
+                    (L.self || (get(kCl2, c2 * 3 * sizeof(float4), &L.cl2) &&
+                                get(kVb2, (size_t)L.nvox2 * 2 * sizeof(float4), &L.vb2))) &&
+                    get(kTasks, (size_t)L.task_cap * sizeof(LodTask), &L.tasks) &&
+                    get(kEvals, (size_t)L.eval_cap * sizeof(LodEval), &L.evals);
+    if (!ok) return false;
+    L.pmiss = L.pown + Pz;
+    if (L.self) {
+        L.cl2 = L.cl1;
+        L.vb2 = L.vb1;
+    }
+    L.flag2 = L.self ? L.flag1 : L.flag1 + L.nvox1;
+    L.list2 = L.self ? L.list1 : L.list1 + L.nvox1;
+    return true;
+}
+
 }  // namespace
 
 int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const tdp_tile* t2, bool pmx_valid,
@@ -537,13 +747,13 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
     ENS(65, (Pz + 1) * 8);             // offsets
     ENS(78, Pz * 4);                   // U per pair
     ENS(79, Pz * kExK * sizeof(RefineItem));  // phase-1 items, kExK per pair
-    ENS(80, Pz * kExK * sizeof(float4));      // phase-1 FP32 results
+    ENS(80, Pz * sizeof(float4));      // directions
     ENS(75, 64);                       // counters
     int64_t* cnt = (int64_t*)ctx->scratch[64].p;
     int64_t* off = (int64_t*)ctx->scratch[65].p;
     float* Ub = (float*)ctx->scratch[78].p;
     RefineItem* item1 = (RefineItem*)ctx->scratch[79].p;
-    float4* res1 = (float4*)ctx->scratch[80].p;
+    float4* dir = (float4*)ctx->scratch[80].p;
     unsigned* ctr = (unsigned*)ctx->scratch[75].p;
     const uint32_t* vt1 = t1->vtri[kNumLods - 1];
     const uint32_t* vt2 = t2->vtri[kNumLods - 1];
@@ -553,16 +763,14 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
     CU(cudaEventRecord(ctx->xev[0], s));
     k_exact_upper<<<pg, kBlk, 0, s>>>(d, pmx_valid ? 1 : 0, vt1, vt2, Ub, item1);
     CU(cudaGetLastError());
-    // phase 1: the kExK closest-core voxel pairs of every object pair in FP32 tighten U
-    const int64_t n1 = d.P * kExK;
-    if (n1 >= (1LL << 31)) return fail(ctx, TDP_ERR_ARG, "too many object pairs for the exact-distance stage");
+    // phase 1: the closest-core voxel pair of every object pair tightens U
+    const int64_t n1 = d.P;
     CU(launch_fetch_items(item1, nullptr, n1, kNumLods - 1, lz1, lz2, ctx->num_sms, s));
-    CU(launch_refine_tuned(t1->tri[kNumLods - 1], t2->tri[kNumLods - 1], item1, (int)n1, res1, ctr, nullptr,
-                           ctx->num_sms, kExactRefineCfg, s));
-    k_exact_tighten<<<grid(d.P, 256, ctx->num_sms * 8), 256, 0, s>>>(res1, d.P, Ub);
+    k_exact_seed<<<grid(n1, 4, ctx->num_sms * 16), 128, 0, s>>>(t1->tri[kNumLods - 1], t2->tri[kNumLods - 1], item1, n1, Ub,
+                                                              dir);
     CU(cudaGetLastError());
     CU(cudaEventRecord(ctx->xev[1], s));
-    k_exact_vp<false><<<pg, kBlk, 0, s>>>(d, Ub, vt1, vt2, cnt, nullptr, nullptr, nullptr, nullptr);
+    k_exact_vp<Vp::kCount><<<pg, kBlk, 0, s>>>(d, Ub, vt1, vt2, cnt, nullptr, nullptr, nullptr, nullptr, LodDev{});
     CU(cudaGetLastError());
     size_t tb = 0;
     CU(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, off, (int)d.P + 1, s));
@@ -574,6 +782,50 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
     info.launches += 6 + (lz1.on || lz2.on ? 1 : 0);
     info.items = (long)E;
     if (E >= (1LL << 31)) return fail(ctx, TDP_ERR_ARG, "too many voxel pairs for the exact-distance stage");
+    LodDev L{};
+    L.d = d;
+    L.d.V = E;
+    L.pcap = Ub;
+    L.dir = dir;
+    if (LodScratchUse in_use(ctx); E > 0 && task_scratch(ctx, L, t1, t2, Pz)) {
+        // phases 2 and 3 as one pass of the LOD loop's task kernels, over the
+        // candidates as items, with U as the pairs' caps
+        unsigned long long* bits = reinterpret_cast<unsigned long long*>(pexact);
+        CU(cudaMemsetAsync(ctr, 0, 64, s));
+        const int chunks = (int)((E + kChunk - 1) / kChunk);
+        CU(cudaMemsetAsync(L.ctr, 0, (size_t)chunks * kLodCtrWords * sizeof(unsigned), s));
+        CU(cudaMemsetAsync(L.pown, 0, 2 * Pz, s));
+        CU(cudaMemsetAsync(L.pd, 0x7f, Pz * 4, s));
+        CU(cudaMemsetAsync(L.flag1, 0xff, (L.self ? L.nvox1 : L.nvox1 + L.nvox2) * 4, s));
+        k_exact_vp<Vp::kTasks><<<pg, kBlk, 0, s>>>(d, Ub, vt1, vt2, nullptr, off, L.items, nullptr, nullptr, L);
+        CU(cudaGetLastError());
+        CU(cudaEventRecord(ctx->xev[2], s));
+        L.n_full = reinterpret_cast<unsigned long long*>(ctr + 12);
+        CU(launch_fetch_items(L.items, nullptr, E, kNumLods - 1, lz1, lz2, ctx->num_sms, s));
+        CU(launch_lod_exact_begin(L, kChunk, chunks, s));
+        for (int c = 0; c < chunks; ++c) {
+            LodDev C = L;
+            C.items += c * kChunk;
+            C.ext += c * kChunk;
+            C.vox += c * kChunk;
+            C.mg += c * kChunk;
+            C.ctr += (size_t)c * kLodCtrWords;
+            C.d.V = std::min(kChunk, E - c * kChunk);
+            CU(launch_lod_exact(C, s));
+            if (c + 1 == chunks) CU(cudaEventRecord(ctx->xev[3], s));
+            CU(launch_lod_f64(C, bits, ctr + 4, s));
+            k_exact_over_f64<<<ctx->num_sms * 2, kExWarps * 32, 0, s>>>(C, bits, ctr + 4);
+        }
+        CU(launch_lod_exact_count(L, ctr + 14, s));
+        k_exact_err<<<grid(d.P, 256, ctx->num_sms * 8), 256, 0, s>>>(d, reinterpret_cast<const unsigned*>(L.pd), pexact, ctr + 8);
+        CU(cudaGetLastError());
+        CU(cudaEventRecord(ctx->xev[4], s));
+        info.launches += 5 + 5 * chunks + (lz1.on || lz2.on ? 1 : 0);
+        if ((rc = read_info(ctx, ctr, 0, info))) return rc;
+        return TDP_OK;
+    }
+    cudaGetLastError();
+    // no room for the task queues: the lazy refine of one warp per candidate
     const size_t Ez = (size_t)std::max<int64_t>(E, 1);
     ENS(67, Ez * sizeof(RefineItem));  // items
     ENS(68, Ez * 4);                   // item -> pair
@@ -597,7 +849,7 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
     float2* sel_thr = (float2*)ctx->scratch[74].p;
     float* preset = (float*)ctx->scratch[81].p;
     ctr = (unsigned*)ctx->scratch[75].p;
-    k_exact_vp<true><<<pg, kBlk, 0, s>>>(d, Ub, vt1, vt2, nullptr, off, items, item_pair, preset);
+    k_exact_vp<Vp::kLazy><<<pg, kBlk, 0, s>>>(d, Ub, vt1, vt2, nullptr, off, items, item_pair, preset, LodDev{});
     CU(cudaGetLastError());
     CU(cudaMemsetAsync(best32, 0x7f, Pz * 4, s));  // 0x7f7f7f7f = 3.4e38, above any distance
     CU(cudaMemsetAsync(emax, 0, Pz * 4, s));
@@ -637,19 +889,7 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
         CU(cudaGetLastError());
         CU(cudaEventRecord(ctx->xev[4], s));
         info.launches += 6 + (lz1.on || lz2.on ? 1 : 0);
-        unsigned ns[12] = {0};
-        CU(cudaMemcpyAsync(ns, ctr + 4, 48, cudaMemcpyDeviceToHost, s));
-        CU(cudaStreamSynchronize(s));
-        info.f64_items = ns[0];
-        float e32;
-        std::memcpy(&e32, &ns[4], 4);
-        info.max_rel_err32 = e32;
-        std::memcpy(&info.full_evals, &ns[8], 8);
-        info.dropped_items = (long)(E - E2) + ns[10];
-        info.below_items = ns[11];
-        float ms[4] = {0, 0, 0, 0};
-        for (int k = 0; k < 4; ++k) cudaEventElapsedTime(&ms[k], ctx->xev[k], ctx->xev[k + 1]);
-        for (int k = 0; k < 4; ++k) info.phase_ms[k] = ms[k];
+        if ((rc = read_info(ctx, ctr, (long)(E - E2), info))) return rc;
     }
 #undef ENS
 #undef CU

@@ -64,28 +64,10 @@ enum Mode {
     kLast,    // the last LOD: the distance itself
 };
 
-// words of a pass's counters
-enum Ctr { cList1, cList2, cTasks, cOver, cWork, cWorkOver, cRedo, cEvals };
 
 __device__ __forceinline__ float sqrt_up(float x) { return radius_sqrt(fmaxf(x, 0.f)); }
 
-__device__ __forceinline__ size_t cluster_base(uint32_t first_tri, int voxel) {
-    // sum over earlier voxels of ceil(n / 8) <= first_tri / 8 + voxel
-    return (size_t)(first_tri >> 3) + (size_t)voxel;
-}
-
 // ---------------------------------------------------------------- items
-__device__ __forceinline__ void claim(bool want, int voxel, int stamp, int* flag, int* list, unsigned* n, int lane) {
-    bool mine = false;
-    if (want && __ldcg(flag + voxel) != stamp) mine = atomicExch(flag + voxel, stamp) != stamp;
-    const unsigned m = __ballot_sync(kFull, mine);
-    if (!m) return;
-    unsigned base = 0;
-    if (lane == 0) base = atomicAdd(n, (unsigned)__popc(m));
-    base = __shfl_sync(kFull, base, 0);
-    if (mine) list[base + __popc(m & ((1u << lane) - 1u))] = voxel;
-}
-
 // One thread per voxel pair.  A pair all of whose voxel pairs, once refined,
 // are refined at every later LOD has one cap (its smallest upper bound can
 // only fall); a voxel that is empty at a later LOD breaks that, and its pairs
@@ -159,9 +141,9 @@ __global__ void __launch_bounds__(256) k_lod_items(LodDev L, int k) {
             else if (d.vupd[v] < 0) atomicMin((unsigned*)L.pcap + p, c);
         }
         if (m) {
-            claim(ok, a, k, L.flag1, L.list1, ctr + cList1, lane);
-            if (L.self) claim(ok, b, k, L.flag1, L.list1, ctr + cList1, lane);
-            else claim(ok, b, k, L.flag2, L.list2, ctr + cList2, lane);
+            lod_claim(ok, a, k, L.flag1, L.list1, ctr + cList1, lane);
+            if (L.self) lod_claim(ok, b, k, L.flag1, L.list1, ctr + cList1, lane);
+            else lod_claim(ok, b, k, L.flag2, L.list2, ctr + cList2, lane);
         }
     }
 }
@@ -335,6 +317,13 @@ __device__ __forceinline__ void pre_rel(const float4* __restrict__ t, float4 o, 
            v3(t2.x - o.x, t2.y - o.y, t2.z - o.z));
     ph = t0.w;
     h = t1.w;
+}
+
+__device__ __forceinline__ void pre_rel64(const float4* __restrict__ t, float4 o, PreTri<double>& P) {
+    const float4 a = t[0], b = t[1], c = t[2];
+    const double ox = o.x, oy = o.y, oz = o.z;
+    pretri(P, v3<double>(a.x - ox, a.y - oy, a.z - oz), v3<double>(b.x - ox, b.y - oy, b.z - oz),
+           v3<double>(c.x - ox, c.y - oy, c.z - oz));
 }
 
 // Margin, slack and preset of an item (uniform over a warp).  The margin
@@ -1041,6 +1030,88 @@ __global__ void __launch_bounds__(256) k_lod_update(LodDev L, int k, int stamp, 
     }
 }
 
+// ---------------------------------------------------------------- exact
+// The queued triangle pairs of a last-LOD pass over reported pairs, once all
+// their FP32 distances are known: the one that holds a pair's minimum is in the
+// queue (its gap is below every cap that ever stood) unless its item is in
+// `over`.  A lane takes one: its gap against the pair's final cap, its FP32
+// distance with its error against the same, and what is left in FP64.  A
+// warp collects those, to run the FP64 distance with all its lanes.
+
+__global__ void __launch_bounds__(kEvalBlock, 2) k_lod_f64(LodDev L, unsigned long long* __restrict__ exact,
+                                                           unsigned* __restrict__ n_items) {
+    __shared__ uint2 queues[kEvalBlock / 32][64];  // (entry, pair)
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    uint2* q = queues[threadIdx.x >> 5];
+    const unsigned n = min(L.ctr[cEvals], L.eval_cap);
+    const unsigned nw = (gridDim.x * blockDim.x) >> 5, gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    int qn = 0;
+    for (unsigned e0 = gw * 32; ; e0 += nw * 32) {
+        const bool fin = e0 >= n;
+        if (!fin) {
+            bool have = e0 + lane < n;
+            unsigned p = 0;
+            if (have) {
+                const LodEval e = L.evals[e0 + lane];
+                const float4 g = L.mg[e.w];
+                p = (unsigned)L.ext[e.w].y;
+                if (!(__float_as_int(g.w) & kEvalFlag)) atomicOr((int*)&L.mg[e.w].w, kEvalFlag);
+                const float lim = fminf(L.pd[p], L.pcap[p]) + g.y;
+                have = !(e.z >= lim + g.x);
+                if (have) {
+                    const float4 o4 = L.tri1[0][(size_t)L.items[e.w].a_off * kTriF4];
+                    PreTri<float> A, B;
+                    float x0, x1, x2, x3;
+                    pre_rel(L.tri1[0] + (size_t)e.a * kTriF4, o4, A, x0, x1);
+                    pre_rel(L.tri2[0] + (size_t)e.b * kTriF4, o4, B, x2, x3);
+                    have = !(sqrtf(tri_dist2(A, B)) - g.x > lim);
+                    if (have && !(atomicOr((int*)&L.mg[e.w].w, kExactFlag) & kExactFlag)) atomicAdd(n_items, 1u);
+                }
+            }
+            const unsigned m = __ballot_sync(kFull, have);
+            if (have) q[qn + __popc(m & lt)] = make_uint2(e0 + lane, p);
+            qn += __popc(m);
+        }
+        __syncwarp();
+        while (qn >= 32 || (fin && qn > 0)) {
+            const int take = min(qn, 32);
+            if (lane < take) {
+                const uint2 u = q[lane];
+                const LodEval e = L.evals[u.x];
+                const float4 o4 = L.tri1[0][(size_t)L.items[e.w].a_off * kTriF4];
+                PreTri<double> A, B;
+                pre_rel64(L.tri1[0] + (size_t)e.a * kTriF4, o4, A);
+                pre_rel64(L.tri2[0] + (size_t)e.b * kTriF4, o4, B);
+                // non-negative doubles order like their bit patterns
+                atomicMin(exact + u.y, (unsigned long long)__double_as_longlong(sqrt(tri_dist2(A, B))));
+            }
+            const uint2 moved = lane + take < qn ? q[lane + take] : make_uint2(0, 0);
+            __syncwarp();
+            qn -= take;
+            if (lane < qn) q[lane] = moved;
+            __syncwarp();
+        }
+        if (fin) break;
+    }
+}
+
+// counts[0]: items none of whose triangle pairs was queued; counts[1]: items
+// with a triangle pair below the pair's cap
+__global__ void k_lod_count(LodDev L, unsigned n, unsigned* __restrict__ counts) {
+    unsigned none = 0, below = 0;
+    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x) {
+        none += !(__float_as_int(L.mg[w].w) & (kEvalFlag | 1));
+        below += L.vres[w] < FLT_MAX;
+    }
+    none = __reduce_add_sync(kFull, none);
+    below = __reduce_add_sync(kFull, below);
+    if ((threadIdx.x & 31) == 0) {
+        if (none) atomicAdd(counts, none);
+        if (below) atomicAdd(counts + 1, below);
+    }
+}
+
 int blocks_for(int64_t n, int per_block, int cap) {
     int64_t g = (n + per_block - 1) / per_block;
     if (g < 1) g = 1;
@@ -1091,6 +1162,32 @@ cudaError_t launch_lod_redo(const LodDev& L, int k, int decide, cudaStream_t s) 
     const cudaError_t e = refine_pass<kLast>(L, k, k + 1, L.ctr + (k + 1) * kLodCtrWords + cRedo, k, s);
     if (e != cudaSuccess) return e;
     k_lod_update<true><<<blocks_for(L.d.P, 8, L.num_sms * 32), 256, 0, s>>>(L, k, k, decide, 1);
+    return cudaGetLastError();
+}
+
+__global__ void k_lod_chunks(unsigned* ctr, int64_t n, int64_t chunk, int n_chunks) {
+    for (int c = threadIdx.x; c < n_chunks; c += blockDim.x)
+        ctr[(size_t)c * kLodCtrWords + cRedo] = (unsigned)(n - c * chunk < chunk ? n - c * chunk : chunk);
+}
+
+cudaError_t launch_lod_exact_begin(const LodDev& L, int64_t chunk, int n_chunks, cudaStream_t s) {
+    const long nv = L.self ? L.nvox1 : L.nvox1 + L.nvox2;
+    k_lod_clusters<<<blocks_for(nv < 2 * L.d.V ? nv : 2 * L.d.V, 8, L.num_sms * 8), 256, 0, s>>>(L, 0);
+    k_lod_chunks<<<1, 256, 0, s>>>(L.ctr, L.d.V, chunk, n_chunks);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_lod_exact(const LodDev& L, cudaStream_t s) {
+    return refine_pass<kLast>(L, 0, 0, L.ctr + cRedo, 0, s);
+}
+
+cudaError_t launch_lod_f64(const LodDev& L, unsigned long long* exact, unsigned* n_f64, cudaStream_t s) {
+    k_lod_f64<<<L.num_sms * 2, kEvalBlock, 0, s>>>(L, exact, n_f64);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_lod_exact_count(const LodDev& L, unsigned* counts, cudaStream_t s) {
+    k_lod_count<<<blocks_for(L.d.V, 256, L.num_sms * 8), 256, 0, s>>>(L, (unsigned)L.d.V, counts);
     return cudaGetLastError();
 }
 

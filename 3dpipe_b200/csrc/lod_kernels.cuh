@@ -77,6 +77,31 @@ struct LodDev {
     int num_sms;
 };
 
+// mg.w of an item beyond 1: evaluated in FP64; a triangle pair was queued
+constexpr int kExactFlag = 2, kEvalFlag = 4;
+
+// words of a pass's counters
+enum LodCtr { cList1, cList2, cTasks, cOver, cWork, cWorkOver, cRedo, cEvals };
+
+#ifdef __CUDACC__
+__device__ __forceinline__ size_t cluster_base(uint32_t first_tri, int voxel) {
+    // sum over earlier voxels of ceil(n / 8) <= first_tri / 8 + voxel
+    return (size_t)(first_tri >> 3) + (size_t)voxel;
+}
+
+// a whole warp: the lanes' voxels that are not stamped yet join the list
+__device__ __forceinline__ void lod_claim(bool want, int voxel, int stamp, int* flag, int* list, unsigned* n, int lane) {
+    bool mine = false;
+    if (want && __ldcg(flag + voxel) != stamp) mine = atomicExch(flag + voxel, stamp) != stamp;
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (!m) return;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(n, (unsigned)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (mine) list[base + __popc(m & ((1u << lane) - 1u))] = voxel;
+}
+#endif
+
 cudaError_t launch_lod_items(const LodDev& L, int k, cudaStream_t s);
 // clusters, (first LOD) seeds, cull, tests and evaluation of LOD k's items
 cudaError_t launch_lod_refine(const LodDev& L, int k, int highest, cudaStream_t s);
@@ -85,5 +110,18 @@ cudaError_t launch_lod_refine(const LodDev& L, int k, int highest, cudaStream_t 
 cudaError_t launch_lod_update(const LodDev& L, int k, int highest, int decide, cudaStream_t s);
 // the last LOD again for those pairs (normally none)
 cudaError_t launch_lod_redo(const LodDev& L, int k, int decide, cudaStream_t s);
+
+// The last LOD's rules over items that the caller wrote (L has that one LOD),
+// in chunks that the queues hold.  First the clusters of the voxels in use and
+// the chunks' counters (kLodCtrWords words each; the claims are in the first's):
+cudaError_t launch_lod_exact_begin(const LodDev& L, int64_t chunk, int n_chunks, cudaStream_t s);
+// then chunk by chunk, L's item arrays and counters moved to the chunk's and V
+// its items: each pair's smallest FP32 distance below its cap so far in pd,
+cudaError_t launch_lod_exact(const LodDev& L, cudaStream_t s);
+// and the FP64 minimum of the queued triangle pairs that can hold it, per pair
+// into exact (bits); the items they belong to are counted in n_f64
+cudaError_t launch_lod_f64(const LodDev& L, unsigned long long* exact, unsigned* n_f64, cudaStream_t s);
+// last: items without a queued triangle pair, items with a distance below the cap
+cudaError_t launch_lod_exact_count(const LodDev& L, unsigned* counts, cudaStream_t s);
 
 }  // namespace tdp

@@ -87,9 +87,11 @@ typedef struct {
                                         2 captured (or updated) it in this call */
     double refine_ms_lod[5];         /* tuned refine time per LOD 20..100      */
     double exact_phase_ms[4];        /* exact stage, device time of: upper
-                                        bounds (with their FP32 refine),
+                                        bounds (with their FP32 seeds),
                                         candidate voxel pairs, the FP32 pass,
-                                        the FP64 pass                          */
+                                        the FP64 pass (of more than 524,288
+                                        candidates: of the last part; the
+                                        others' FP64 counts as FP32)           */
     unsigned long long exact_full_evals; /* exact stage: triangle pairs fully
                                         evaluated by its FP32 pass             */
     long candidates_on_device;       /* 1: object candidates were computed on
@@ -97,9 +99,8 @@ typedef struct {
     long candidate_redone;           /* kNN queries whose ring search outgrew a
                                         warp's shared-memory buffer and were
                                         redone on the GPU with a global one    */
-    long exact_dropped_items;        /* exact stage: FP32-pass voxel pairs
-                                        dropped by the refine's item-level
-                                        bound test (no triangle staged)        */
+    long exact_dropped_items;        /* exact stage: FP32-pass voxel pairs whose
+                                        bounds left no triangle pair           */
     long exact_below_items;          /* exact stage: FP32-pass voxel pairs with
                                         a triangle pair below their preset     */
 } tdp_stats;
