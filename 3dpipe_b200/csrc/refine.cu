@@ -19,6 +19,7 @@
 //                        cluster- then triangle-level lower bounds against the
 //                        warp's running minima skip pairs that cannot lower any
 //                        of the three minima (details above the kernel).
+#include <cooperative_groups.h>
 #include <float.h>
 #include "common.cuh"
 #include "tridist.cuh"
@@ -1040,23 +1041,29 @@ cudaError_t launch_refine_tuned(const float4* triA, const float4* triB, const Re
 // ------------------------------------------------------------------ FP64 recheck
 // Exact (FP64) minimum triangle distance of a few voxel pairs: the tuned form's
 // recheck of object pairs whose FP32 decision fell inside the error band.
-constexpr int kF64Block = 128;
+// A cluster of blocks per voxel pair: there are few of them (2 pairs left 13 in
+// the 10-NN of 20,000 x 100) and a block of 128 went through its 10,000 triangle
+// pairs in 80 rounds, 200 us; this way 32.
+constexpr int kF64Block = 128, kF64Cluster = 8;
 
-__global__ void __launch_bounds__(kF64Block) refine_f64_kernel(const float4* __restrict__ triA,
+__global__ void __cluster_dims__(kF64Cluster, 1, 1) __launch_bounds__(kF64Block) refine_f64_kernel(const float4* __restrict__ triA,
                                                                const float4* __restrict__ triB,
                                                                const RefineItem* __restrict__ items, int n_items_host,
                                                                const unsigned* n_items_dev, double* __restrict__ out) {
     __shared__ double red[kF64Block / 32];
+    __shared__ double share;
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const unsigned rank = cl.block_rank();
     const int n_items = n_items_dev ? (int)*n_items_dev : n_items_host;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+    for (int it = blockIdx.x / kF64Cluster; it < n_items; it += gridDim.x / kF64Cluster) {  // the same for the cluster
         const RefineItem w = items[it];
         double best = 1e300;
         if (w.a_cnt && w.b_cnt) {
             const float4 o4 = triA[(size_t)w.a_off * kTriF4];
             const double ox = o4.x, oy = o4.y, oz = o4.z;
             const uint64_t total = (uint64_t)w.a_cnt * w.b_cnt;
-            for (uint64_t p = tid; p < total; p += kF64Block) {
+            for (uint64_t p = rank * kF64Block + tid; p < total; p += kF64Cluster * kF64Block) {
                 const uint32_t i = (uint32_t)(p / w.b_cnt), j = (uint32_t)(p - (uint64_t)i * w.b_cnt);
                 const float4* a = triA + ((size_t)w.a_off + i) * kTriF4;
                 const float4* b = triB + ((size_t)w.b_off + j) * kTriF4;
@@ -1079,15 +1086,25 @@ __global__ void __launch_bounds__(kF64Block) refine_f64_kernel(const float4* __r
         __syncthreads();
         if (tid == 0) {
             for (int k = 1; k < kF64Block / 32; ++k) best = red[k] < best ? red[k] : best;
+            share = best;
+        }
+        cl.sync();  // every block's share is written
+        if (rank == 0 && tid == 0) {
+            for (unsigned k = 1; k < kF64Cluster; ++k) {
+                const double v = *cl.map_shared_rank(&share, k);
+                best = v < best ? v : best;
+            }
             out[it] = (w.a_cnt && w.b_cnt) ? sqrt(best) : 1e300;
         }
+        cl.sync();  // and read: the next item's may be written, or the block end
     }
 }
 
 cudaError_t launch_refine_f64(const float4* triA, const float4* triB, const RefineItem* items, int n_items,
                               double* out, cudaStream_t s, const unsigned* n_items_dev) {
     if (n_items <= 0) return cudaSuccess;
-    int grid = n_items < 148 * 16 ? n_items : 148 * 16;
+    const int clusters = n_items < 148 * 2 ? n_items : 148 * 2;
+    const int grid = clusters * kF64Cluster;
     refine_f64_kernel<<<grid, kF64Block, 0, s>>>(triA, triB, items, n_items, n_items_dev, out);
     return cudaGetLastError();
 }
