@@ -801,7 +801,8 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
         CU(cudaGetLastError());
         CU(cudaEventRecord(ctx->xev[2], s));
         L.n_full = reinterpret_cast<unsigned long long*>(ctr + 12);
-        CU(launch_fetch_items(L.items, nullptr, E, kNumLods - 1, lz1, lz2, ctx->num_sms, s));
+        CU(launch_fetch_list(kNumLods - 1, lz1, lz2, L.list1, L.ctr + cList1, L.self ? nullptr : L.list2, L.ctr + cList2,
+                             ctx->num_sms, s));
         CU(launch_lod_exact_begin(L, kChunk, chunks, s));
         for (int c = 0; c < chunks; ++c) {
             LodDev C = L;

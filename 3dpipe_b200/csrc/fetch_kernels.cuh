@@ -48,9 +48,15 @@ cudaError_t launch_fetch_all(const LazyTile& t, int num_sms, cudaStream_t s);
 // alive and whose object pair is undecided (valive[v], pstat[vpair[v]] == 0):
 // a superset of the next LOD's refine items, run on a second stream beside
 // the current LOD's refine.  The flags may change meanwhile; a voxel that is
-// missed here is fetched by that LOD's own launch_fetch_items.
+// missed here is fetched by that LOD's own launch.
+// list: one word and one per voxel of the attached tiles.
 cudaError_t launch_prefetch_pairs(const uint8_t* valive, const int* vpair, const uint8_t* pstat, const int* vpa,
                                   const int* vpb, int64_t V, int lod, const LazyTile& a, const LazyTile& b,
-                                  int num_sms, cudaStream_t s);
+                                  int* list, int num_sms, cudaStream_t s);
+// fetch the *na voxels of tile a in la and the *nb of tile b in lb, at LOD index
+// lod, unless they are there (no voxel listed twice, counts in device memory);
+// one tile that is both sides: its voxels in la, lb null
+cudaError_t launch_fetch_list(int lod, const LazyTile& a, const LazyTile& b, const int* la, const unsigned* na,
+                              const int* lb, const unsigned* nb, int num_sms, cudaStream_t s);
 
 }  // namespace tdp

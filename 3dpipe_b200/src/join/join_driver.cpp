@@ -51,6 +51,7 @@ enum Slot {
     kPreset = 91,                     // the last LOD's item presets (within queries)
     kLodExt = kLodScratchFirst, kLodVox, kLodMg, kLodCaps, kLodFlags, kLodZero, kLodVres, kLodCl1, kLodCl2, kLodVb1, kLodVb2,
     kLodLists, kLodTasks, kLodOver, kLodEvals, kLodBest, kLodDir,   // the LOD loop's task form
+    kPfList = kLodScratchEnd,                                       // voxels to prefetch
 };
 
 template <typename T>
@@ -86,6 +87,7 @@ struct LodLoop {
     LazyTile lz1, lz2;  // attached tiles: fetch each LOD's voxels before its refine
     cudaStream_t side;  // attached tiles: the next LOD's prefetch runs here
     cudaEvent_t pf[16];
+    int* pf_list;       // its voxels
     // configuration 0 at every LOD (the default): the loop as task kernels
     // (csrc/lod_kernels.cuh), 3 to 5 times as fast on kNN joins as the fastest
     // of the other configurations, which stay for callers that pin one
@@ -113,12 +115,15 @@ int enqueue_task_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captu
         const int highest = k == L.highest_k;
         CUL(launch_lod_items(L.t, k, s));
         if (prefetch && k > 0) CUL(cudaStreamWaitEvent(s, L.pf[2 * (k - 1) + 1], 0));
-        CUL(launch_fetch_items(L.items, L.t.n_items + k, 0, L.li[k], L.lz1, L.lz2, L.num_sms, s));
+        // the voxels in use, listed by the items
+        const unsigned* in_use = L.t.ctr + (size_t)k * kLodCtrWords;
+        CUL(launch_fetch_list(L.li[k], L.lz1, L.lz2, L.t.list1, in_use + cList1, L.t.self ? nullptr : L.t.list2,
+                              in_use + cList2, L.num_sms, s));
         if (prefetch && k + 1 < L.nl) {
             CUL(cudaEventRecord(L.pf[2 * k], s));
             CUL(cudaStreamWaitEvent(L.side, L.pf[2 * k], 0));
             CUL(launch_prefetch_pairs(L.d.valive, L.d.vpair, L.d.pstat, L.d.vpa, L.d.vpb, L.V, L.li[k + 1], L.lz1,
-                                      L.lz2, L.num_sms, L.side));
+                                      L.lz2, L.pf_list, L.num_sms, L.side));
             CUL(cudaEventRecord(L.pf[2 * k + 1], L.side));
         }
         CUL(rec(L.ev[2 * k]));
@@ -166,7 +171,7 @@ int enqueue_lod_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captur
             CUL(cudaEventRecord(L.pf[2 * k], s));
             CUL(cudaStreamWaitEvent(L.side, L.pf[2 * k], 0));
             CUL(launch_prefetch_pairs(L.d.valive, L.d.vpair, L.d.pstat, L.d.vpa, L.d.vpb, L.V, L.li[k + 1], L.lz1,
-                                      L.lz2, L.num_sms, L.side));
+                                      L.lz2, L.pf_list, L.num_sms, L.side));
             CUL(cudaEventRecord(L.pf[2 * k + 1], L.side));
         }
         CUL(cudaMemcpyAsync(lod_counts + k, cnt_items, 4, cudaMemcpyDeviceToDevice, s));
@@ -185,7 +190,7 @@ int enqueue_lod_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captur
         CUL(launch_count_status(L.d, cnt_recheck, s));
         CUL(cudaMemsetAsync(cnt_items, 0, 4, s));
         CUL(launch_recheck_items(L.d, L.vt1_100, L.vt2_100, L.items, L.item_vp, L.vexact, cnt_items, s));
-        CUL(launch_fetch_items(L.items, cnt_items, 0, kNumLods - 1, L.lz1, L.lz2, L.num_sms, s));
+        // (its voxel pairs were items of LOD 100: nothing to fetch)
         CUL(launch_refine_f64(L.tri1_100, L.tri2_100, L.items, V, L.res64, s, cnt_items));
         CUL(launch_recheck_finish(L.d, L.res64, L.item_vp, V, L.vexact, L.pexact, L.knn, L.K, L.tau, s, cnt_items));
     }
@@ -522,6 +527,12 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         L.lz1 = lz1; L.lz2 = lz2;
         L.preset = presets ? buf<float>(ctx, kPreset) : nullptr;
         L.side = ctx->side;
+        if ((lz1.on || lz2.on) && L.side) {  // without room for the list: no prefetch
+            if (ensure(ctx, ctx->scratch[kPfList], ((size_t)t1->n_vox + (size_t)t2->n_vox + 1) * 4) == TDP_OK)
+                L.pf_list = buf<int>(ctx, kPfList);
+            else
+                L.side = nullptr;
+        }
         for (int k = 0; k < 16; ++k) L.pf[k] = ctx->pf_ev[k];
         L.tasks = 1;
         for (int k = 0; k < L.nl; ++k) L.tasks = L.tasks && L.cfg[k] == 0;
@@ -591,9 +602,9 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             const bool attached = L.lz1.on || L.lz2.on;
             // (a fetch or a prefetch is a mark launch and a copy launch)
             // (task form: six a LOD, the seeds of the first and four of the redo)
-            launches += ((L.tasks ? 6 : 4) + (L.any_knn ? 1 : 0) + (attached ? 2 : 0)) * L.nl + (L.tasks ? 5 : 0) +
+            launches += ((L.tasks ? 6 : 4) + (L.any_knn ? 1 : 0) + (attached ? (L.tasks ? 1 : 2) : 0)) * L.nl + (L.tasks ? 5 : 0) +
                         (attached && L.side ? 2 * (L.nl - 1) : 0) +
-                        (L.recheck ? (knn ? 5 : 4) + (attached ? 2 : 0) : 0);
+                        (L.recheck ? (knn ? 5 : 4) : 0);
         }
         st.refine_launches += L.nl;
     }
