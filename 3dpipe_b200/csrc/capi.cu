@@ -1,6 +1,7 @@
 // capi.cu -- context management and the refine seam of the C ABI (include/tdp.h).
 #include <float.h>
 #include <algorithm>
+#include <climits>
 #include <string.h>
 #include <vector>
 #include "ctx.cuh"
@@ -312,6 +313,20 @@ int tdp_ctx_memory(const tdp_ctx* ctx, size_t* in_use, size_t* peak) {
     return TDP_OK;
 }
 
+namespace {
+
+// The eager refine gives a voxel pair to one warp, and a batch ends with its
+// largest: 236 us for 3,000 pairs of up to 130 triangles a side, 203 us for 300.
+// Pairs are cut into runs of B triangles (whole stagings of 32) until a resident
+// warp has about four parts: 143 and 69 us (50 pairs: 107 -> 48).  A part is not made
+// smaller than 2,048 triangle pairs (about 25 us): with 3,000 pairs of up to 40 a
+// side the cut saved 13 us of the kernel and cost 40 on the host.  In large
+// batches nothing is above the share and they stay whole.  Only for the default
+// refine: the other configurations are pinned by callers that compare them.
+constexpr int kPartB = 32, kPartsPerWarp = 4, kRefineWarpsPerSm = 12, kPartLeast = 2048;
+
+}  // namespace
+
 int tdp_refine_batch(tdp_ctx* ctx, const float* data, const float* hausdorff, size_t element_num,
                      const size_t* offset_size, uint32_t pair_num, int form, float* out) {
     if (!ctx) return TDP_ERR_ARG;
@@ -322,6 +337,7 @@ int tdp_refine_batch(tdp_ctx* ctx, const float* data, const float* hausdorff, si
     cudaSetDevice(ctx->device);
     std::vector<RefineItem> items(pair_num);
     double tri_pairs = 0;
+    uint64_t most = 0;
     for (uint32_t i = 0; i < pair_num; ++i) {
         size_t o1 = offset_size[4 * i], n1 = offset_size[4 * i + 1];
         size_t o2 = offset_size[4 * i + 2], n2 = offset_size[4 * i + 3];
@@ -329,47 +345,96 @@ int tdp_refine_batch(tdp_ctx* ctx, const float* data, const float* hausdorff, si
             return fail(ctx, TDP_ERR_ARG, "offset_size entry " + std::to_string(i) + " out of range");
         items[i] = RefineItem{(uint32_t)o1, (uint32_t)n1, (uint32_t)o2, (uint32_t)n2};
         tri_pairs += (double)n1 * (double)n2;
+        most = std::max(most, (uint64_t)n1 * n2);
     }
     int rc;
     if ((rc = ensure(ctx, ctx->scratch[kSlotRawData], element_num * 9 * sizeof(float)))) return rc;
     if (hausdorff && (rc = ensure(ctx, ctx->scratch[kSlotRawHd], element_num * 2 * sizeof(float)))) return rc;
     if ((rc = ensure(ctx, ctx->scratch[kSlotTris], element_num * kTriF4 * sizeof(float4)))) return rc;
+    std::vector<RefineItem> parts;  // empty: the pairs are refined whole
+    size_t n_cut = 0;               // parts; after them, the pairs' first parts
+    if (form == TDP_FORM_TUNED && ctx->tuned_cfg == 0 && most > kPartLeast && pair_num < (1u << 30)) {
+        const double share = std::max((double)kPartLeast, tri_pairs / ((double)ctx->num_sms * kRefineWarpsPerSm * kPartsPerWarp));
+        if (share < (double)most) {
+            std::vector<uint32_t> first(pair_num + 1);
+            parts.reserve(2 * (size_t)pair_num);
+            for (uint32_t i = 0; i < pair_num; ++i) {
+                const RefineItem& it = items[i];
+                first[i] = (uint32_t)parts.size();
+                if ((double)it.a_cnt * it.b_cnt <= share || parts.size() > (size_t)INT_MAX / 2) {
+                    parts.push_back(it);
+                    continue;
+                }
+                const double want = share / it.a_cnt;  // B triangles of a part, in whole stagings
+                const uint32_t run = want >= it.b_cnt ? it.b_cnt : ((uint32_t)want / kPartB + 1) * kPartB;
+                for (uint32_t b = 0; b < it.b_cnt; b += std::min(run, it.b_cnt - b))
+                    parts.push_back(RefineItem{it.a_off, it.a_cnt, it.b_off + b, std::min(run, it.b_cnt - b)});
+            }
+            n_cut = parts.size();
+            first[pair_num] = (uint32_t)n_cut;
+            first.resize((first.size() + 3) / 4 * 4);
+            const RefineItem* f = reinterpret_cast<const RefineItem*>(first.data());
+            parts.insert(parts.end(), f, f + first.size() / 4);
+        }
+    }
     if ((rc = ensure(ctx, ctx->scratch[kSlotItems], pair_num * sizeof(RefineItem)))) return rc;
     if ((rc = ensure(ctx, ctx->scratch[kSlotOut], pair_num * sizeof(float4)))) return rc;
+    if (!parts.empty() && (ensure(ctx, ctx->scratch[kSlotParts], parts.size() * sizeof(RefineItem)) != TDP_OK ||
+                           ensure(ctx, ctx->scratch[kSlotPartOut], n_cut * sizeof(float4)) != TDP_OK)) {
+        cudaGetLastError();
+        parts.clear();  // no room for them
+    }
+    const size_t n_parts = parts.empty() ? pair_num : n_cut;
     float* d_data = (float*)ctx->scratch[kSlotRawData].p;
     float* d_hd = hausdorff ? (float*)ctx->scratch[kSlotRawHd].p : nullptr;
     float4* d_tri = (float4*)ctx->scratch[kSlotTris].p;
-    RefineItem* d_items = (RefineItem*)ctx->scratch[kSlotItems].p;
+    RefineItem* d_items = (RefineItem*)ctx->scratch[parts.empty() ? kSlotItems : kSlotParts].p;
     float4* d_out = (float4*)ctx->scratch[kSlotOut].p;
     cudaStream_t s = ctx->stream;
     TDP_CUDA_TRY(cudaMemcpyAsync(d_data, data, element_num * 9 * sizeof(float), cudaMemcpyHostToDevice, s));
     if (d_hd) TDP_CUDA_TRY(cudaMemcpyAsync(d_hd, hausdorff, element_num * 2 * sizeof(float), cudaMemcpyHostToDevice, s));
-    TDP_CUDA_TRY(cudaMemcpyAsync(d_items, items.data(), pair_num * sizeof(RefineItem), cudaMemcpyHostToDevice, s));
-    TDP_CUDA_TRY(launch_pack_triangles(d_data, d_hd, element_num, d_tri, s));
-    TDP_CUDA_TRY(cudaMemsetAsync(ctx->d_stats, 0, sizeof(unsigned long long), s));
+    const std::vector<RefineItem>& up = parts.empty() ? items : parts;
+    TDP_CUDA_TRY(cudaMemcpyAsync(d_items, up.data(), up.size() * sizeof(RefineItem), cudaMemcpyHostToDevice, s));
+    TDP_CUDA_TRY(cudaMemsetAsync(ctx->d_stats, 0, 2 * sizeof(unsigned long long), s));
+    TDP_CUDA_TRY(launch_pack_triangles(d_data, d_hd, element_num, d_tri, s, parts.empty() ? nullptr : ctx->d_stats + 1));
     TDP_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
     if (form == TDP_FORM_PLAIN) {
         TDP_CUDA_TRY(launch_refine_plain(d_tri, d_tri, d_items, (int)pair_num, d_out, s));
     } else {
-        TDP_CUDA_TRY(launch_refine_tuned(d_tri, d_tri, d_items, (int)pair_num, d_out, ctx->d_counter, ctx->d_stats,
+        float4* po = parts.empty() ? d_out : (float4*)ctx->scratch[kSlotPartOut].p;
+        TDP_CUDA_TRY(launch_refine_tuned(d_tri, d_tri, d_items, (int)n_parts, po, ctx->d_counter, ctx->d_stats,
                                          ctx->num_sms, ctx->tuned_cfg, s));
+        if (!parts.empty())
+            TDP_CUDA_TRY(launch_merge_parts(po, (const uint32_t*)(d_items + n_cut), (int)pair_num, d_out, s));
     }
     TDP_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
     std::vector<float4> res(pair_num);
-    unsigned long long full = 0;
-    TDP_CUDA_TRY(cudaMemcpyAsync(res.data(), d_out, pair_num * sizeof(float4), cudaMemcpyDeviceToHost, s));
-    TDP_CUDA_TRY(cudaMemcpyAsync(&full, ctx->d_stats, sizeof(full), cudaMemcpyDeviceToHost, s));
-    TDP_CUDA_TRY(cudaStreamSynchronize(s));
+    unsigned long long full[2] = {0, 0};  // evaluations, non-finite input
+    for (;;) {
+        TDP_CUDA_TRY(cudaMemcpyAsync(res.data(), d_out, pair_num * sizeof(float4), cudaMemcpyDeviceToHost, s));
+        TDP_CUDA_TRY(cudaMemcpyAsync(full, ctx->d_stats, sizeof(full), cudaMemcpyDeviceToHost, s));
+        TDP_CUDA_TRY(cudaStreamSynchronize(s));
+        if (!full[1]) break;
+        // A bound that is not a number drops every triangle pair under it, and
+        // parts have other bounds than the whole: such a batch is done whole.
+        d_items = (RefineItem*)ctx->scratch[kSlotItems].p;
+        TDP_CUDA_TRY(cudaMemcpyAsync(d_items, items.data(), pair_num * sizeof(RefineItem), cudaMemcpyHostToDevice, s));
+        TDP_CUDA_TRY(cudaMemsetAsync(ctx->d_stats, 0, 2 * sizeof(unsigned long long), s));
+        TDP_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
+        TDP_CUDA_TRY(launch_refine_tuned(d_tri, d_tri, d_items, (int)pair_num, d_out, ctx->d_counter, ctx->d_stats,
+                                         ctx->num_sms, ctx->tuned_cfg, s));
+        TDP_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+    }
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     ctx->stats = LastStats();
     ctx->stats.refine_ms = ms;
     ctx->stats.total_ms = ms;
     ctx->stats.tri_pairs = tri_pairs;
-    ctx->stats.full_evals = form == TDP_FORM_PLAIN ? (unsigned long long)tri_pairs : full;
+    ctx->stats.full_evals = form == TDP_FORM_PLAIN ? (unsigned long long)tri_pairs : full[0];
     ctx->stats.refine_items = pair_num;
     ctx->stats.refine_launches = 1;
-    ctx->stats.kernel_launches = 2;
+    ctx->stats.kernel_launches = parts.empty() ? 2 : 3;
     for (uint32_t i = 0; i < pair_num; ++i) {
         out[3 * i] = res[i].x;
         out[3 * i + 1] = hausdorff ? res[i].y : FLT_MAX;

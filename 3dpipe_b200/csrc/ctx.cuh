@@ -63,7 +63,7 @@ struct tdp_ctx {
     cudaEvent_t pf_ev[16] = {};   // fork / join of the prefetches (no timing)
     std::string last_error;
     std::unordered_map<void*, size_t> allocs;
-    tdp::Buf scratch[120];  // slots: refine-batch 0-4, tile upload 12-13, join 20-48, candidates 50-59 and 88-90, result sort 60-63, exact distances 64-81 and 84-86, per-object queries 82-83, last-LOD presets 91, GPU attach pass 96-100, LOD task form 101-117
+    tdp::Buf scratch[120];  // slots: refine-batch 0-6, tile upload 12-13, join 20-48, candidates 50-59 and 88-90, result sort 60-63, exact distances 64-81 and 84-86, per-object queries 82-83, last-LOD presets 91, GPU attach pass 96-100, LOD task form 101-117
     unsigned* d_counter = nullptr;            // work counters (device)
     bool lod_busy = false;                    // the LOD task scratch is in use (LodScratchUse)
     unsigned long long* d_stats = nullptr;    // device-side statistics
@@ -130,7 +130,7 @@ struct LodScratchUse {
 };
 
 enum ScratchSlot {
-    kSlotRawData = 0, kSlotRawHd, kSlotTris, kSlotItems, kSlotOut,
+    kSlotRawData = 0, kSlotRawHd, kSlotTris, kSlotItems, kSlotOut, kSlotParts, kSlotPartOut,
 };
 
 }  // namespace tdp

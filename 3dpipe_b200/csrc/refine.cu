@@ -20,6 +20,8 @@
 //                        warp's running minima skip pairs that cannot lower any
 //                        of the three minima (details above the kernel).
 #include <cooperative_groups.h>
+
+#include <algorithm>
 #include <float.h>
 #include "common.cuh"
 #include "tridist.cuh"
@@ -1109,24 +1111,51 @@ cudaError_t launch_refine_f64(const float4* triA, const float4* triB, const Refi
     return cudaGetLastError();
 }
 
+// A voxel pair refined in parts (the same A triangles, a run of B triangles
+// each): every value is a minimum over its triangle pairs, w the largest coordinate.
+__global__ void merge_parts_kernel(const float4* __restrict__ parts, const uint32_t* __restrict__ first, int n,
+                                   float4* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        float4 r = parts[first[i]];
+        for (uint32_t k = first[i] + 1; k < first[i + 1]; ++k) {
+            const float4 p = parts[k];
+            r = make_float4(fminf(r.x, p.x), fminf(r.y, p.y), fminf(r.z, p.z), fmaxf(r.w, p.w));
+        }
+        out[i] = r;
+    }
+}
+
+cudaError_t launch_merge_parts(const float4* parts, const uint32_t* first, int n, float4* out, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    merge_parts_kernel<<<std::min((n + 127) / 128, 148 * 16), 128, 0, s>>>(parts, first, n, out);
+    return cudaGetLastError();
+}
+
 // Pack the reference's flat layout (9 floats per triangle + 2 Hausdorff floats)
 // into 48-byte triangle records.
 __global__ void pack_triangles_kernel(const float* __restrict__ data, const float* __restrict__ hd, size_t n,
-                                      float4* __restrict__ tri) {
+                                      float4* __restrict__ tri, unsigned long long* __restrict__ odd) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float* d = data + 9 * i;
         float ph = hd ? hd[2 * i] : 0.f, h = hd ? hd[2 * i + 1] : 0.f;
         tri[3 * i + 0] = make_float4(d[0], d[1], d[2], ph);
         tri[3 * i + 1] = make_float4(d[3], d[4], d[5], h);
         tri[3 * i + 2] = make_float4(d[6], d[7], d[8], 0.f);
+        if (odd) {  // x - x is 0 for a finite x only
+            float z = (ph - ph) + (h - h);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) z += d[k] - d[k];
+            if (!(z == 0.f)) *odd = 1;
+        }
     }
 }
 
-cudaError_t launch_pack_triangles(const float* data, const float* hd, size_t n, float4* tri, cudaStream_t s) {
+cudaError_t launch_pack_triangles(const float* data, const float* hd, size_t n, float4* tri, cudaStream_t s,
+                                  unsigned long long* odd) {
     if (n == 0) return cudaSuccess;
     size_t blocks = (n + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;
-    pack_triangles_kernel<<<(unsigned)blocks, 256, 0, s>>>(data, hd, n, tri);
+    pack_triangles_kernel<<<(unsigned)blocks, 256, 0, s>>>(data, hd, n, tri, odd);
     return cudaGetLastError();
 }
 
