@@ -31,6 +31,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -421,12 +422,13 @@ struct TileBoxes {
 }  // namespace
 
 int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool self, bool knn, int K, float tau,
-                      Buf& pq_buf, Buf& pt_buf, Buf& qoff_buf, long& P, long& n_redone, const int* qk,
+                      Buf& pq_buf, Buf& pt_buf, Buf& qoff_buf, long& P, long& n_redone, long& most, const int* qk,
                       const float* qtau, bool isect, long q_begin, long q_end) {
     cudaStream_t s = ctx->stream;
     const long n1 = t1->n_obj, n2 = t2->n_obj;
     const long qb0 = std::max(0L, q_begin), qe0 = q_end < 0 ? n1 : std::min(n1, q_end);
     n_redone = 0;
+    most = 0;
     P = 0;
     int rc;
     // grids over tile 2, built once per tile
@@ -502,9 +504,11 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
         CU(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, qoff, (int)n1 + 1, s));
         if ((rc = ensure(ctx, tmp, tb + 16))) return rc;
         CU(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt, qoff, (int)n1 + 1, s));
-        CU(cudaMemcpyAsync(&total, qoff + n1, 8, cudaMemcpyDeviceToHost, s));
-        CU(cudaMemcpyAsync(found, d_over, 8, cudaMemcpyDeviceToHost, s));
+        CU(cudaMemcpyAsync(ctx->hwords, qoff + n1, 8, cudaMemcpyDeviceToHost, s));
+        CU(cudaMemcpyAsync(ctx->hwords + 1, d_over, 8, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
+        total = (int64_t)ctx->hwords[0];
+        std::memcpy(found, ctx->hwords + 1, 8);
         if (!over || pass > 0) break;
         // Some kNN ring searches saw more points than a warp's shared-memory
         // buffer holds: redo just those on the device with a global buffer of
@@ -523,6 +527,7 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
     }
     if (total >= (1LL << 31) - 1) return fail(ctx, TDP_ERR_ARG, "too many candidate pairs");
     P = (long)total;
+    most = found[1];
     const size_t Pz = (size_t)std::max<long>(P, 1);
     if ((rc = ensure(ctx, keys, Pz * 8))) return rc;
     if ((rc = ensure(ctx, keys2, Pz * 8))) return rc;
@@ -560,11 +565,11 @@ extern "C" long tdp_tile_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_
     const bool self = (t2 == nullptr || t2 == t1);
     if (!t2) t2 = t1;
     cudaSetDevice(ctx->device);
-    long P = 0, redone = 0;
+    long P = 0, redone = 0, most = 0;
     Buf& pq = ctx->scratch[57];
     Buf& pt = ctx->scratch[58];
     Buf& qo = ctx->scratch[59];
-    if (device_candidates(ctx, t1, t2, self, is_knn != 0, is_knn ? knn : 0, within, pq, pt, qo, P, redone))
+    if (device_candidates(ctx, t1, t2, self, is_knn != 0, is_knn ? knn : 0, within, pq, pt, qo, P, redone, most))
         return LONG_MIN;
     ctx->stats.candidate_redone = redone;
     cudaMemcpyAsync(off, qo.p, (t1->n_obj + 1) * 8, cudaMemcpyDeviceToHost, ctx->stream);

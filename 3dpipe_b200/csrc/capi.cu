@@ -177,6 +177,10 @@ int tdp_ctx_create(int device, size_t budget_bytes, unsigned flags, tdp_ctx** ou
         tdp_ctx_destroy(ctx);
         return TDP_ERR_NOMEM;
     }
+    if (cudaHostAlloc((void**)&ctx->hwords, sizeof ctx->pageable_words, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->hwords = ctx->pageable_words;
+    }
     *out = ctx;
     return TDP_OK;
 }
@@ -200,6 +204,7 @@ int tdp_ctx_destroy(tdp_ctx* ctx) {
     if (ctx->lod_graph) cudaGraphExecDestroy(ctx->lod_graph);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->hres) cudaFreeHost(ctx->hres);
+    if (ctx->hwords && ctx->hwords != ctx->pageable_words) cudaFreeHost(ctx->hwords);
     for (int k = 0; k < 2; ++k) {
         if (ctx->hstage[k]) cudaFreeHost(ctx->hstage[k]);
         if (ctx->hstage_ev[k]) cudaEventDestroy(ctx->hstage_ev[k]);

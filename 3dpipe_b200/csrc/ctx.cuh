@@ -74,6 +74,9 @@ struct tdp_ctx {
     int lod_cfg[tdp::kNumLods] = {-1, -1, -1, -1, -1};
     void* hres = nullptr;  // page-locked staging of join results (grow-only)
     size_t hres_cap = 0;
+    // counts read back in mid-join: page-locked, or pageable where that is short
+    unsigned long long* hwords = nullptr;
+    unsigned long long pageable_words[4] = {};
     // CUDA graph of the tuned form's LOD loop (tdp_set_lod_graph): the
     // executable, the launch arguments it was captured with, and the last
     // arguments launched directly (auto mode captures a key on its second use)

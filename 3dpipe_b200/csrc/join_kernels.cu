@@ -644,17 +644,96 @@ __global__ void k_collect_keys(JoinDev d, long long n2, unsigned long long none,
     }
 }
 
+__device__ __forceinline__ void write_row(const JoinDev& d, const JoinRows& o, int64_t i, int q, int t, int64_t p,
+                                          const double* __restrict__ pexact) {
+    if (i >= o.cap) return;
+    o.q[i] = q;
+    o.t[i] = t;
+    o.d[i] = d.pmx[p];
+    if (o.d64) o.d64[i] = pexact ? pexact[p] : (double)d.pmx[p];
+}
+__device__ __forceinline__ void write_header(const JoinRows& o, unsigned rows) {  // one block
+    if (threadIdx.x == 0) o.head->rows = rows;
+    if (threadIdx.x < 32) o.head->counters[threadIdx.x] = o.counters[threadIdx.x];
+    if (threadIdx.x < 2) o.head->stats[threadIdx.x] = o.stats[threadIdx.x];
+    if (threadIdx.x == 2) o.head->stats[2] = *o.fetched;
+}
+
 __global__ void k_split(JoinDev d, const unsigned long long* __restrict__ keys, const int* __restrict__ vals,
                         long long n2, unsigned long long none, const double* __restrict__ pexact,
-                        int* __restrict__ oq, int* __restrict__ ot, float* __restrict__ od, double* __restrict__ od64) {
+                        const unsigned* __restrict__ rows, JoinRows out) {
+    if (blockIdx.x == 0) write_header(out, *rows);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < d.P; i += (int64_t)gridDim.x * blockDim.x) {
         const unsigned long long k = keys[i];
         if (k == none) break;  // sorted: every later key is `none` too
-        const int p = vals[i];
-        oq[i] = (int)(k / (unsigned long long)n2);
-        ot[i] = (int)(k % (unsigned long long)n2);
-        od[i] = d.pmx[p];
-        if (od64) od64[i] = pexact ? pexact[p] : (double)d.pmx[p];
+        write_row(d, out, i, (int)(k / (unsigned long long)n2), (int)(k % (unsigned long long)n2), vals[i], pexact);
+    }
+}
+
+// reported candidates of every query, one warp a query
+__global__ void __launch_bounds__(kBlock) k_row_counts(JoinDev d, int64_t* __restrict__ cnt) {
+    const int lane = threadIdx.x & 31;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < d.N1; q += nw) {
+        int n = 0;
+        for (int64_t p = d.qoff[q] + lane; p < d.qoff[q + 1]; p += 32) n += d.pstat[p] == kReported;
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) cnt[q] = n;
+    }
+}
+
+// The rows of every query, one warp a query: a pair's place is the number of
+// reported candidates with a smaller result id (kNN lists are in order of
+// distance; within lists are in order of id, and a place is a prefix count).
+// off: the rows before each query; NULL: each block adds up the counts itself
+// (a block's 4,096 counts are 16 loads a thread; the scan is two more launches).
+__global__ void __launch_bounds__(kBlock) k_rows(JoinDev d, int knn_all, const int64_t* __restrict__ cnt,
+                                                 const int64_t* __restrict__ off, const double* __restrict__ pexact,
+                                                 JoinRows out) {
+    __shared__ int64_t part[kBlock / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int q0 = blockIdx.x * (kBlock / 32); q0 < d.N1; q0 += gridDim.x * (kBlock / 32)) {
+        const int q = q0 + w;
+        int64_t at = 0;
+        if (off) {
+            at = off[min(q, d.N1)];
+        } else {
+            int64_t n = 0;
+            for (int k = threadIdx.x; k < q0; k += kBlock) n += cnt[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+            __syncthreads();
+            if (lane == 0) part[w] = n;
+            __syncthreads();
+            for (int k = 0; k < kBlock / 32; ++k) at += part[k];
+            for (int k = q0; k < min(q, d.N1); ++k) at += cnt[k];
+        }
+        if (q0 + kBlock / 32 >= d.N1) {  // the block of the last query
+            if (q == d.N1 - 1 && lane == 0) part[0] = at + cnt[q];
+            __syncthreads();
+            write_header(out, (unsigned)part[0]);
+        }
+        if (q >= d.N1) continue;
+        const int64_t b = d.qoff[q], e = d.qoff[q + 1];
+        if (d.qk ? d.qk[q] > 0 : knn_all) {
+            for (int64_t p = b + lane; p < e; p += 32) {
+                if (d.pstat[p] != kReported) continue;
+                const int t = d.pt[p];
+                int before = 0;
+#pragma unroll 4
+                for (int64_t k = b; k < e; ++k) before += d.pstat[k] == kReported && d.pt[k] < t;
+                write_row(d, out, at + before, q, t, p, pexact);
+            }
+        } else {
+            for (int64_t p0 = b; p0 < e; p0 += 32) {
+                const int64_t p = p0 + lane;
+                const bool rep = p < e && d.pstat[p] == kReported;
+                const unsigned m = __ballot_sync(0xffffffffu, rep);
+                if (rep) write_row(d, out, at + __popc(m & lt), q, d.pt[p], p, pexact);
+                at += __popc(m);
+            }
+        }
     }
 }
 
@@ -742,8 +821,8 @@ cudaError_t collect_sort_bytes(int64_t P, long long n1, long long n2, size_t& by
                                            key_bits((unsigned long long)n1 * (unsigned long long)n2));
 }
 cudaError_t launch_collect(const JoinDev& d, long long n2, unsigned long long* keys[2], int* vals[2], void* temp,
-                           size_t temp_bytes, unsigned* counter, const double* pexact, int* oq, int* ot, float* od,
-                           double* od64, cudaStream_t s) {
+                           size_t temp_bytes, unsigned* counter, const double* pexact, const JoinRows& out,
+                           cudaStream_t s) {
     if (d.P <= 0) return cudaSuccess;
     const unsigned long long none = (unsigned long long)d.N1 * (unsigned long long)n2;
     k_collect_keys<<<grid_for(d.P, 256), 256, 0, s>>>(d, n2, none, keys[0], vals[0], counter);
@@ -753,7 +832,19 @@ cudaError_t launch_collect(const JoinDev& d, long long n2, unsigned long long* k
     cub::DoubleBuffer<int> v(vals[0], vals[1]);
     e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, k, v, (int)d.P, 0, key_bits(none), s);
     if (e != cudaSuccess) return e;
-    k_split<<<grid_for(d.P, 256), 256, 0, s>>>(d, k.Current(), v.Current(), n2, none, pexact, oq, ot, od, od64);
+    k_split<<<grid_for(d.P, 256), 256, 0, s>>>(d, k.Current(), v.Current(), n2, none, pexact, counter, out);
+    return cudaGetLastError();
+}
+cudaError_t launch_collect_ranked(const JoinDev& d, int knn, int64_t* cnt, int64_t* off, void* temp, size_t temp_bytes,
+                                  const double* pexact, const JoinRows& out, cudaStream_t s) {
+    if (d.P <= 0) return cudaSuccess;
+    k_row_counts<<<grid_for(d.N1, kBlock / 32), kBlock, 0, s>>>(d, cnt);
+    cudaError_t e = cudaGetLastError();
+    const bool own = d.N1 <= kOwnPrefix;
+    if (e == cudaSuccess && !own) e = cudaMemsetAsync(cnt + d.N1, 0, 8, s);
+    if (e == cudaSuccess && !own) e = scan_counts(cnt, off, d.N1, temp, temp_bytes, s);
+    if (e != cudaSuccess) return e;
+    k_rows<<<grid_for(d.N1, kBlock / 32), kBlock, 0, s>>>(d, knn, cnt, own ? nullptr : off, pexact, out);
     return cudaGetLastError();
 }
 

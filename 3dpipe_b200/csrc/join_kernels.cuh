@@ -93,17 +93,35 @@ cudaError_t launch_recheck_finish(const JoinDev& d, const double* res, const int
                                   double* pexact, int knn, int K, float tau, cudaStream_t s,
                                   const unsigned* W_dev = nullptr);
 cudaError_t launch_count_status(const JoinDev& d, unsigned* counters, cudaStream_t s);
-// Reported pairs as (query, result id, distance) rows sorted by (query,
-// result id) on the device: the first *counter rows of out_q/out_t/out_d
-// (out_d = the pair's upper bound pmx; out_d64, if not NULL, = pexact when
-// given, else pmx widened).  keys[0..1] / vals[0..1] are P-element double
-// buffers for the radix sort, temp its workspace of collect_sort_bytes()
-// bytes; n2 is the tile-2 object count.
+// What a join reads back beside its rows.
+struct JoinHeader {
+    unsigned rows;
+    unsigned counters[32];           // the context's work counters from word 8
+    unsigned long long stats[3];     // full evaluations, filter voxel pairs, bytes fetched
+};
+// Where the rows go.
+struct JoinRows {
+    JoinHeader* head;
+    int *q, *t;
+    float* d;                        // the pair's upper bound pmx
+    double* d64;                     // if not NULL: pexact when given, else pmx widened
+    int64_t cap;
+    const unsigned* counters;        // the header's sources
+    const unsigned long long *stats, *fetched;
+};
+// Reported pairs as (query, result id, distance) rows sorted by (query, result
+// id).  Ranked: every query's candidates are ordered by its own warp (cnt, off:
+// N1 + 1 words each, temp the workspace of scan_counts over N1); the general
+// form sorts (query, result id) keys of every pair (keys[0..1] / vals[0..1] are
+// P-element buffers, temp its workspace of collect_sort_bytes() bytes, counter
+// a zeroed word).  n2 is the tile-2 object count.
+constexpr int kRankRows = 512;       // most candidates of a kNN query in the ranked form
+constexpr int kOwnPrefix = 4096;     // most queries whose blocks add up the counts before theirs
+cudaError_t launch_collect_ranked(const JoinDev& d, int knn, int64_t* cnt, int64_t* off, void* temp, size_t temp_bytes,
+                                  const double* pexact, const JoinRows& out, cudaStream_t s);
 cudaError_t collect_sort_bytes(int64_t P, long long n1, long long n2, size_t& bytes);
 cudaError_t launch_collect(const JoinDev& d, long long n2, unsigned long long* keys[2], int* vals[2], void* temp,
-                           size_t temp_bytes, unsigned* counter, const double* pexact, int* out_q, int* out_t,
-                           float* out_d, double* out_d64, cudaStream_t s);
-// exclusive scan of n int64 counts into out[0..n] (out[n] = total)
+                           size_t temp_bytes, unsigned* counter, const double* pexact, const JoinRows& out, cudaStream_t s);
 cudaError_t scan_counts(const int64_t* cnt, int64_t* out, int n, void* temp, size_t& temp_bytes, cudaStream_t s);
 
 }  // namespace tdp

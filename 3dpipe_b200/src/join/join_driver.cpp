@@ -43,16 +43,37 @@ namespace {
 
 enum Slot {
     kPq = 20, kPt, kQoff, kPmn, kPmx, kPerr, kPstat, kPvp, kQconf, kCnt, kScanTmp, kRankSt,
-    kVpa, kVpb, kVpair, kVmn, kVmx, kVerr, kValive, kVupd, kItems, kItemVp, kRes, kOutQ, kOutT, kOutD,
+    kVpa, kVpb, kVpair, kVmn, kVmx, kVerr, kValive, kVupd, kItems, kItemVp, kRes, kOut,
     kVexact, kPexact, kRes64,
     kKeyA = 60, kKeyB, kValA, kValB,  // result sort (50-59 hold the candidate buffers)
-    kPexOut = 76, kOutD64,            // exact distances (64-75 and 78-81 are the exact stage's own)
+    kPexOut = 76,                     // exact distances (64-75 and 78-81 are the exact stage's own)
     kQk = 82, kQtau,                  // per query object queries
     kPreset = 91,                     // the last LOD's item presets (within queries)
     kLodExt = kLodScratchFirst, kLodVox, kLodMg, kLodCaps, kLodFlags, kLodZero, kLodVres, kLodCl1, kLodCl2, kLodVb1, kLodVb2,
     kLodLists, kLodTasks, kLodOver, kLodEvals, kLodBest, kLodDir,   // the LOD loop's task form
     kPfList = kLodScratchEnd,                                       // voxels to prefetch
 };
+
+// Rows up to here come back in one copy with the counters (1.3 M rows: 0.3 ms at
+// 55 GB/s).  Written by the kernel over the link instead they took as long at
+// 2,000 rows and 30 us more at 21,000.
+constexpr size_t kResultWhole = (size_t)16 << 20;
+
+// the page-locked result buffer, of at least `need` bytes
+bool grow_hres(tdp_ctx* ctx, size_t need) {
+    if (need <= ctx->hres_cap) return true;
+    if (ctx->hres) cudaFreeHost(ctx->hres);
+    ctx->hres = nullptr;
+    ctx->hres_cap = 0;
+    const size_t cap = need + need / 4 + 4096;
+    if (cudaHostAlloc(&ctx->hres, cap, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->hres = nullptr;
+        return false;
+    }
+    ctx->hres_cap = cap;
+    return true;
+}
 
 template <typename T>
 T* buf(tdp_ctx* ctx, int slot) { return (T*)ctx->scratch[slot].p; }
@@ -336,7 +357,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
 #define CU(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) return fail(ctx, TDP_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(_e)); } while (0)
     std::vector<int64_t> qoff;
     std::vector<int32_t> ids, pq;
-    long P = 0;
+    long P = 0, most = 0;
     bool on_device = false;
     const auto c0 = std::chrono::steady_clock::now();
     const int* dqk = nullptr;
@@ -352,7 +373,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     }
     if (tuned) {
         if ((rc = device_candidates(ctx, t1, t2, self, knn, knn ? prm->knn : 0, within_dist, ctx->scratch[kPq],
-                                    ctx->scratch[kPt], ctx->scratch[kQoff], P, st.candidate_redone, dqk, dqtau,
+                                    ctx->scratch[kPt], ctx->scratch[kQoff], P, st.candidate_redone, most, dqk, dqtau,
                                     isect, q_begin, q_end)))
             return rc;
         on_device = true;
@@ -375,7 +396,6 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     ENS(kPq, Pz * 4); ENS(kPt, Pz * 4); ENS(kQoff, (t1->n_obj + 1) * 8);
     ENS(kPmn, Pz * 4); ENS(kPmx, Pz * 4); ENS(kPerr, Pz * 4); ENS(kPstat, Pz);
     ENS(kPvp, (Pz + 1) * 8); ENS(kQconf, (t1->n_obj + 1) * 4); ENS(kCnt, (Pz + 1) * 8); ENS(kRankSt, Pz * 4);
-    ENS(kOutQ, Pz * 4); ENS(kOutT, Pz * 4); ENS(kOutD, Pz * 4);
 
     JoinDev d;
     std::memset(&d, 0, sizeof d);  // padding too: the LOD loop's graph key holds these bytes
@@ -423,9 +443,9 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     CU(scan_counts(cnt, d.pvp, (int)P, nullptr, tmp_bytes, s));
     ENS(kScanTmp, tmp_bytes + 16);
     CU(scan_counts(cnt, d.pvp, (int)P, ctx->scratch[kScanTmp].p, tmp_bytes, s)); ++launches;
-    int64_t V = 0;
-    CU(cudaMemcpyAsync(&V, d.pvp + P, 8, cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(ctx->hwords, d.pvp + P, 8, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
+    const int64_t V = (int64_t)ctx->hwords[0];
     const size_t Vz = (size_t)std::max<int64_t>(V, 1);
     ENS(kVpa, Vz * 4); ENS(kVpb, Vz * 4); ENS(kVpair, Vz * 4); ENS(kVmn, Vz * 4); ENS(kVmx, Vz * 4);
     ENS(kVerr, Vz * 4); ENS(kValive, Vz); ENS(kVupd, Vz * 4);
@@ -615,7 +635,6 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     ExactInfo xi;
     if (exact) {
         ENS(kPexOut, Pz * 8);
-        ENS(kOutD64, Pz * 8);
         pex = buf<double>(ctx, kPexOut);
         CU(cudaEventRecord(ctx->ev[6], s));
         if ((rc = exact_distances(ctx, d, t1, t2, prm->hausdorff_level == 2, pex, xi, lz1, lz2))) return rc;
@@ -625,33 +644,47 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     }
 
     // ---- 5. results ----
-    CU(cudaMemsetAsync(cnt_collect, 0, 4, s));
-    {
-        size_t sort_bytes = 0;
-        CU(collect_sort_bytes(P, t1->n_obj, t2->n_obj, sort_bytes));
-        ENS(kKeyA, Pz * 8); ENS(kKeyB, Pz * 8); ENS(kValA, Pz * 4); ENS(kValB, Pz * 4);
-        ENS(kScanTmp, sort_bytes + 16);
-        unsigned long long* keys[2] = {buf<unsigned long long>(ctx, kKeyA), buf<unsigned long long>(ctx, kKeyB)};
-        int* vals[2] = {buf<int>(ctx, kValA), buf<int>(ctx, kValB)};
-        CU(launch_collect(d, t2->n_obj, keys, vals, ctx->scratch[kScanTmp].p, sort_bytes, cnt_collect, pex,
-                          buf<int>(ctx, kOutQ), buf<int>(ctx, kOutT), buf<float>(ctx, kOutD),
-                          exact ? buf<double>(ctx, kOutD64) : nullptr, s));
+    // The rows (at most `bound`) and the counters come back in one copy, before
+    // the number of rows is known; only where they may be many is it read first.
+    const size_t bound = knn && !mixed ? std::min<size_t>(P, (size_t)t1->n_obj * (size_t)prm->knn) : (size_t)P;
+    const size_t head = (sizeof(JoinHeader) + 63) / 64 * 64;
+    const size_t at_q = head + (exact ? bound * 8 : 0), at_t = at_q + bound * 4, at_d = at_t + bound * 4, out_bytes = at_d + bound * 4;
+    const bool whole = out_bytes <= kResultWhole && grow_hres(ctx, out_bytes);
+    JoinHeader H{};
+    uint8_t* rows_at = nullptr;
+    if (P > 0) {
+        ENS(kOut, out_bytes);
+        rows_at = buf<uint8_t>(ctx, kOut);
+        JoinRows rows{(JoinHeader*)rows_at, (int*)(rows_at + at_q), (int*)(rows_at + at_t), (float*)(rows_at + at_d),
+                      exact ? (double*)(rows_at + head) : nullptr, (int64_t)bound, ctx->d_counter + 8, ctx->d_stats, fetch_ctr};
+        if (on_device && (!any_knn || most <= kRankRows)) {
+            size_t scan_bytes = 0;
+            CU(scan_counts(nullptr, nullptr, (int)t1->n_obj, nullptr, scan_bytes, s));
+            const size_t n1z = (size_t)t1->n_obj + 1;
+            ENS(kKeyA, n1z * 8); ENS(kKeyB, n1z * 8); ENS(kScanTmp, scan_bytes + 16);
+            CU(launch_collect_ranked(d, knn, buf<int64_t>(ctx, kKeyA), buf<int64_t>(ctx, kKeyB),
+                                     ctx->scratch[kScanTmp].p, scan_bytes, pex, rows, s));
+        } else {
+            CU(cudaMemsetAsync(cnt_collect, 0, 4, s));
+            size_t sort_bytes = 0;
+            CU(collect_sort_bytes(P, t1->n_obj, t2->n_obj, sort_bytes));
+            ENS(kKeyA, Pz * 8); ENS(kKeyB, Pz * 8); ENS(kValA, Pz * 4); ENS(kValB, Pz * 4);
+            ENS(kScanTmp, sort_bytes + 16);
+            unsigned long long* keys[2] = {buf<unsigned long long>(ctx, kKeyA), buf<unsigned long long>(ctx, kKeyB)};
+            int* vals[2] = {buf<int>(ctx, kValA), buf<int>(ctx, kValB)};
+            CU(launch_collect(d, t2->n_obj, keys, vals, ctx->scratch[kScanTmp].p, sort_bytes, cnt_collect, pex, rows, s));
+        }
         launches += 2;
     }
     CU(cudaEventRecord(ctx->ev[4], s));
-    unsigned nres = 0;
-    unsigned tc[32] = {0};
-    unsigned long long fe = 0;
-    CU(cudaMemcpyAsync(&nres, cnt_collect, 4, cudaMemcpyDeviceToHost, s));
-    unsigned long long fvp = 0, fetched = 0;
-    CU(cudaMemcpyAsync(&fvp, ctx->d_stats + 1, 8, cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(&fetched, fetch_ctr, 8, cudaMemcpyDeviceToHost, s));
-    if (tuned && V > 0) {
-        CU(cudaMemcpyAsync(tc, ctx->d_counter + 8, 32 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        CU(cudaMemcpyAsync(&fe, ctx->d_stats, 8, cudaMemcpyDeviceToHost, s));
-    }
+    if (P > 0) CU(cudaMemcpyAsync(whole ? ctx->hres : (void*)&H, rows_at, whole ? out_bytes : sizeof H, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     ++syncs;
+    if (P > 0 && whole) std::memcpy(&H, ctx->hres, sizeof H);
+    const unsigned nres = H.rows;
+    if (nres > bound) return fail(ctx, TDP_ERR_CUDA, "more result rows than the query can have");
+    const unsigned* tc = H.counters;
+    const unsigned long long fe = H.stats[0], fvp = H.stats[1], fetched = H.stats[2];
     st.filter_voxel_pairs = (double)fvp;
     st.fetch_bytes = (double)fetched;
     if (tuned && V > 0) {
@@ -672,45 +705,27 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     // rows were sorted by (query, result id) on the device
     tdp_result* R = new tdp_result();
     if (nres) {
-        // through a page-locked staging buffer: a fast copy, then one pass
-        // into the result (no zero-fill of the vectors first)
-        const size_t need = (size_t)nres * (exact ? 20 : 12);
-        if (need > ctx->hres_cap) {
-            if (ctx->hres) cudaFreeHost(ctx->hres);
-            ctx->hres = nullptr;
-            ctx->hres_cap = 0;
-            const size_t cap = need + need / 4 + 4096;
-            if (cudaHostAlloc(&ctx->hres, cap, cudaHostAllocDefault) == cudaSuccess) ctx->hres_cap = cap;
-            else ctx->hres = nullptr;
-        }
-        cudaError_t e;
-        if (ctx->hres) {
-            uint8_t* h = (uint8_t*)ctx->hres;
-            double* h64 = (double*)h;  // 8-byte aligned first
-            int* hq = (int*)(h + (exact ? (size_t)nres * 8 : 0));
-            int* ht = hq + nres;
-            float* hd = (float*)(ht + nres);
-            if (exact) cudaMemcpyAsync(h64, buf<double>(ctx, kOutD64), nres * 8, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(hq, buf<int>(ctx, kOutQ), nres * 4, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(ht, buf<int>(ctx, kOutT), nres * 4, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(hd, buf<float>(ctx, kOutD), nres * 4, cudaMemcpyDeviceToHost, s);
+        const uint8_t* h = (const uint8_t*)ctx->hres;
+        size_t hq = at_q, ht = at_t, hd = at_d;
+        cudaError_t e = cudaSuccess;
+        if (!whole) {
+            // through a page-locked staging buffer: a fast copy, then one pass
+            // into the result (no zero-fill of the vectors first)
+            std::vector<uint8_t> pageable;
+            const size_t need = head + (size_t)nres * (exact ? 20 : 12);
+            if (!grow_hres(ctx, need)) pageable.resize(need);
+            uint8_t* to = pageable.empty() ? (uint8_t*)ctx->hres : pageable.data();
+            hq = head + (exact ? (size_t)nres * 8 : 0);
+            ht = hq + (size_t)nres * 4;
+            hd = ht + (size_t)nres * 4;
+            if (exact) cudaMemcpyAsync(to + head, rows_at + head, (size_t)nres * 8, cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(to + hq, rows_at + at_q, (size_t)nres * 4, cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(to + ht, rows_at + at_t, (size_t)nres * 4, cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(to + hd, rows_at + at_d, (size_t)nres * 4, cudaMemcpyDeviceToHost, s);
             e = cudaStreamSynchronize(s);
-            if (e == cudaSuccess) {
-                R->q.assign(hq, hq + nres);
-                R->t.assign(ht, ht + nres);
-                R->d.assign(hd, hd + nres);
-                if (exact) R->d64.assign(h64, h64 + nres);
-            }
+            R->take(to + head, to + hq, to + ht, to + hd, nres, exact);
         } else {
-            R->q.resize(nres); R->t.resize(nres); R->d.resize(nres);
-            cudaMemcpyAsync(R->q.data(), buf<int>(ctx, kOutQ), nres * 4, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(R->t.data(), buf<int>(ctx, kOutT), nres * 4, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(R->d.data(), buf<float>(ctx, kOutD), nres * 4, cudaMemcpyDeviceToHost, s);
-            if (exact) {
-                R->d64.resize(nres);
-                cudaMemcpyAsync(R->d64.data(), buf<double>(ctx, kOutD64), nres * 8, cudaMemcpyDeviceToHost, s);
-            }
-            e = cudaStreamSynchronize(s);
+            R->take(h + head, h + hq, h + ht, h + hd, nres, exact);
         }
         if (e != cudaSuccess) { delete R; return fail(ctx, TDP_ERR_CUDA, cudaGetErrorString(e)); }
     }
