@@ -25,7 +25,6 @@
 //                orders its query's by rank (a key is preceded by those below
 //                it) while no query has more than kRankMost; beyond that a CUB
 //                segmented sort and k_cand_finish order them.
-#include <cub/device/device_scan.cuh>
 #include <cub/device/device_segmented_sort.cuh>
 #include <float.h>
 
@@ -36,6 +35,7 @@
 #include <vector>
 
 #include "cand_kernels.cuh"
+#include "join_kernels.cuh"
 #include "index/candidates.h"
 
 namespace tdp {
@@ -495,17 +495,15 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
     int found[2] = {0, 0};
     const int& over = found[0];
     for (int pass = 0;; ++pass) {
-        CU(cudaMemsetAsync(cnt + n1, 0, 8, s));
         k_cand_pass<false><<<std::max(pblocks, 1), 256, 0, s>>>(bg, box1, xf1, box2, xf2, fc, (int)n1, self, knn, tau,
                                                                qk, qtau, isect ? 1 : 0, kth, cnt, nullptr, nullptr,
                                                                (int)qb0, (int)qe0, d_over + 1, nullptr, nullptr);
         CU(cudaGetLastError());
         size_t tb = 0;
-        CU(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, qoff, (int)n1 + 1, s));
+        CU(scan_to_host_bytes((int)n1, tb));
         if ((rc = ensure(ctx, tmp, tb + 16))) return rc;
-        CU(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt, qoff, (int)n1 + 1, s));
-        CU(cudaMemcpyAsync(ctx->hwords, qoff + n1, 8, cudaMemcpyDeviceToHost, s));
-        CU(cudaMemcpyAsync(ctx->hwords + 1, d_over, 8, cudaMemcpyDeviceToHost, s));
+        CU(scan_to_host(cnt, qoff, (int)n1, tmp.p, tb, (const unsigned long long*)d_over, ctx->hwords,
+                        ctx->hwords != ctx->pageable_words, s));
         CU(cudaStreamSynchronize(s));
         total = (int64_t)ctx->hwords[0];
         std::memcpy(found, ctx->hwords + 1, 8);

@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_bounds(JoinDev d, int decide, f
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     unsigned long long vp = 0;  // voxel pairs of this warp's object pairs (lane 0)
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < d.N1; q += gridDim.x * blockDim.x) d.qconf[q] = 0;
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < d.P; p += nw) {
         const int q = d.pq[p], t = d.pt[p];
         const uint32_t a0 = d.ovox1[q], a1 = d.ovox1[q + 1], b0 = d.ovox2[t], b1 = d.ovox2[t + 1];
@@ -493,10 +494,29 @@ __global__ void k_apply_results(JoinDev d, const float4* __restrict__ res, const
     }
 }
 
+// undecided and reported pairs (whole warps)
+__device__ __forceinline__ void count_status(const JoinDev& d, unsigned* __restrict__ c) {
+    unsigned und = 0, rep = 0;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < d.P; p += gridDim.x * blockDim.x) {
+        und += d.pstat[p] == kUndecided;
+        rep += d.pstat[p] == kReported;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        und += __shfl_xor_sync(0xffffffffu, und, o);
+        rep += __shfl_xor_sync(0xffffffffu, rep, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (und) atomicAdd(c + 0, und);
+        if (rep) atomicAdd(c + 1, rep);
+    }
+}
+
 // ---- FP64 recheck (tuned form) of pairs still undecided after the last LOD ----
 __global__ void k_recheck_items(JoinDev d, const uint32_t* __restrict__ vt1, const uint32_t* __restrict__ vt2,
                                 RefineItem* __restrict__ items, int* __restrict__ item_vp, double* __restrict__ vexact,
-                                unsigned* __restrict__ counter) {
+                                unsigned* __restrict__ counter, unsigned* __restrict__ status) {
+    count_status(d, status);
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < d.V; v += (int64_t)gridDim.x * blockDim.x) {
         if (!d.valive[v] || d.pstat[d.vpair[v]] != kUndecided) continue;
         vexact[v] = 1e300;
@@ -507,12 +527,6 @@ __global__ void k_recheck_items(JoinDev d, const uint32_t* __restrict__ vt1, con
         items[w] = RefineItem{o1, n1, o2, n2};
         item_vp[w] = (int)v;
     }
-}
-
-__global__ void k_recheck_apply(const double* __restrict__ res, const int* __restrict__ item_vp, int W_host,
-                                const unsigned* W_dev, double* __restrict__ vexact) {
-    const int W = W_dev ? (int)*W_dev : W_host;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < W; w += gridDim.x * blockDim.x) vexact[item_vp[w]] = res[w];
 }
 
 __global__ void __launch_bounds__(kBlock) k_recheck_pairs(JoinDev d, const double* __restrict__ vexact,
@@ -609,22 +623,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_update(JoinDev d, int stamp, in
     }
 }
 
-__global__ void k_count_status(JoinDev d, unsigned* __restrict__ c) {
-    unsigned und = 0, rep = 0;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < d.P; p += gridDim.x * blockDim.x) {
-        und += d.pstat[p] == kUndecided;
-        rep += d.pstat[p] == kReported;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        und += __shfl_xor_sync(0xffffffffu, und, o);
-        rep += __shfl_xor_sync(0xffffffffu, rep, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (und) atomicAdd(c + 0, und);
-        if (rep) atomicAdd(c + 1, rep);
-    }
-}
+__global__ void k_count_status(JoinDev d, unsigned* __restrict__ c) { count_status(d, c); }
 
 // Result keys: query * n2 + result id for reported pairs, `none` (= n1 * n2)
 // for the rest, so one radix sort over every pair puts the reported ones
@@ -790,14 +789,13 @@ cudaError_t launch_pair_update(const JoinDev& d, int stamp, int tuned, cudaStrea
     return cudaGetLastError();
 }
 cudaError_t launch_recheck_items(const JoinDev& d, const uint32_t* vt1, const uint32_t* vt2, RefineItem* items,
-                                 int* item_vp, double* vexact, unsigned* counter, cudaStream_t s) {
+                                 int* item_vp, double* vexact, unsigned* counter, unsigned* status, cudaStream_t s) {
     if (d.V <= 0) return cudaSuccess;
-    k_recheck_items<<<grid_for(d.V, 256), 256, 0, s>>>(d, vt1, vt2, items, item_vp, vexact, counter);
+    k_recheck_items<<<grid_for(d.V, 256), 256, 0, s>>>(d, vt1, vt2, items, item_vp, vexact, counter, status);
     return cudaGetLastError();
 }
-cudaError_t launch_recheck_finish(const JoinDev& d, const double* res, const int* item_vp, int W, double* vexact,
-                                  double* pexact, int knn, int K, float tau, cudaStream_t s, const unsigned* W_dev) {
-    if (W > 0) k_recheck_apply<<<grid_for(W, 256), 256, 0, s>>>(res, item_vp, W, W_dev, vexact);
+cudaError_t launch_recheck_finish(const JoinDev& d, double* vexact, double* pexact, int knn, int K, float tau,
+                                  cudaStream_t s) {
     if (d.P > 0) k_recheck_pairs<<<grid_for(d.P, kBlock / 32), kBlock, 0, s>>>(d, vexact, pexact, !knn, tau);
     if ((knn || d.qk) && d.N1 > 0) k_recheck_knn<<<grid_for(d.N1, 128), 128, 0, s>>>(d, K, pexact);
     return cudaGetLastError();
@@ -846,6 +844,59 @@ cudaError_t launch_collect_ranked(const JoinDev& d, int knn, int64_t* cnt, int64
     if (e != cudaSuccess) return e;
     k_rows<<<grid_for(d.N1, kBlock / 32), kBlock, 0, s>>>(d, knn, cnt, own ? nullptr : off, pexact, out);
     return cudaGetLastError();
+}
+
+namespace {
+constexpr int kScanThreads = 1024, kScanSmall = 16 * kScanThreads;
+
+// Exclusive scan of n counts by one block, each thread a run of them; the total
+// goes to out[n] and, with *extra, to the host's page-locked words.
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(const int64_t* __restrict__ cnt, int64_t* __restrict__ out, int n,
+                                                            const unsigned long long* __restrict__ extra,
+                                                            unsigned long long* __restrict__ host) {
+    __shared__ int64_t sums[kScanThreads / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int per = (n + kScanThreads - 1) / kScanThreads, b = min(n, (int)threadIdx.x * per), e = min(n, b + per);
+    int64_t mine = 0;
+    for (int i = b; i < e; ++i) mine += cnt[i];
+    int64_t inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) sums[w] = inc;
+    __syncthreads();
+    int64_t at = inc - mine;
+    for (int k = 0; k < w; ++k) at += sums[k];
+    for (int i = b; i < e; ++i) {
+        const int64_t c = cnt[i];
+        out[i] = at;
+        at += c;
+    }
+    if (threadIdx.x == kScanThreads - 1) {
+        out[n] = at;
+        host[0] = (unsigned long long)at;
+        if (extra) host[1] = *extra;
+    }
+}
+}  // namespace
+
+cudaError_t scan_to_host_bytes(int n, size_t& bytes) {
+    bytes = 0;
+    return n <= kScanSmall ? cudaSuccess : scan_counts(nullptr, nullptr, n, nullptr, bytes, nullptr);
+}
+cudaError_t scan_to_host(int64_t* cnt, int64_t* out, int n, void* temp, size_t temp_bytes, const unsigned long long* extra,
+                         unsigned long long* host, bool host_locked, cudaStream_t s) {
+    if (n <= kScanSmall && host_locked) {
+        k_scan_small<<<1, kScanThreads, 0, s>>>(cnt, out, n, extra, host);
+        return cudaGetLastError();
+    }
+    cudaError_t e = cudaMemsetAsync(cnt + n, 0, 8, s);
+    if (e == cudaSuccess) e = scan_counts(cnt, out, n, temp, temp_bytes, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host, out + n, 8, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && extra) e = cudaMemcpyAsync(host + 1, extra, 8, cudaMemcpyDeviceToHost, s);
+    return e;
 }
 
 cudaError_t scan_counts(const int64_t* cnt, int64_t* out, int n, void* temp, size_t& temp_bytes, cudaStream_t s) {

@@ -87,11 +87,12 @@ cudaError_t launch_apply_results(const JoinDev& d, const float4* res, const int*
 // decide != 0 also takes the within decision (k_within_decide) of each pair
 cudaError_t launch_pair_update(const JoinDev& d, int stamp, int tuned, cudaStream_t s, int decide = 0, float tau = 0.f);
 // tuned form: FP64 recheck of the pairs left undecided after LOD 100
+// items of the undecided pairs; status: undecided and reported pairs (added)
 cudaError_t launch_recheck_items(const JoinDev& d, const uint32_t* vtri1, const uint32_t* vtri2, RefineItem* items,
-                                 int* item_vp, double* vexact, unsigned* counter, cudaStream_t s);
-cudaError_t launch_recheck_finish(const JoinDev& d, const double* res, const int* item_vp, int W, double* vexact,
-                                  double* pexact, int knn, int K, float tau, cudaStream_t s,
-                                  const unsigned* W_dev = nullptr);
+                                 int* item_vp, double* vexact, unsigned* counter, unsigned* status, cudaStream_t s);
+// the pairs decided by vexact, the items' FP64 distances by voxel pair
+cudaError_t launch_recheck_finish(const JoinDev& d, double* vexact, double* pexact, int knn, int K, float tau,
+                                  cudaStream_t s);
 cudaError_t launch_count_status(const JoinDev& d, unsigned* counters, cudaStream_t s);
 // What a join reads back beside its rows.
 struct JoinHeader {
@@ -123,5 +124,12 @@ cudaError_t collect_sort_bytes(int64_t P, long long n1, long long n2, size_t& by
 cudaError_t launch_collect(const JoinDev& d, long long n2, unsigned long long* keys[2], int* vals[2], void* temp,
                            size_t temp_bytes, unsigned* counter, const double* pexact, const JoinRows& out, cudaStream_t s);
 cudaError_t scan_counts(const int64_t* cnt, int64_t* out, int n, void* temp, size_t& temp_bytes, cudaStream_t s);
+// The same (cnt[n] need not be 0), the total and *extra also into host[0], [1]
+// once the stream is done: up to 16,384 counts by one block that writes
+// page-locked host words itself (one launch instead of two, a memset and two
+// copies: 8 us less), else by scan_counts with scan_to_host_bytes of workspace.
+cudaError_t scan_to_host_bytes(int n, size_t& bytes);
+cudaError_t scan_to_host(int64_t* cnt, int64_t* out, int n, void* temp, size_t temp_bytes, const unsigned long long* extra,
+                         unsigned long long* host, bool host_locked, cudaStream_t s);
 
 }  // namespace tdp

@@ -46,6 +46,8 @@
 
 #include <float.h>
 
+#include <algorithm>
+
 #include "cull.cuh"
 #include "lod_kernels.cuh"
 #include "pair_rules.cuh"
@@ -66,6 +68,21 @@ enum Mode {
 
 
 __device__ __forceinline__ float sqrt_up(float x) { return radius_sqrt(fmaxf(x, 0.f)); }
+
+// ---------------------------------------------------------------- init
+__global__ void __launch_bounds__(256) k_lod_init(LodDev L, unsigned* words, int n_words, unsigned long long* dstats,
+                                                  size_t caps, size_t best, size_t flags, size_t zero) {
+    const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    if (i0 < (size_t)n_words) words[i0] = 0;
+    if (i0 == 0) *dstats = 0;
+    for (size_t i = i0; i < caps; i += step) L.pcap[i] = __uint_as_float(0x7f7f7f7fu);  // above any bound; pd too
+    for (size_t i = i0; i < best; i += step) {
+        L.pbest[i] = ~0ull;
+        L.dir[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (size_t i = i0; i < flags; i += step) L.flag1[i] = -1;  // flag2 too
+    for (size_t i = i0; i < zero; i += step) L.ctr[i] = 0;      // pown and pmiss too
+}
 
 // ---------------------------------------------------------------- items
 // One thread per voxel pair.  A pair all of whose voxel pairs, once refined,
@@ -1128,6 +1145,14 @@ cudaError_t refine_pass(const LodDev& L, int k, int pass, const unsigned* n_item
 }
 
 }  // namespace
+
+cudaError_t launch_lod_init(const LodDev& L, unsigned* words, int n_words, unsigned long long* dstats, size_t caps_bytes,
+                            size_t best_bytes, size_t flags_bytes, size_t zero_bytes, cudaStream_t s) {
+    const size_t most = std::max({caps_bytes, 2 * best_bytes, flags_bytes, zero_bytes});
+    k_lod_init<<<blocks_for((int64_t)(most / 4), 256, L.num_sms * 8), 256, 0, s>>>(L, words, n_words, dstats, caps_bytes / 4, best_bytes / 8,
+                                                                           flags_bytes / 4, (zero_bytes + 3) / 4);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_lod_items(const LodDev& L, int k, cudaStream_t s) {
     k_lod_items<<<blocks_for(L.d.V, 256, L.num_sms * 32), 256, 0, s>>>(L, k);

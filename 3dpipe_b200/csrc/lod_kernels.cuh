@@ -102,6 +102,11 @@ __device__ __forceinline__ void lod_claim(bool want, int voxel, int stamp, int* 
 }
 #endif
 
+// the loop's state before its first LOD, in one launch instead of seven memsets
+// (n_words counters and dstats 0; caps far, seeds and stamps ~0, the rest of L 0;
+// every size a multiple of 4 bytes or rounded up to one within its buffer)
+cudaError_t launch_lod_init(const LodDev& L, unsigned* words, int n_words, unsigned long long* dstats, size_t caps_bytes,
+                            size_t best_bytes, size_t flags_bytes, size_t zero_bytes, cudaStream_t s);
 cudaError_t launch_lod_items(const LodDev& L, int k, cudaStream_t s);
 // clusters, (first LOD) seeds, cull, tests and evaluation of LOD k's items
 cudaError_t launch_lod_refine(const LodDev& L, int k, int highest, cudaStream_t s);

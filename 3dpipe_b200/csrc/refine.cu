@@ -1051,7 +1051,8 @@ constexpr int kF64Block = 128, kF64Cluster = 8;
 __global__ void __cluster_dims__(kF64Cluster, 1, 1) __launch_bounds__(kF64Block) refine_f64_kernel(const float4* __restrict__ triA,
                                                                const float4* __restrict__ triB,
                                                                const RefineItem* __restrict__ items, int n_items_host,
-                                                               const unsigned* n_items_dev, double* __restrict__ out) {
+                                                               const unsigned* n_items_dev, double* __restrict__ out,
+                                                               const int* __restrict__ at) {
     __shared__ double red[kF64Block / 32];
     __shared__ double share;
     const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -1096,18 +1097,18 @@ __global__ void __cluster_dims__(kF64Cluster, 1, 1) __launch_bounds__(kF64Block)
                 const double v = *cl.map_shared_rank(&share, k);
                 best = v < best ? v : best;
             }
-            out[it] = (w.a_cnt && w.b_cnt) ? sqrt(best) : 1e300;
+            out[at ? at[it] : it] = (w.a_cnt && w.b_cnt) ? sqrt(best) : 1e300;
         }
         cl.sync();  // and read: the next item's may be written, or the block end
     }
 }
 
 cudaError_t launch_refine_f64(const float4* triA, const float4* triB, const RefineItem* items, int n_items,
-                              double* out, cudaStream_t s, const unsigned* n_items_dev) {
+                              double* out, cudaStream_t s, const unsigned* n_items_dev, const int* at) {
     if (n_items <= 0) return cudaSuccess;
     const int clusters = n_items < 148 * 2 ? n_items : 148 * 2;
     const int grid = clusters * kF64Cluster;
-    refine_f64_kernel<<<grid, kF64Block, 0, s>>>(triA, triB, items, n_items, n_items_dev, out);
+    refine_f64_kernel<<<grid, kF64Block, 0, s>>>(triA, triB, items, n_items, n_items_dev, out, at);
     return cudaGetLastError();
 }
 

@@ -26,7 +26,8 @@ cudaError_t launch_refine_tuned(const float4* triA, const float4* triB, const Re
 // exact FP64 minimum distance per item (recheck of undecided object pairs)
 // n_items is an upper bound when n_items_dev (the exact count, in device memory) is given
 cudaError_t launch_refine_f64(const float4* triA, const float4* triB, const RefineItem* items, int n_items,
-                              double* out, cudaStream_t s, const unsigned* n_items_dev = nullptr);
+                              double* out, cudaStream_t s, const unsigned* n_items_dev = nullptr,
+                              const int* at = nullptr);  // item i's distance goes to out[at[i]] (at NULL: out[i])
 // out[i] = the least of parts [first[i], first[i + 1]) by component, the largest w
 cudaError_t launch_merge_parts(const float4* parts, const uint32_t* first, int n, float4* out, cudaStream_t s);
 // *odd (optional) becomes 1 when a value is infinite or not a number

@@ -44,7 +44,7 @@ namespace {
 enum Slot {
     kPq = 20, kPt, kQoff, kPmn, kPmx, kPerr, kPstat, kPvp, kQconf, kCnt, kScanTmp, kRankSt,
     kVpa, kVpb, kVpair, kVmn, kVmx, kVerr, kValive, kVupd, kItems, kItemVp, kRes, kOut,
-    kVexact, kPexact, kRes64,
+    kVexact, kPexact,
     kKeyA = 60, kKeyB, kValA, kValB,  // result sort (50-59 hold the candidate buffers)
     kPexOut = 76,                     // exact distances (64-75 and 78-81 are the exact stage's own)
     kQk = 82, kQtau,                  // per query object queries
@@ -99,7 +99,7 @@ struct LodLoop {
     int64_t V;
     float tau;
     int* rankst;
-    double *vexact, *res64, *pexact;
+    double *vexact, *pexact;
     // within queries with LOD 100 last: each last-LOD item's preset (its
     // query's distance plus the FP32 error band), so that the refine drops the
     // items and triangle pairs that cannot come within it; NULL otherwise
@@ -124,13 +124,7 @@ int enqueue_task_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captu
     auto rec = [&](cudaEvent_t e) {
         return capturing ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
     };
-    CUL(cudaMemsetAsync(L.counter + 8, 0, 26 * sizeof(unsigned), s));
-    CUL(cudaMemsetAsync(L.dstats, 0, 8, s));
-    CUL(cudaMemsetAsync(L.t.pcap, 0x7f, L.caps_bytes, s));     // 3.4e38: above any bound
-    CUL(cudaMemsetAsync(L.t.dir, 0, L.best_bytes * 2, s));
-    CUL(cudaMemsetAsync(L.t.pbest, 0xff, L.best_bytes, s));
-    CUL(cudaMemsetAsync(L.t.flag1, 0xff, L.flags_bytes, s));
-    CUL(cudaMemsetAsync(L.t.ctr, 0, L.zero_bytes, s));
+    CUL(launch_lod_init(L.t, L.counter + 8, 26, L.dstats, L.caps_bytes, L.best_bytes, L.flags_bytes, L.zero_bytes, s));
     const bool prefetch = (L.lz1.on || L.lz2.on) && L.side;
     for (int k = 0; k < L.nl; ++k) {
         const int highest = k == L.highest_k;
@@ -208,12 +202,11 @@ int enqueue_lod_loop(tdp_ctx* ctx, const LodLoop& L, cudaStream_t s, bool captur
     }
     }
     if (L.recheck) {
-        CUL(launch_count_status(L.d, cnt_recheck, s));
-        CUL(cudaMemsetAsync(cnt_items, 0, 4, s));
-        CUL(launch_recheck_items(L.d, L.vt1_100, L.vt2_100, L.items, L.item_vp, L.vexact, cnt_items, s));
+        if (!L.tasks) CUL(cudaMemsetAsync(cnt_items, 0, 4, s));  // (the task form leaves it 0)
+        CUL(launch_recheck_items(L.d, L.vt1_100, L.vt2_100, L.items, L.item_vp, L.vexact, cnt_items, cnt_recheck, s));
         // (its voxel pairs were items of LOD 100: nothing to fetch)
-        CUL(launch_refine_f64(L.tri1_100, L.tri2_100, L.items, V, L.res64, s, cnt_items));
-        CUL(launch_recheck_finish(L.d, L.res64, L.item_vp, V, L.vexact, L.pexact, L.knn, L.K, L.tau, s, cnt_items));
+        CUL(launch_refine_f64(L.tri1_100, L.tri2_100, L.items, V, L.vexact, s, cnt_items, L.item_vp));
+        CUL(launch_recheck_finish(L.d, L.vexact, L.pexact, L.knn, L.K, L.tau, s));
     }
 #undef CUL
     return TDP_OK;
@@ -422,14 +415,13 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         }
         CU(cudaMemcpyAsync((void*)d.qoff, qoff.data(), qoff.size() * 8, cudaMemcpyHostToDevice, s));
     }
-    CU(cudaMemsetAsync(d.qconf, 0, t1->n_obj * 4, s));
-    CU(cudaMemsetAsync(ctx->d_stats + 1, 0, 8, s));
+    if (P == 0) CU(cudaMemsetAsync(d.qconf, 0, t1->n_obj * 4, s));  // (k_pair_bounds clears it)
+    CU(cudaMemsetAsync(ctx->d_stats + 1, 0, 64, s));  // filter voxel pairs .. bytes fetched
     // attached tiles: voxels fetched on demand, bytes counted per join
     LazyTile lz1 = lazy_view(t1), lz2 = lazy_view(t2);
     unsigned long long* fetch_ctr = ctx->d_stats + 8;
     if (lz1.on) lz1.bytes = fetch_ctr;
     if (lz2.on) lz2.bytes = fetch_ctr;
-    CU(cudaMemsetAsync(fetch_ctr, 0, 8, s));
     d.stat_vp = ctx->d_stats + 1;
     long launches = 0;
 
@@ -437,13 +429,12 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     CU(launch_pair_bounds(d, s, any_within, within_dist, tuned)); ++launches;
     if (any_knn) { CU(launch_knn_rank(d, prm->knn, tuned, buf<int>(ctx, kRankSt), s)); ++launches; }
     int64_t* cnt = buf<int64_t>(ctx, kCnt);
-    CU(cudaMemsetAsync(cnt + P, 0, 8, s));
     CU(launch_count_vps(d, !knn, within_dist, tuned, cnt, s)); ++launches;
     size_t tmp_bytes = 0;
-    CU(scan_counts(cnt, d.pvp, (int)P, nullptr, tmp_bytes, s));
+    CU(scan_to_host_bytes((int)P, tmp_bytes));
     ENS(kScanTmp, tmp_bytes + 16);
-    CU(scan_counts(cnt, d.pvp, (int)P, ctx->scratch[kScanTmp].p, tmp_bytes, s)); ++launches;
-    CU(cudaMemcpyAsync(ctx->hwords, d.pvp + P, 8, cudaMemcpyDeviceToHost, s));
+    CU(scan_to_host(cnt, d.pvp, (int)P, ctx->scratch[kScanTmp].p, tmp_bytes, nullptr, ctx->hwords,
+                    ctx->hwords != ctx->pageable_words, s)); ++launches;
     CU(cudaStreamSynchronize(s));
     const int64_t V = (int64_t)ctx->hwords[0];
     const size_t Vz = (size_t)std::max<int64_t>(V, 1);
@@ -515,7 +506,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         // tuned form: every count stays on the device, so the whole loop (and
         // the FP64 recheck) is enqueued without a host round trip; kernels with
         // nothing left to do exit at once
-        ENS(kVexact, Vz * 8); ENS(kPexact, Pz * 8); ENS(kRes64, Vz * 8);
+        ENS(kVexact, Vz * 8); ENS(kPexact, Pz * 8);
         const bool presets = any_within && !isect && lods.back() == 100;
         if (presets) ENS(kPreset, Vz * 4);
         // 3b. after LOD 100, the FP64 recheck of pairs whose FP32 ranges
@@ -543,7 +534,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         L.any_knn = any_knn; L.any_within = any_within; L.K = prm->knn; L.knn = knn;
         L.V = V; L.tau = within_dist;
         L.rankst = buf<int>(ctx, kRankSt);
-        L.vexact = buf<double>(ctx, kVexact); L.res64 = buf<double>(ctx, kRes64); L.pexact = buf<double>(ctx, kPexact);
+        L.vexact = buf<double>(ctx, kVexact); L.pexact = buf<double>(ctx, kPexact);
         L.lz1 = lz1; L.lz2 = lz2;
         L.preset = presets ? buf<float>(ctx, kPreset) : nullptr;
         L.side = ctx->side;
@@ -571,7 +562,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             L.caps_bytes = 2 * Pz * 4;
             L.best_bytes = Pz * 8;
             L.flags_bytes = (nv1 + nv2) * 4;
-            L.zero_bytes = ctr_bytes + 2 * Pz;
+            L.zero_bytes = ctr_bytes + (2 * Pz + 3) / 4 * 4;
             const struct { int slot; size_t bytes; } need[] = {
                 {kLodExt, Vz * sizeof(int4)}, {kLodVox, Vz * sizeof(int2)}, {kLodMg, Vz * sizeof(float4)},
                 {kLodCaps, L.caps_bytes}, {kLodBest, L.best_bytes}, {kLodDir, 2 * L.best_bytes},
@@ -624,7 +615,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             // (task form: six a LOD, the seeds of the first and four of the redo)
             launches += ((L.tasks ? 6 : 4) + (L.any_knn ? 1 : 0) + (attached ? (L.tasks ? 1 : 2) : 0)) * L.nl + (L.tasks ? 5 : 0) +
                         (attached && L.side ? 2 * (L.nl - 1) : 0) +
-                        (L.recheck ? (knn ? 5 : 4) : 0);
+                        (L.recheck ? (knn ? 4 : 3) : 0);
         }
         st.refine_launches += L.nl;
     }

@@ -59,3 +59,16 @@ def test_coinciding_transforms_are_ordered_by_id(pkg, ctx):
             np.testing.assert_array_equal(off, hoff)
             np.testing.assert_array_equal(ids, hids)
     T.free()
+
+
+@pytest.mark.parametrize("nv,npv", [(1, 1), (5, 205), (16, 1024), (5, 3277)])
+def test_offsets_where_the_scan_changes(pkg, ctx, nv, npv):
+    """1, 1,025, 16,384 and 16,385 queries: one block's scan, or the general one."""
+    raw, _ = pkg.tdp.gen_tiles(nv, npv, seed=54, nucleus_subdiv=1, only="nuclei")
+    T = pkg.tdp.Tile(ctx, raw)
+    b, x = _boxes(raw)
+    off, ids = pkg.tdp.tile_candidates(ctx, T, None, within=3.0)
+    hoff, hids = pkg.tdp.candidates(b, x, b, x, self_join=True, within=3.0)
+    np.testing.assert_array_equal(off, hoff)
+    np.testing.assert_array_equal(ids, hids)
+    T.free()
