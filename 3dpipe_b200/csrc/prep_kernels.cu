@@ -45,6 +45,7 @@
 // vessels 191 -> 34 ms, 1,000 nuclei of 1,280 facets 7.7 -> 4.6 ms).  This file
 // is built with -fmad=false: every product and sum is rounded on its own, as on
 // the host.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cub/device/device_scan.cuh>
@@ -589,6 +590,11 @@ __device__ __forceinline__ uint32_t nearest_core(double3 p, const float* P, cons
 }
 
 // ------------------------------------------------------------------ voxels
+// A cluster of C blocks per object (1 for many objects, so that the chip is
+// full either way): the FP64 nearest-seed and nearest-core searches, which bound
+// it, are spread over all its threads, the small prefix sums are its first
+// block's.  6 vessels of 20,160 facets: 14.1 ms with one block of 256 threads
+// each, 8.9 with 1,024, 3.3 with eight blocks of 1,024.
 template <int T>
 __global__ void __launch_bounds__(T) k_voxels(Meshes M, int voxel_size, const uint32_t* __restrict__ lodF,
                                               const uint32_t* __restrict__ lodCnt, VoxScratch S,
@@ -596,9 +602,17 @@ __global__ void __launch_bounds__(T) k_voxels(Meshes M, int voxel_size, const ui
     constexpr int NW = T / 32;
     __shared__ double s_v[NW];
     __shared__ uint32_t s_i[NW], s_red[NW];
-    __shared__ uint32_t s_cur, s_nvox;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int o = blockIdx.x; o < M.n; o += gridDim.x) {
+    __shared__ double best_v[2];    // the block's farthest vertex, by the round's parity
+    __shared__ uint32_t best_i[2];
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t tid = rank * T + threadIdx.x, TT = C * T;  // within the cluster
+    auto sync = [&] {
+        if (C == 1) __syncthreads();
+        else cl.sync();
+    };
+    for (int o = blockIdx.x / C; o < M.n; o += gridDim.x / C) {
         const int64_t v0 = M.voff[o], f0 = M.foff[o], s0 = S.soff[o];
         const uint32_t n = (uint32_t)(M.voff[o + 1] - v0), m = (uint32_t)(M.foff[o + 1] - f0);
         const uint32_t ns = m / (uint32_t)voxel_size + 1;
@@ -607,6 +621,7 @@ __global__ void __launch_bounds__(T) k_voxels(Meshes M, int voxel_size, const ui
         double* sd = S.seed + 3 * s0;
         double* dmin = S.dmin + v0;
         uint32_t* asg = S.asg + v0;
+        volatile uint32_t* nvox_at = S.nvox + o;
         // 2a. farthest-point seeds from vertex 0
         uint32_t cur = 0;
         for (uint32_t s = 0; s < ns; ++s) {
@@ -614,36 +629,44 @@ __global__ void __launch_bounds__(T) k_voxels(Meshes M, int voxel_size, const ui
             if (tid == 0) { sd[3 * s] = c.x; sd[3 * s + 1] = c.y; sd[3 * s + 2] = c.z; }
             double bv = -1.0;
             uint32_t bi = UINT_MAX;
-            for (uint32_t i = tid; i < n; i += T) {
+            auto better = [&](double v2, uint32_t i2) {
+                if (v2 > bv || (v2 == bv && i2 < bi)) { bv = v2; bi = i2; }
+            };
+            for (uint32_t i = tid; i < n; i += TT) {
                 const double d = sqrt(dist2(vtx(P, i), c));
                 const double dm = s == 0 ? d : fmin(dmin[i], d);
                 dmin[i] = dm;
                 if (dm > bv) { bv = dm; bi = i; }
             }
 #pragma unroll
-            for (int k = 16; k > 0; k >>= 1) {
-                const double v2 = __shfl_xor_sync(0xffffffffu, bv, k);
-                const uint32_t i2 = __shfl_xor_sync(0xffffffffu, bi, k);
-                if (v2 > bv || (v2 == bv && i2 < bi)) { bv = v2; bi = i2; }
-            }
+            for (int k = 16; k > 0; k >>= 1)
+                better(__shfl_xor_sync(0xffffffffu, bv, k), __shfl_xor_sync(0xffffffffu, bi, k));
             if (lane == 0) { s_v[wid] = bv; s_i[wid] = bi; }
             __syncthreads();
-            if (tid == 0) {
-                for (int w = 1; w < NW; ++w)
-                    if (s_v[w] > bv || (s_v[w] == bv && s_i[w] < bi)) { bv = s_v[w]; bi = s_i[w]; }
-                s_cur = bi;
+            if (wid == 0) {
+                bv = lane < NW ? s_v[lane] : -1.0;
+                bi = lane < NW ? s_i[lane] : UINT_MAX;
+#pragma unroll
+                for (int k = 16; k > 0; k >>= 1)
+                    better(__shfl_xor_sync(0xffffffffu, bv, k), __shfl_xor_sync(0xffffffffu, bi, k));
+                if (lane == 0) { best_v[s & 1] = bv; best_i[s & 1] = bi; }
             }
-            __syncthreads();
-            cur = s_cur;
+            sync();  // (the other parity's values are read until the next round's)
+            bv = best_v[s & 1];
+            bi = best_i[s & 1];
+            for (int k = 0; k < C; ++k)
+                if (k != rank) better(*cl.map_shared_rank(&best_v[s & 1], k), *cl.map_shared_rank(&best_i[s & 1], k));
+            cur = bi;
         }
+        sync();
         // 2b. two Lloyd steps
         for (int it = 0; it < 2; ++it) {
-            for (uint32_t i = tid; i < n; i += T) {
+            for (uint32_t i = tid; i < n; i += TT) {
                 double d;
                 asg[i] = nearest(vtx(P, i), sd, ns, d);
             }
-            __syncthreads();
-            for (uint32_t s = tid; s < ns; s += T) {  // sums in vertex order
+            sync();
+            for (uint32_t s = tid; s < ns; s += TT) {  // sums in vertex order
                 double ax = 0.0, ay = 0.0, az = 0.0;
                 uint32_t cnt = 0;
                 for (uint32_t i = 0; i < n; ++i)
@@ -657,15 +680,15 @@ __global__ void __launch_bounds__(T) k_voxels(Meshes M, int voxel_size, const ui
                     sd[3 * s] = ax * r; sd[3 * s + 1] = ay * r; sd[3 * s + 2] = az * r;
                 }
             }
-            __syncthreads();
+            sync();
         }
         // 2c. facets to seeds by barycentre; a seed's nearest facet gives its core
         unsigned long long* bestd = S.bestd + s0;
         uint32_t* bestf = S.bestf + s0;
-        for (uint32_t s = tid; s < ns; s += T) { bestd[s] = ~0ull; bestf[s] = UINT_MAX; }
-        __syncthreads();
+        for (uint32_t s = tid; s < ns; s += TT) { bestd[s] = ~0ull; bestf[s] = UINT_MAX; }
+        sync();
         for (int pass = 0; pass < 2; ++pass) {
-            for (uint32_t f = tid; f < m; f += T) {
+            for (uint32_t f = tid; f < m; f += TT) {
                 const double3 a = vtx(P, F100[3 * f]), b = vtx(P, F100[3 * f + 1]), c = vtx(P, F100[3 * f + 2]);
                 const double k3 = 1.0 / 3.0;
                 const double3 q = make_double3(((a.x + b.x) + c.x) * k3, ((a.y + b.y) + c.y) * k3, ((a.z + b.z) + c.z) * k3);
@@ -675,78 +698,87 @@ __global__ void __launch_bounds__(T) k_voxels(Meshes M, int voxel_size, const ui
                 if (pass == 0) atomicMin(bestd + g, bits);
                 else if (bestd[g] == bits) atomicMin(bestf + g, f);
             }
-            __syncthreads();
+            sync();
         }
         uint32_t* core = S.core + s0;
-        uint32_t nvox = 0;
-        for (uint32_t c0 = 0; c0 < ns; c0 += T) {  // cores of the seeds with a facet, in seed order
-            const uint32_t s = c0 + tid;
-            const bool has = s < ns && bestf[s] != UINT_MAX;
-            const uint32_t fb = has ? bestf[s] : 0;
-            uint32_t total;
-            const uint32_t at = block_count_before<T>(has, s_red, total);
-            if (has) core[nvox + at] = F100[3 * fb];
-            nvox += total;
-        }
-        __syncthreads();
-        // 3. LOD-100 triangles to cores; keep the cores that receive one
         uint32_t* cnt100 = S.vcnt + (size_t)(kNumLods - 1) * S.Stot + s0;
-        for (uint32_t v = tid; v < nvox; v += T) cnt100[v] = 0;
-        __syncthreads();
-        for (uint32_t f = tid; f < m; f += T) atomicAdd(cnt100 + nearest_core(vtx(P, F100[3 * f]), P, core, nvox), 1u);
-        __syncthreads();
-        uint32_t kept = 0;
-        for (uint32_t c0 = 0; c0 < nvox; c0 += T) {  // in place: kept cores move down
-            const uint32_t v = c0 + tid;
-            const bool has = v < nvox && cnt100[v] > 0;
-            const uint32_t cv = has ? core[v] : 0;
-            uint32_t total;
-            const uint32_t at = block_count_before<T>(has, s_red, total);
-            if (has) core[kept + at] = cv;
-            kept += total;
-            __syncthreads();
+        if (rank == 0) {
+            uint32_t found = 0;
+            for (uint32_t c0 = 0; c0 < ns; c0 += T) {  // cores of the seeds with a facet, in seed order
+                const uint32_t s = c0 + threadIdx.x;
+                const bool has = s < ns && bestf[s] != UINT_MAX;
+                const uint32_t fb = has ? bestf[s] : 0;
+                uint32_t total;
+                const uint32_t at = block_count_before<T>(has, s_red, total);
+                if (has) core[found + at] = F100[3 * fb];
+                found += total;
+            }
+            for (uint32_t v = threadIdx.x; v < found; v += T) cnt100[v] = 0;
+            if (threadIdx.x == 0) *nvox_at = found;
         }
-        nvox = kept;
+        sync();
+        // 3. LOD-100 triangles to cores; keep the cores that receive one
+        uint32_t nvox = *nvox_at;
+        for (uint32_t f = tid; f < m; f += TT) atomicAdd(cnt100 + nearest_core(vtx(P, F100[3 * f]), P, core, nvox), 1u);
+        sync();
+        if (rank == 0) {
+            uint32_t kept = 0;
+            for (uint32_t c0 = 0; c0 < nvox; c0 += T) {  // in place: kept cores move down
+                const uint32_t v = c0 + threadIdx.x;
+                const bool has = v < nvox && cnt100[v] > 0;
+                const uint32_t cv = has ? core[v] : 0;
+                uint32_t total;
+                const uint32_t at = block_count_before<T>(has, s_red, total);
+                if (has) core[kept + at] = cv;
+                kept += total;
+                __syncthreads();
+            }
+            if (threadIdx.x == 0) *nvox_at = kept;
+        }
+        sync();
+        nvox = *nvox_at;
         // every LOD: triangles to the kept voxels, grouped by voxel in LOD order
         uint32_t ntri = 0;
         for (int l = 0; l < kNumLods; ++l) {
             const uint32_t* LF = l < kNumLods - 1 ? lodF + (size_t)l * 3 * S.Ftot + 3 * f0 : F100;
-            const uint32_t cl = l < kNumLods - 1 ? lodCnt[(size_t)o * kDecLods + l] : m;
+            const uint32_t cl_n = l < kNumLods - 1 ? lodCnt[(size_t)o * kDecLods + l] : m;
             uint32_t* tv = S.tvox + (size_t)l * S.Ftot + f0;
             uint32_t* od = S.ord + (size_t)l * S.Ftot + f0;
             uint32_t* vc = S.vcnt + (size_t)l * S.Stot + s0;
             uint32_t* vs = S.vst + (size_t)l * S.Stot + s0;
-            for (uint32_t v = tid; v < nvox; v += T) vc[v] = 0;
-            __syncthreads();
-            for (uint32_t t = tid; t < cl; t += T) {
+            for (uint32_t v = tid; v < nvox; v += TT) vc[v] = 0;
+            sync();
+            for (uint32_t t = tid; t < cl_n; t += TT) {
                 const uint32_t g = nearest_core(vtx(P, LF[3 * t]), P, core, nvox);
                 tv[t] = g;
                 atomicAdd(vc + g, 1u);
             }
-            __syncthreads();
-            uint32_t run = 0;
-            for (uint32_t c0 = 0; c0 < nvox; c0 += T) {
-                const uint32_t v = c0 + tid;
-                const uint32_t x = v < nvox ? vc[v] : 0;
-                uint32_t total;
-                const uint32_t at = block_excl_sum<T>(x, s_red, total);
-                if (v < nvox) vs[v] = run + at;
-                run += total;
+            sync();
+            if (rank == 0) {
+                uint32_t run = 0;
+                for (uint32_t c0 = 0; c0 < nvox; c0 += T) {
+                    const uint32_t v = c0 + threadIdx.x;
+                    const uint32_t x = v < nvox ? vc[v] : 0;
+                    uint32_t total;
+                    const uint32_t at = block_excl_sum<T>(x, s_red, total);
+                    if (v < nvox) vs[v] = run + at;
+                    run += total;
+                }
             }
-            __syncthreads();
-            for (uint32_t v = tid; v < nvox; v += T) {  // stable: each voxel walks the LOD in order
+            sync();
+            for (uint32_t v = tid >> 5; v < nvox; v += TT >> 5) {  // stable: a warp per voxel walks the LOD in order
                 uint32_t c = vs[v];
-                for (uint32_t t = 0; t < cl; ++t)
-                    if (tv[t] == v) od[c++] = t;
+                for (uint32_t t0 = 0; t0 < cl_n; t0 += 32) {
+                    const bool mine = t0 + lane < cl_n && tv[t0 + lane] == v;
+                    const unsigned ms = __ballot_sync(0xffffffffu, mine);
+                    if (mine) od[c + __popc(ms & ((1u << lane) - 1u))] = t0 + lane;
+                    c += __popc(ms);
+                }
             }
-            ntri += cl;
-            __syncthreads();
+            ntri += cl_n;
         }
-        if (tid == 0) {
-            S.nvox[o] = nvox;
-            obj_bytes[o] = 68ull + 44ull * ntri + 116ull * nvox;
-        }
-        __syncthreads();
+        if (tid == 0) obj_bytes[o] = 68ull + 44ull * ntri + 116ull * nvox;
+        sync();
     }
 }
 
@@ -1112,10 +1144,24 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
         unsigned long long *dbytes, *dpos;
         CU(dm.get(&dbytes, (size_t)nb));
         CU(dm.get(&dpos, (size_t)nb));
-        // fewer objects than SMs: more threads for each (6 vessels of 20,160
-        // facets 14.1 -> 8.9 ms; the FP64 nearest-seed searches wait on latency)
-        if (nb < ctx->num_sms) k_voxels<1024><<<(int)nb, 1024, 0, s>>>(Mh, voxel_size, lodF, lodCnt, S, dbytes);
-        else k_voxels<kPrepThreads><<<(int)nb, kPrepThreads, 0, s>>>(Mh, voxel_size, lodF, lodCnt, S, dbytes);
+        // fewer objects than SMs: more threads for each, and as many blocks as fit
+        if (nb < ctx->num_sms) {
+            int C = 1;
+            while (C < 8 && 2 * C * nb <= ctx->num_sms) C *= 2;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = (unsigned)C;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(nb * C));
+            cfg.blockDim = dim3(1024);
+            cfg.stream = s;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            CU(cudaLaunchKernelEx(&cfg, k_voxels<1024>, Mh, voxel_size, (const uint32_t*)lodF, (const uint32_t*)lodCnt, S, dbytes));
+        } else {
+            k_voxels<kPrepThreads><<<(int)nb, kPrepThreads, 0, s>>>(Mh, voxel_size, lodF, lodCnt, S, dbytes);
+        }
         CU(cudaGetLastError());
         CU(cudaEventRecord(ev[2], s));
         bytes.assign(nb, 0);
