@@ -134,6 +134,7 @@ struct tdp_server {
     std::mutex mu;
     std::condition_variable cv;
     std::deque<Request*> pending;
+    Request* held = nullptr;       // the admitter's current request, until it is appended or failed
     std::unordered_map<uint64_t, std::unique_ptr<Request>> table;
     uint64_t next_id = 1;
     long batches = 0, completed = 0, failed = 0, split_batches = 0;
@@ -303,7 +304,7 @@ void admitter_loop(tdp_server* S) {
         if (!cur) {
             S->cv.wait(lk, [&] { return S->stop || !S->pending.empty(); });
             if (S->stop) return;
-            cur = S->pending.front();
+            cur = S->held = S->pending.front();
             S->pending.pop_front();
             t_cur = Clock::now();
             lk.unlock();
@@ -373,12 +374,17 @@ void admitter_loop(tdp_server* S) {
             else finish(S, r, rc);
             S->cv.notify_all();
         }
-        cur = nxt;
+        cur = S->held = nxt;
         cur_rc = nxt_rc;
         t_cur = t_nxt;
         j = 1 - j;
     }
 }
+
+// A lone request waits this long for one that the admitter already has, if the
+// arena has room for both: a join takes 0.5 ms and more whatever its size, and
+// the next one's bytes are usually there before that.
+constexpr auto kCompany = std::chrono::microseconds(1000);
 
 void executor_loop(tdp_server* S) {
     tdp_ctx* ctx = S->ctx;
@@ -386,6 +392,7 @@ void executor_loop(tdp_server* S) {
     std::vector<int> obj_knn;
     std::vector<float> obj_within;
     std::unique_lock<std::mutex> lk(S->mu);
+    Request* waited = nullptr;  // the lone request that has had its wait
     for (;;) {
         Arena* a = nullptr;
         S->cv.wait(lk, [&] {
@@ -396,6 +403,15 @@ void executor_loop(tdp_server* S) {
             return S->stop;
         });
         if (!a) return;  // stopping with nothing admitted left to run
+        if (a->state == ArenaState::kFilling && a->reqs.size() == 1 && a->reqs[0] != waited) {
+            waited = a->reqs[0];
+            S->cv.wait_for(lk, kCompany, [&] {
+                const Request* next = S->held ? S->held : S->pending.empty() ? nullptr : S->pending.front();
+                return S->stop || a->state != ArenaState::kFilling || a->reqs.size() > 1 ||
+                       (!a->appending && (!next || !fits(S, *a, *next)));
+            });
+            continue;  // (it may be in the middle of an append: looked at again)
+        }
         a->state = ArenaState::kRunning;
         const long batch = S->batches++;
         const auto t_start = Clock::now();
