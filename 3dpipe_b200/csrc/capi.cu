@@ -23,16 +23,12 @@ void cache_trim(tdp_ctx* ctx) {
 
 bool lod_scratch_drop(tdp_ctx* ctx) {
     if (ctx->lod_busy) return false;
-    bool any = false;
-    for (int k = kLodScratchFirst; k < kLodScratchEnd; ++k) {
-        Buf& b = ctx->scratch[k];
-        if (!b.p) continue;
-        if (!any) cudaStreamSynchronize(ctx->stream);
-        any = true;
-        dfree(ctx, b.p);
-        b = Buf{};
-    }
-    return any;
+    Buf& b = ctx->scratch[kLodScratch];
+    if (!b.p) return false;
+    cudaStreamSynchronize(ctx->stream);
+    dfree(ctx, b.p);
+    b = Buf{};
+    return true;
 }
 
 cudaError_t dmalloc(tdp_ctx* ctx, void** p, size_t bytes) {

@@ -681,8 +681,6 @@ constexpr int64_t kChunk = 1 << 19;
 // stage's own slots); false when it does not fit.
 bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t2, size_t Pz) {
     if (!t1->d_boxes || !t2->d_boxes) return false;
-    enum { kCl1 = kLodScratchFirst + 7, kCl2, kVb1, kVb2, kLists, kTasks, kOver, kEvals, kFlags = kLodScratchFirst + 4,
-           kCtr = kLodScratchFirst + 5 };  // the LOD loop's slots
     const size_t E = (size_t)L.d.V;
     L.self = t1 == t2;
     L.nl = 1;
@@ -710,15 +708,28 @@ bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t
     };
     const bool ok = get(67, E * sizeof(RefineItem), &L.items) && get(72, E * sizeof(int4), &L.ext) &&
                     get(74, E * sizeof(int2), &L.vox) && get(69, E * sizeof(float4), &L.mg) && get(68, E * 4, &L.vres) &&
-                    get(73, E * 4, &L.d.vmx) && get(81, E * 4, &L.d.vupd) && get(kOver, C * 4, &L.over) &&
-                    get(70, Pz * 4, &L.pd) && get(71, 2 * Pz, &L.pown) && get(kFlags, nv * 4, &L.flag1) &&
-                    get(kLists, nv * 4, &L.list1) && get(kCtr, (E / kChunk + 1) * kLodCtrWords * sizeof(unsigned), &L.ctr) &&
-                    get(kCl1, c1 * 3 * sizeof(float4), &L.cl1) && get(kVb1, (size_t)L.nvox1 * 2 * sizeof(float4), &L.vb1) &&
-                    (L.self || (get(kCl2, c2 * 3 * sizeof(float4), &L.cl2) &&
-                                get(kVb2, (size_t)L.nvox2 * 2 * sizeof(float4), &L.vb2))) &&
-                    get(kTasks, (size_t)L.task_cap * sizeof(LodTask), &L.tasks) &&
-                    get(kEvals, (size_t)L.eval_cap * sizeof(LodEval), &L.evals);
+                    get(73, E * 4, &L.d.vmx) && get(81, E * 4, &L.d.vupd) && get(70, Pz * 4, &L.pd) &&
+                    get(71, 2 * Pz, &L.pown);
     if (!ok) return false;
+    // the LOD loop's block: that loop is done with it
+    Carve c;
+    const size_t over = c.take(C * 4), flag = c.take(nv * 4), list = c.take(nv * 4);
+    const size_t words = c.take((E / kChunk + 1) * kLodCtrWords * sizeof(unsigned));
+    const size_t cl1 = c.take(c1 * 3 * sizeof(float4)), vb1 = c.take((size_t)L.nvox1 * 2 * sizeof(float4));
+    const size_t cl2 = c.take(L.self ? 0 : c2 * 3 * sizeof(float4)), vb2 = c.take((size_t)L.nvox2 * 2 * sizeof(float4));
+    const size_t tasks = c.take((size_t)L.task_cap * sizeof(LodTask)), evals = c.take((size_t)L.eval_cap * sizeof(LodEval));
+    if (ensure(ctx, ctx->scratch[kLodScratch], c.bytes) != TDP_OK) return false;
+    char* base = (char*)ctx->scratch[kLodScratch].p;
+    L.over = (unsigned*)(base + over);
+    L.flag1 = (int*)(base + flag);
+    L.list1 = (int*)(base + list);
+    L.ctr = (unsigned*)(base + words);
+    L.cl1 = (float4*)(base + cl1);
+    L.vb1 = (float4*)(base + vb1);
+    L.cl2 = (float4*)(base + cl2);
+    L.vb2 = (float4*)(base + vb2);
+    L.tasks = (LodTask*)(base + tasks);
+    L.evals = (LodEval*)(base + evals);
     L.pmiss = L.pown + Pz;
     if (L.self) {
         L.cl2 = L.cl1;

@@ -49,9 +49,7 @@ enum Slot {
     kPexOut = 76,                     // exact distances (64-75 and 78-81 are the exact stage's own)
     kQk = 82, kQtau,                  // per query object queries
     kPreset = 91,                     // the last LOD's item presets (within queries)
-    kLodExt = kLodScratchFirst, kLodVox, kLodMg, kLodCaps, kLodFlags, kLodZero, kLodVres, kLodCl1, kLodCl2, kLodVb1, kLodVb2,
-    kLodLists, kLodTasks, kLodOver, kLodEvals, kLodBest, kLodDir,   // the LOD loop's task form
-    kPfList = kLodScratchEnd,                                       // voxels to prefetch
+    kPfList = kLodScratch + 1,        // voxels to prefetch
 };
 
 // Rows up to here come back in one copy with the counters (1.3 M rows: 0.3 ms at
@@ -548,6 +546,9 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         L.tasks = 1;
         for (int k = 0; k < L.nl; ++k) L.tasks = L.tasks && L.cfg[k] == 0;
         LodScratchUse in_use(ctx);
+        // the task form's arrays, by their offsets in its block
+        enum { kExt, kVox, kMg, kCaps, kBest, kDir, kFlags, kZero, kVres, kCl1, kVb1, kCl2, kVb2, kLists, kOver, kTasks, kEvals, kArrays };
+        size_t at[kArrays] = {};
         if (L.tasks) {
             LodDev& t = L.t;
             size_t c1 = 0, c2 = 0;  // cluster records of a LOD: at most one per 8 triangles and one more per voxel
@@ -563,16 +564,14 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             L.best_bytes = Pz * 8;
             L.flags_bytes = (nv1 + nv2) * 4;
             L.zero_bytes = ctr_bytes + (2 * Pz + 3) / 4 * 4;
-            const struct { int slot; size_t bytes; } need[] = {
-                {kLodExt, Vz * sizeof(int4)}, {kLodVox, Vz * sizeof(int2)}, {kLodMg, Vz * sizeof(float4)},
-                {kLodCaps, L.caps_bytes}, {kLodBest, L.best_bytes}, {kLodDir, 2 * L.best_bytes},
-                {kLodFlags, L.flags_bytes}, {kLodZero, L.zero_bytes}, {kLodVres, Vz * 4},
-                {kLodCl1, c1 * 3 * sizeof(float4)}, {kLodVb1, nv1 * 2 * sizeof(float4)},
-                {kLodCl2, self ? 0 : c2 * 3 * sizeof(float4)}, {kLodVb2, self ? 0 : nv2 * 2 * sizeof(float4)},
-                {kLodLists, (nv1 + nv2) * 4}, {kLodOver, Vz * 4}, {kLodTasks, (size_t)t.task_cap * sizeof(LodTask)},
-                {kLodEvals, (size_t)t.eval_cap * sizeof(LodEval)}};
-            for (const auto& n : need)
-                if (n.bytes && L.tasks && ensure(ctx, ctx->scratch[n.slot], n.bytes) != TDP_OK) L.tasks = 0;
+            const size_t need[kArrays] = {
+                Vz * sizeof(int4), Vz * sizeof(int2), Vz * sizeof(float4), L.caps_bytes, L.best_bytes, 2 * L.best_bytes,
+                L.flags_bytes, L.zero_bytes, Vz * 4, c1 * 3 * sizeof(float4), nv1 * 2 * sizeof(float4),
+                self ? 0 : c2 * 3 * sizeof(float4), nv2 * 2 * sizeof(float4), (nv1 + nv2) * 4, Vz * 4,
+                (size_t)t.task_cap * sizeof(LodTask), (size_t)t.eval_cap * sizeof(LodEval)};
+            Carve c;
+            for (int a = 0; a < kArrays; ++a) at[a] = c.take(need[a]);
+            if (ensure(ctx, ctx->scratch[kLodScratch], c.bytes) != TDP_OK) L.tasks = 0;
         }
         if (!L.tasks) {  // no room for the queues: the refine of one warp per voxel pair
             cudaGetLastError();
@@ -588,20 +587,21 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             for (int k = 0; k < L.nl; ++k) {
                 t.vt1[k] = L.vt1[k]; t.vt2[k] = L.vt2[k]; t.tri1[k] = L.tri1[k]; t.tri2[k] = L.tri2[k]; t.li[k] = L.li[k];
             }
-            t.items = items; t.ext = buf<int4>(ctx, kLodExt); t.vox = buf<int2>(ctx, kLodVox); t.mg = buf<float4>(ctx, kLodMg);
-            t.pbest = buf<unsigned long long>(ctx, kLodBest); t.evals = buf<LodEval>(ctx, kLodEvals);
-            t.dir = buf<float4>(ctx, kLodDir);
-            t.pcap = buf<float>(ctx, kLodCaps); t.pd = t.pcap + Pz;
-            t.ctr = buf<unsigned>(ctx, kLodZero);
+            char* base = buf<char>(ctx, kLodScratch);
+            t.items = items; t.ext = (int4*)(base + at[kExt]); t.vox = (int2*)(base + at[kVox]); t.mg = (float4*)(base + at[kMg]);
+            t.pbest = (unsigned long long*)(base + at[kBest]); t.evals = (LodEval*)(base + at[kEvals]);
+            t.dir = (float4*)(base + at[kDir]);
+            t.pcap = (float*)(base + at[kCaps]); t.pd = t.pcap + Pz;
+            t.ctr = (unsigned*)(base + at[kZero]);
             t.pown = (uint8_t*)t.ctr + ctr_bytes; t.pmiss = t.pown + Pz;
-            t.vres = buf<float>(ctx, kLodVres);
-            t.cl1 = buf<float4>(ctx, kLodCl1); t.vb1 = buf<float4>(ctx, kLodVb1);
-            t.cl2 = self ? t.cl1 : buf<float4>(ctx, kLodCl2); t.vb2 = self ? t.vb1 : buf<float4>(ctx, kLodVb2);
-            t.flag1 = buf<int>(ctx, kLodFlags); t.flag2 = self ? t.flag1 : t.flag1 + nv1;
-            t.list1 = buf<int>(ctx, kLodLists); t.list2 = self ? t.list1 : t.list1 + nv1;
+            t.vres = (float*)(base + at[kVres]);
+            t.cl1 = (float4*)(base + at[kCl1]); t.vb1 = (float4*)(base + at[kVb1]);
+            t.cl2 = self ? t.cl1 : (float4*)(base + at[kCl2]); t.vb2 = self ? t.vb1 : (float4*)(base + at[kVb2]);
+            t.flag1 = (int*)(base + at[kFlags]); t.flag2 = self ? t.flag1 : t.flag1 + nv1;
+            t.list1 = (int*)(base + at[kLists]); t.list2 = self ? t.list1 : t.list1 + nv1;
             t.nvox1 = (long)nv1; t.nvox2 = (long)nv2;
-            t.tasks = buf<LodTask>(ctx, kLodTasks);
-            t.over = buf<unsigned>(ctx, kLodOver);
+            t.tasks = (LodTask*)(base + at[kTasks]);
+            t.over = (unsigned*)(base + at[kOver]);
             t.n_items = ctx->d_counter + 24;
             t.tri_pairs = (unsigned long long*)(ctx->d_counter + 10);
             t.n_full = ctx->d_stats;
