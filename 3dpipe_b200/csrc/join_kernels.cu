@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(kBlock) k_row_counts(JoinDev d, int64_t* __res
 __global__ void __launch_bounds__(kBlock) k_rows(JoinDev d, int knn_all, const int64_t* __restrict__ cnt,
                                                  const int64_t* __restrict__ off, const double* __restrict__ pexact,
                                                  JoinRows out) {
-    __shared__ int64_t part[kBlock / 32];
+    __shared__ int64_t part[kBlock / 32], all;  // (all: apart from part, which other warps may still be adding up)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     for (int q0 = blockIdx.x * (kBlock / 32); q0 < d.N1; q0 += gridDim.x * (kBlock / 32)) {
@@ -709,9 +709,9 @@ __global__ void __launch_bounds__(kBlock) k_rows(JoinDev d, int knn_all, const i
             for (int k = q0; k < min(q, d.N1); ++k) at += cnt[k];
         }
         if (q0 + kBlock / 32 >= d.N1) {  // the block of the last query
-            if (q == d.N1 - 1 && lane == 0) part[0] = at + cnt[q];
+            if (q == d.N1 - 1 && lane == 0) all = at + cnt[q];
             __syncthreads();
-            write_header(out, (unsigned)part[0]);
+            write_header(out, (unsigned)all);
         }
         if (q >= d.N1) continue;
         const int64_t b = d.qoff[q], e = d.qoff[q + 1];
