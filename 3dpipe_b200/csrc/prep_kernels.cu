@@ -918,7 +918,8 @@ __global__ void __launch_bounds__(T) k_write(Meshes M, const uint32_t* __restric
         for (uint32_t i = tid; i < n; i += T) {
             const float dx = P[3 * (size_t)i] - cx, dy = P[3 * (size_t)i + 1] - cy, dz = P[3 * (size_t)i + 2] - cz;
             const float d = dx * dx + dy * dy + dz * dz;
-            if (d < bd) { bd = d; bi = i; }
+            // (FP32 squares overflow on meshes of 1e19 units: all infinite, the lowest index)
+            if (d < bd || bi == UINT_MAX) { bd = d; bi = i; }
         }
 #pragma unroll
         for (int k = 16; k > 0; k >>= 1) {
