@@ -171,6 +171,12 @@ __device__ inline float rmax32(float v) {
     return r;
 }
 
+// no more than the length of (x, y, z >= 0), also where its square overflows
+__device__ inline float length_down(float x, float y, float z) {
+    const float s = x * x + y * y + z * z;
+    return (s < INFINITY ? sqrtf(s) : fmaxf(x, fmaxf(y, z))) * 0.999999f;
+}
+
 // one copy of the FP64 distance in a kernel
 __device__ __noinline__ double point_tri2(D3 p, D3 a, D3 b, D3 c) { return pd::tri2_dev(p, a, b, c); }
 
@@ -346,8 +352,9 @@ __device__ inline void search(Search<K>& S, int n, const float4* T, const uint32
             if (!mask) {
                 if (base >= ve) return;
                 const uint32_t w = base + lane;
-                float gap = INFINITY;
-                if (w < ve && w != first && VT[w] != VT[w + 1]) {
+                const bool other = w < ve && w != first && VT[w] != VT[w + 1];
+                float gap = 0.f;
+                if (other) {
                     const float4 lo = box[2 * (size_t)w], hi = box[2 * (size_t)w + 1];
                     ulx = lo.x - ox; uly = lo.y - oy; ulz = lo.z - oz;
                     uhx = hi.x - ox; uhy = hi.y - oy; uhz = hi.z - oz;
@@ -355,10 +362,10 @@ __device__ inline void search(Search<K>& S, int n, const float4* T, const uint32
                                 z = fmaxf(fmaxf(ulz - bhz, blz - uhz), 0.f);
                     const float mg = 4e-6f * (fmaxf(fabsf(ulx), fabsf(uhx)) + fmaxf(fabsf(uly), fabsf(uhy)) +
                                               fmaxf(fabsf(ulz), fabsf(uhz)) + scale) + 1e-6f;
-                    gap = sqrtf(x * x + y * y + z * z) * 0.999999f - mg;
+                    gap = length_down(x, y, z) - mg;
                 }
                 const float most = rmax32(on ? bf : 0.f);
-                mask = __ballot_sync(0xffffffffu, gap < INFINITY && !(gap > most));
+                mask = __ballot_sync(0xffffffffu, other && !(gap > most));  // (what is not a number is looked at)
                 base += 32;
                 continue;
             }
@@ -372,7 +379,7 @@ __device__ inline void search(Search<K>& S, int n, const float4* T, const uint32
             for (int c = 0; c < K; ++c) {
                 const float x = fmaxf(fmaxf(ax - Q.x[c], Q.x[c] - ex), 0.f), y = fmaxf(fmaxf(ay - Q.y[c], Q.y[c] - ey), 0.f),
                             z = fmaxf(fmaxf(az - Q.z[c], Q.z[c] - ez), 0.f);
-                near = near && !(sqrtf(x * x + y * y + z * z) * 0.999999f - mg > bf);
+                near = near && !(length_down(x, y, z) - mg > bf);
             }
             if (!__any_sync(0xffffffffu, near)) continue;
             u = base - 32 + k;
