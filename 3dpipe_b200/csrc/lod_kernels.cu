@@ -768,7 +768,9 @@ __global__ void __launch_bounds__(kTestWarps * 32, 5) k_lod_test(LodDev L, int k
                 const float z = za + __shfl_sync(kFull, s.z, lb);
                 const float y = MODE == kLast ? 0.f : ya + __shfl_sync(kFull, s.y, lb);
                 const bool ky = MODE != kLast && !(y >= T.yt);
-                const bool keep = live && (!(z >= T.zt) || ky);
+                // (a bound that is not a number passes: a missing triangle's too, beside one that has none)
+                const bool there = (hl & 7) < (int)(T.n & 0xffu) && bj < (int)(T.n >> 8);
+                const bool keep = live && there && (!(z >= T.zt) || ky);
                 const unsigned km = __ballot_sync(kFull, keep);
                 if (!km) continue;
                 if (keep) buf[bn + __popc(km & lt)] = LodEval{T.w, T.a0 + (hl & 7), T.b0 + bj, ky ? -INFINITY : z};
