@@ -51,6 +51,7 @@
 #include "cull.cuh"
 #include "lod_kernels.cuh"
 #include "pair_rules.cuh"
+#include "task_queue.cuh"
 #include "tridist.cuh"
 
 namespace tdp {
@@ -471,11 +472,14 @@ constexpr int kSide = 16;     // clusters of one side that are looked at togethe
 
 // Queue `cnt` of the warp's collected tasks.  Items whose tasks find the
 // queue full go to the list of items that are evaluated whole, once each.
-__device__ __forceinline__ void flush_tasks(const LodDev& L, unsigned* ctr, const LodTask* buf, int cnt, int lane) {
+__device__ __forceinline__ void flush_tasks(const LodDev& L, unsigned* ctr, const LodTask* buf, int cnt, int lane,
+                                            QueueClaims& queue) {
     __syncwarp();
-    unsigned base = 0;
-    if (lane == 0) base = atomicAdd(ctr + cTasks, (unsigned)cnt);
-    base = __shfl_sync(kFull, base, 0);
+    const unsigned base = queue.claim((unsigned)cnt, L.task_cap, [&](unsigned n) {
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(ctr + cTasks, n);
+        return __shfl_sync(kFull, at, 0);
+    });
     for (int i = lane; i < cnt; i += 32) {
         const LodTask t = buf[i];
         if (base + i < L.task_cap) L.tasks[base + i] = t;
@@ -532,6 +536,7 @@ __global__ void __launch_bounds__(kCullWarps * 32) k_lod_cull(LodDev L, int k, i
     LodTask* buf = bufs[wid];
     CullItem* rec = recs[wid];
     int bn = 0;
+    QueueClaims queue;
     unsigned* ctr = L.ctr + pass * kLodCtrWords;
     const unsigned n = *n_items;
     const unsigned nw = gridDim.x * kCullWarps, gw = blockIdx.x * kCullWarps + wid;
@@ -635,7 +640,7 @@ __global__ void __launch_bounds__(kCullWarps * 32) k_lod_cull(LodDev L, int k, i
                     if (go) buf[bn + __popc(m & lt)] = t;
                     bn += __popc(m);
                     if (bn >= 64) {
-                        flush_tasks(L, ctr, buf, bn, lane);
+                        flush_tasks(L, ctr, buf, bn, lane, queue);
                         bn = 0;
                     }
                     c += 32;
@@ -649,7 +654,7 @@ __global__ void __launch_bounds__(kCullWarps * 32) k_lod_cull(LodDev L, int k, i
         }
         __syncwarp();
     }
-    if (bn > 0) flush_tasks(L, ctr, buf, bn, lane);
+    if (bn > 0) flush_tasks(L, ctr, buf, bn, lane, queue);
 }
 
 // ---------------------------------------------------------------- triangle tests
@@ -721,7 +726,7 @@ __global__ void __launch_bounds__(kTestWarps * 32, 5) k_lod_test(LodDev L, int k
     const float4* tri1 = L.tri1[k];
     const float4* tri2 = L.tri2[k];
     const float4* cl2 = L.self ? L.cl1 : L.cl2;
-    auto flush = [&] {
+    auto flush = [&] {  // (at most 64 for each of the tasks: the counter does not wrap)
         __syncwarp();
         unsigned base = 0;
         if (lane == 0) base = atomicAdd(ctr + cEvals, (unsigned)bn);
