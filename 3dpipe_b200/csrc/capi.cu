@@ -122,6 +122,12 @@ int ensure(tdp_ctx* ctx, Buf& b, size_t bytes) {
     return TDP_OK;
 }
 
+bool lod_scratch(tdp_ctx* ctx, size_t bytes) {
+    Buf& b = ctx->scratch[kLodScratch];
+    if (b.cap < bytes && 2 * b.cap > bytes && ensure(ctx, b, 2 * b.cap) == TDP_OK) return true;
+    return ensure(ctx, b, bytes) == TDP_OK;
+}
+
 // FP32 FMA throughput probe: 8 independent FMA chains per thread.
 __global__ void fma_probe_kernel(float* out, int iters, float b, float c) {
     float a[8];

@@ -138,6 +138,9 @@ struct Carve {
         return at;
     }
 };
+// the block with at least `bytes`, grown to twice its size where there is room
+// (growing waits for the device twice); false without room
+bool lod_scratch(tdp_ctx* ctx, size_t bytes);
 bool lod_scratch_drop(tdp_ctx* ctx);
 struct LodScratchUse {
     tdp_ctx* ctx;

@@ -718,7 +718,7 @@ bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t
     const size_t cl1 = c.take(c1 * 3 * sizeof(float4)), vb1 = c.take((size_t)L.nvox1 * 2 * sizeof(float4));
     const size_t cl2 = c.take(L.self ? 0 : c2 * 3 * sizeof(float4)), vb2 = c.take((size_t)L.nvox2 * 2 * sizeof(float4));
     const size_t tasks = c.take((size_t)L.task_cap * sizeof(LodTask)), evals = c.take((size_t)L.eval_cap * sizeof(LodEval));
-    if (ensure(ctx, ctx->scratch[kLodScratch], c.bytes) != TDP_OK) return false;
+    if (!lod_scratch(ctx, c.bytes)) return false;
     char* base = (char*)ctx->scratch[kLodScratch].p;
     L.over = (unsigned*)(base + over);
     L.flag1 = (int*)(base + flag);

@@ -52,10 +52,16 @@ enum Slot {
     kPfList = kLodScratch + 1,        // voxels to prefetch
 };
 
-// Rows up to here come back in one copy with the counters (1.3 M rows: 0.3 ms at
-// 55 GB/s).  Written by the kernel over the link instead they took as long at
-// 2,000 rows and 30 us more at 21,000.
+// Up to here the rows of a join whose bound is as good as its rows (kNN) come
+// back in one copy with the counters (1.3 M rows: 0.3 ms at 55 GB/s).  Written by
+// the kernel over the link instead they took as long at 2,000 rows and 30 us more
+// at 21,000.
 constexpr size_t kResultWhole = (size_t)16 << 20;
+// Where the bound is loose (every candidate of a within query) as many rows come
+// with the counters as the page-locked buffer already holds, and at most these
+// (7 us): the buffer grows by the rows that there are, as page-locking costs
+// 2 to 4 ms a MB (700 KB for the bound of a served batch: 1.5 to 3.1 ms).
+constexpr size_t kResultLoose = 32768;
 
 // the page-locked result buffer, of at least `need` bytes
 bool grow_hres(tdp_ctx* ctx, size_t need) {
@@ -571,7 +577,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
                 (size_t)t.task_cap * sizeof(LodTask), (size_t)t.eval_cap * sizeof(LodEval)};
             Carve c;
             for (int a = 0; a < kArrays; ++a) at[a] = c.take(need[a]);
-            if (ensure(ctx, ctx->scratch[kLodScratch], c.bytes) != TDP_OK) L.tasks = 0;
+            if (!lod_scratch(ctx, c.bytes)) L.tasks = 0;
         }
         if (!L.tasks) {  // no room for the queues: the refine of one warp per voxel pair
             cudaGetLastError();
@@ -635,18 +641,28 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     }
 
     // ---- 5. results ----
-    // The rows (at most `bound`) and the counters come back in one copy, before
-    // the number of rows is known; only where they may be many is it read first.
-    const size_t bound = knn && !mixed ? std::min<size_t>(P, (size_t)t1->n_obj * (size_t)prm->knn) : (size_t)P;
+    // With the counters come all rows (at most `bound`) or as many as there are
+    // places for; the rest once their number is known.
+    const bool tight = knn && !mixed;
+    const size_t bound = tight ? std::min<size_t>(P, (size_t)t1->n_obj * (size_t)prm->knn) : (size_t)P;
     const size_t head = (sizeof(JoinHeader) + 63) / 64 * 64;
-    const size_t at_q = head + (exact ? bound * 8 : 0), at_t = at_q + bound * 4, at_d = at_t + bound * 4, out_bytes = at_d + bound * 4;
-    const bool whole = out_bytes <= kResultWhole && grow_hres(ctx, out_bytes);
+    const size_t row_bytes = exact ? 20 : 12;
+    // n rows' arrays behind the header: FP64 distances, queries, results, distances
+    struct Places { size_t q, t, d, end; };
+    auto places = [&](size_t n) {
+        const size_t q = head + (exact ? n * 8 : 0);
+        return Places{q, q + n * 4, q + n * 8, q + n * 12};
+    };
+    const Places all = places(bound);
+    size_t first = 0;
+    if (tight && all.end <= kResultWhole && grow_hres(ctx, all.end)) first = bound;
+    else if (!tight && ctx->hres_cap > head) first = std::min({bound, (ctx->hres_cap - head) / row_bytes, kResultLoose});
     JoinHeader H{};
     uint8_t* rows_at = nullptr;
     if (P > 0) {
-        ENS(kOut, out_bytes);
+        ENS(kOut, all.end);
         rows_at = buf<uint8_t>(ctx, kOut);
-        JoinRows rows{(JoinHeader*)rows_at, (int*)(rows_at + at_q), (int*)(rows_at + at_t), (float*)(rows_at + at_d),
+        JoinRows rows{(JoinHeader*)rows_at, (int*)(rows_at + all.q), (int*)(rows_at + all.t), (float*)(rows_at + all.d),
                       exact ? (double*)(rows_at + head) : nullptr, (int64_t)bound, ctx->d_counter + 8, ctx->d_stats, fetch_ctr};
         if (on_device && (!any_knn || most <= kRankRows)) {
             size_t scan_bytes = 0;
@@ -668,10 +684,19 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         launches += 2;
     }
     CU(cudaEventRecord(ctx->ev[4], s));
-    if (P > 0) CU(cudaMemcpyAsync(whole ? ctx->hres : (void*)&H, rows_at, whole ? out_bytes : sizeof H, cudaMemcpyDeviceToHost, s));
+    // n rows and their header to a buffer with room for them
+    auto fetch_rows = [&](uint8_t* to, size_t n) {
+        if (n == bound) return cudaMemcpyAsync(to, rows_at, all.end, cudaMemcpyDeviceToHost, s);
+        const Places at = places(n);
+        cudaError_t e = cudaMemcpyAsync(to, rows_at, head + (exact ? n * 8 : 0), cudaMemcpyDeviceToHost, s);
+        for (size_t k = 0; k < 3 && e == cudaSuccess; ++k)
+            e = cudaMemcpyAsync(to + at.q + k * n * 4, rows_at + all.q + k * bound * 4, n * 4, cudaMemcpyDeviceToHost, s);
+        return e;
+    };
+    if (P > 0) CU(first ? fetch_rows((uint8_t*)ctx->hres, first) : cudaMemcpyAsync(&H, rows_at, sizeof H, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     ++syncs;
-    if (P > 0 && whole) std::memcpy(&H, ctx->hres, sizeof H);
+    if (P > 0 && first) std::memcpy(&H, ctx->hres, sizeof H);
     const unsigned nres = H.rows;
     if (nres > bound) return fail(ctx, TDP_ERR_CUDA, "more result rows than the query can have");
     const unsigned* tc = H.counters;
@@ -696,28 +721,22 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     // rows were sorted by (query, result id) on the device
     tdp_result* R = new tdp_result();
     if (nres) {
-        const uint8_t* h = (const uint8_t*)ctx->hres;
-        size_t hq = at_q, ht = at_t, hd = at_d;
+        size_t n = first;
+        std::vector<uint8_t> pageable;
+        uint8_t* h = (uint8_t*)ctx->hres;
         cudaError_t e = cudaSuccess;
-        if (!whole) {
+        if (nres > first) {
             // through a page-locked staging buffer: a fast copy, then one pass
             // into the result (no zero-fill of the vectors first)
-            std::vector<uint8_t> pageable;
-            const size_t need = head + (size_t)nres * (exact ? 20 : 12);
+            n = nres;
+            const size_t need = places(n).end;
             if (!grow_hres(ctx, need)) pageable.resize(need);
-            uint8_t* to = pageable.empty() ? (uint8_t*)ctx->hres : pageable.data();
-            hq = head + (exact ? (size_t)nres * 8 : 0);
-            ht = hq + (size_t)nres * 4;
-            hd = ht + (size_t)nres * 4;
-            if (exact) cudaMemcpyAsync(to + head, rows_at + head, (size_t)nres * 8, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(to + hq, rows_at + at_q, (size_t)nres * 4, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(to + ht, rows_at + at_t, (size_t)nres * 4, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(to + hd, rows_at + at_d, (size_t)nres * 4, cudaMemcpyDeviceToHost, s);
-            e = cudaStreamSynchronize(s);
-            R->take(to + head, to + hq, to + ht, to + hd, nres, exact);
-        } else {
-            R->take(h + head, h + hq, h + ht, h + hd, nres, exact);
+            h = pageable.empty() ? (uint8_t*)ctx->hres : pageable.data();
+            e = fetch_rows(h, n);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         }
+        const Places at = places(n);
+        if (e == cudaSuccess) R->take(h + head, h + at.q, h + at.t, h + at.d, nres, exact);
         if (e != cudaSuccess) { delete R; return fail(ctx, TDP_ERR_CUDA, cudaGetErrorString(e)); }
     }
     float f_ms = 0, tot_ms = 0;
