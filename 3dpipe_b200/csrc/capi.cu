@@ -294,6 +294,7 @@ int tdp_set_refine_config(tdp_ctx* ctx, int cfg) {
         return tdp::fail(ctx, TDP_ERR_ARG, "refine configuration " + std::to_string(cfg) + " out of range");
     ctx->tuned_cfg = cfg;
     for (int& c : ctx->lod_cfg) c = -1;
+    for (int& c : ctx->lod_alt) c = -1;
     return TDP_OK;
 }
 

@@ -39,6 +39,7 @@ struct LastStats {
     double fp32_max_rel_err = 0;     // max |FP32 minimum - FP64 distance| / max(distance, 1)
     double fetch_bytes = 0;          // RAW bytes fetched from attached tiles
     double refine_ms_lod[kNumLods] = {0, 0, 0, 0, 0};  // tuned refine time per LOD index
+    bool lod_tasks = false;          // the tuned LOD loop ran as task kernels
     long lod_graph = 0;              // tuned LOD loop: 0 direct launches, 1 graph replayed, 2 graph captured
     double exact_phase_ms[4] = {0, 0, 0, 0};  // exact stage: upper bounds, candidates, FP32 pass, FP64 pass
     unsigned long long exact_full_evals = 0;   // exact stage: triangle pairs fully evaluated in FP32
@@ -72,6 +73,10 @@ struct tdp_ctx {
     // per LOD index (20..100): the configuration the autotuner found fastest
     // at that LOD (-1: tuned_cfg); tdp_set_refine_config clears them
     int lod_cfg[tdp::kNumLods] = {-1, -1, -1, -1, -1};
+    // what takes configuration 0's place at a LOD where the task kernels have no
+    // room for their queues: the fastest of the others, once tdp_autotune has
+    // timed them against the task kernels (-1: configuration 0's own refine)
+    int lod_alt[tdp::kNumLods] = {-1, -1, -1, -1, -1};
     void* hres = nullptr;  // page-locked staging of join results (grow-only)
     size_t hres_cap = 0;
     // counts read back in mid-join: page-locked, or pageable where that is short

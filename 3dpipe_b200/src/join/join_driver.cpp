@@ -583,6 +583,8 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             cudaGetLastError();
             std::memset(&L.t, 0, sizeof L.t);
             L.caps_bytes = L.best_bytes = L.flags_bytes = L.zero_bytes = 0;
+            for (int k = 0; k < L.nl; ++k)
+                if (L.cfg[k] == 0 && ctx->lod_alt[L.li[k]] >= 0) L.cfg[k] = ctx->lod_alt[L.li[k]];
         } else {
             LodDev& t = L.t;
             const size_t nv1 = (size_t)std::max<long>(t1->n_vox, 1), nv2 = self ? 0 : (size_t)std::max<long>(t2->n_vox, 1);
@@ -624,6 +626,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
                         (L.recheck ? (knn ? 4 : 3) : 0);
         }
         st.refine_launches += L.nl;
+        st.lod_tasks = L.tasks != 0;
     }
 
     // ---- 4. exact LOD-100 distances of the reported pairs (optional) ----
@@ -777,21 +780,26 @@ int tdp_autotune(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp
     tdp_join_params p = *prm;
     p.form = TDP_FORM_TUNED;
     const int keep = ctx->tuned_cfg;
-    int keep_lod[kNumLods];
+    int keep_lod[kNumLods], keep_alt[kNumLods];
     std::memcpy(keep_lod, ctx->lod_cfg, sizeof(keep_lod));
-    for (int& c : ctx->lod_cfg) c = -1;
+    std::memcpy(keep_alt, ctx->lod_alt, sizeof(keep_alt));
+    for (int l = 0; l < kNumLods; ++l) ctx->lod_cfg[l] = ctx->lod_alt[l] = -1;
     int best_cfg = keep;
     double best_ms = 1e300;
     double lod_best[kNumLods];
     int lod_arg[kNumLods];
     for (int l = 0; l < kNumLods; ++l) { lod_best[l] = 1e300; lod_arg[l] = -1; }
     double ms0 = 0;  // configuration 0: all LODs as task kernels, or none
+    bool tasks = false;
+    double other_ms = 1e300;
+    int other = -1;  // the fastest of the others over the whole join
     auto run = [&] {
         tdp_result* r = nullptr;
         const int rc = tdp_join(ctx, t1, t2, &p, &r);
         if (rc != TDP_OK) {
             ctx->tuned_cfg = keep;
             std::memcpy(ctx->lod_cfg, keep_lod, sizeof(keep_lod));
+            std::memcpy(ctx->lod_alt, keep_alt, sizeof(keep_alt));
         } else {
             tdp_result_free(r);
         }
@@ -809,7 +817,13 @@ int tdp_autotune(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp
             best_ms = ms;
             best_cfg = cfg;
         }
-        if (cfg == 0) ms0 = ms;
+        if (cfg == 0) {
+            ms0 = ms;
+            tasks = ctx->stats.lod_tasks;
+        } else if (ms < other_ms) {
+            other_ms = ms;
+            other = cfg;
+        }
         // the fastest of the other configurations at each LOD the join refined
         for (int l = 0; l < kNumLods && cfg > 0; ++l) {
             const double m = ctx->stats.refine_ms_lod[l];
@@ -835,7 +849,10 @@ int tdp_autotune(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp
         if (loop[0] <= loop[1]) best_cfg = 0;
     }
     if (best_cfg == 0)
-        for (int& l : lod_arg) l = 0;
+        for (int l = 0; l < kNumLods; ++l) {
+            if (tasks) ctx->lod_alt[l] = lod_arg[l] >= 0 ? lod_arg[l] : other;
+            lod_arg[l] = 0;
+        }
     ctx->tuned_cfg = best_cfg;
     for (int l = 0; l < kNumLods; ++l) ctx->lod_cfg[l] = lod_arg[l];
     if (best) *best = best_cfg;

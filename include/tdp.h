@@ -131,7 +131,10 @@ int tdp_get_refine_config(const tdp_ctx *ctx, int *cfg);
 /* The configuration the tuned form uses at one LOD (20, 40, 60, 80, 100):
  * tdp_autotune keeps, besides the fastest configuration over the whole join
  * (its *best), the fastest one at each LOD (configuration 0 at all of them or
- * at none), and the LOD loop launches each LOD's own; tdp_set_refine_config sets one configuration for every LOD. */
+ * at none), and the LOD loop launches each LOD's own; tdp_set_refine_config
+ * sets one configuration for every LOD.  A join that has no room for
+ * configuration 0's queues runs with the fastest of the others that the
+ * autotuner timed (without it, with one warp per voxel pair). */
 int tdp_get_refine_config_lod(const tdp_ctx *ctx, int lod, int *cfg);
 
 /* ---- CUDA graph of the LOD loop --------------------------------------
