@@ -392,7 +392,7 @@ void executor_loop(tdp_server* S) {
     std::vector<int> obj_knn;
     std::vector<float> obj_within;
     std::unique_lock<std::mutex> lk(S->mu);
-    Request* waited = nullptr;  // the lone request that has had its wait
+    uint64_t waited = 0;  // id of the lone request that has had its wait (a finished request's address is used again)
     for (;;) {
         Arena* a = nullptr;
         S->cv.wait(lk, [&] {
@@ -403,8 +403,8 @@ void executor_loop(tdp_server* S) {
             return S->stop;
         });
         if (!a) return;  // stopping with nothing admitted left to run
-        if (a->state == ArenaState::kFilling && a->reqs.size() == 1 && a->reqs[0] != waited) {
-            waited = a->reqs[0];
+        if (a->state == ArenaState::kFilling && a->reqs.size() == 1 && a->reqs[0]->id != waited) {
+            waited = a->reqs[0]->id;
             S->cv.wait_for(lk, kCompany, [&] {
                 const Request* next = S->held ? S->held : S->pending.empty() ? nullptr : S->pending.front();
                 return S->stop || a->state != ArenaState::kFilling || a->reqs.size() > 1 ||
