@@ -500,7 +500,7 @@ int device_candidates(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, bool
                                                                (int)qb0, (int)qe0, d_over + 1, nullptr, nullptr);
         CU(cudaGetLastError());
         size_t tb = 0;
-        CU(scan_to_host_bytes((int)n1, tb));
+        CU(scan_to_host_bytes((int)n1, ctx->hwords != ctx->pageable_words, tb));
         if ((rc = ensure(ctx, tmp, tb + 16))) return rc;
         CU(scan_to_host(cnt, qoff, (int)n1, tmp.p, tb, (const unsigned long long*)d_over, ctx->hwords,
                         ctx->hwords != ctx->pageable_words, s));

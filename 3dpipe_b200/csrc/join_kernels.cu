@@ -882,9 +882,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_small(const int64_t* __re
 }
 }  // namespace
 
-cudaError_t scan_to_host_bytes(int n, size_t& bytes) {
+cudaError_t scan_to_host_bytes(int n, bool host_locked, size_t& bytes) {
     bytes = 0;
-    return n <= kScanSmall ? cudaSuccess : scan_counts(nullptr, nullptr, n, nullptr, bytes, nullptr);
+    return n <= kScanSmall && host_locked ? cudaSuccess : scan_counts(nullptr, nullptr, n, nullptr, bytes, nullptr);
 }
 cudaError_t scan_to_host(int64_t* cnt, int64_t* out, int n, void* temp, size_t temp_bytes, const unsigned long long* extra,
                          unsigned long long* host, bool host_locked, cudaStream_t s) {

@@ -128,7 +128,7 @@ cudaError_t scan_counts(const int64_t* cnt, int64_t* out, int n, void* temp, siz
 // once the stream is done: up to 16,384 counts by one block that writes
 // page-locked host words itself (one launch instead of two, a memset and two
 // copies: 8 us less), else by scan_counts with scan_to_host_bytes of workspace.
-cudaError_t scan_to_host_bytes(int n, size_t& bytes);
+cudaError_t scan_to_host_bytes(int n, bool host_locked, size_t& bytes);
 cudaError_t scan_to_host(int64_t* cnt, int64_t* out, int n, void* temp, size_t temp_bytes, const unsigned long long* extra,
                          unsigned long long* host, bool host_locked, cudaStream_t s);
 

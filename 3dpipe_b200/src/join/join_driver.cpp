@@ -435,7 +435,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     int64_t* cnt = buf<int64_t>(ctx, kCnt);
     CU(launch_count_vps(d, !knn, within_dist, tuned, cnt, s)); ++launches;
     size_t tmp_bytes = 0;
-    CU(scan_to_host_bytes((int)P, tmp_bytes));
+    CU(scan_to_host_bytes((int)P, ctx->hwords != ctx->pageable_words, tmp_bytes));
     ENS(kScanTmp, tmp_bytes + 16);
     CU(scan_to_host(cnt, d.pvp, (int)P, ctx->scratch[kScanTmp].p, tmp_bytes, nullptr, ctx->hwords,
                     ctx->hwords != ctx->pageable_words, s)); ++launches;
