@@ -57,6 +57,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "bounds_kernels.cuh"
@@ -248,7 +249,8 @@ __device__ __forceinline__ uint32_t block_excl_sum(uint32_t x, uint32_t* red, ui
 
 // ------------------------------------------------------------------ decimation
 // The live facets of vertex x, 32 at a time, one a lane: fn(facet, valid) is
-// called by the whole warp.  x's chain of merged vertices is followed 32 at a
+// called by the whole warp (where it returns a bool, until that is false).  The
+// chain of vertices merged into x is followed 32 at a
 // time, their lists taken as one row.  Returns the rows' number; `last` is the
 // lane's facet in the last one (UINT_MAX: none).
 template <typename VI, typename Fn>
@@ -287,7 +289,8 @@ __device__ __forceinline__ int each_facet(uint32_t x, const VI* next, const uint
             const bool on = e0 + lane < total && (fl[f] & 1);
             last = on ? f : UINT_MAX;
             ++rows;
-            fn(f, on);
+            if constexpr (std::is_void<decltype(fn(f, on))>::value) fn(f, on);
+            else if (!fn(f, on)) return rows;
         }
     }
     return rows;
@@ -480,18 +483,22 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
                 } else if (wid < 4) {  // neighbours of the two third vertices
                     const uint32_t x = s_third[wid - 2];
                     uint32_t* mask = wid == 2 ? M1 : M2;
-                    uint32_t cnt = 0, unused;
+                    uint32_t cnt = 0, all = 0, unused;
                     auto add = [&](uint32_t a) {
                         if (a != x && !(atomicOr(mask + (a >> 5), 1u << (a & 31)) & (1u << (a & 31)))) ++cnt;
                     };
+                    // (more than three is all that is asked: the apex of a fan of 10,000
+                    // facets, the third vertex of every edge around it, is not gone round)
                     each_facet<VI>(x, next, start, csr, fl, lane, unused, [&](uint32_t f, bool on) {
-                        if (!on) return;
-                        add(fv[3 * f]);
-                        add(fv[3 * f + 1]);
-                        add(fv[3 * f + 2]);
+                        if (on) {
+                            add(fv[3 * f]);
+                            add(fv[3 * f + 1]);
+                            add(fv[3 * f + 2]);
+                        }
+                        all = __reduce_add_sync(0xffffffffu, cnt);
+                        return all <= 3;
                     });
-                    cnt = __reduce_add_sync(0xffffffffu, cnt);
-                    if (lane == 0) s_cnt[wid - 2] = cnt;
+                    if (lane == 0) s_cnt[wid - 2] = all;
                 }
                 if (wid == (NW > 4 ? 4 : 3)) {  // neighbours that u and v share
                     uint32_t cnt = 0;
