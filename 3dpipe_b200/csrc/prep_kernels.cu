@@ -168,6 +168,12 @@ __device__ __forceinline__ Key facet_key(double3 p, double3 q, double3 r, uint32
 
 constexpr int kGroup = 32;     // facets whose smallest key is kept
 constexpr int kTouched = 128;  // touched groups listed a round (more: all are redone)
+// A chain is rewritten without its dead facets once, past its first rows of 32, it
+// holds more than twice its live ones.  A tube whose short edges are all at one
+// end merges thousands of vertices into one: 1,720 ms for 18,000 facets where every
+// round went through all that its chain had ever held, 42 with this (123 with
+// scans over all facets); a flat sheet of 20,000: 232, 78 (286).
+constexpr int kFewRows = 2;
 
 // bytes of an object's own storage: facets, flags, 4 masks, merge chains, group
 // keys
@@ -178,13 +184,12 @@ __host__ __device__ inline size_t dec_bytes(int64_t n, int64_t m, size_t vi) {
 }
 
 // Per batch in global memory: every facet's smallest key, every vertex's facets
-// as the mesh has them (csr[start[v] .. start[v + 1]), start with one entry more
-// per object), fill cursors.
+// (vertex v's are csr[lists[v].x .. lists[v].y), with room up to lists[v + 1].x:
+// lists has one entry more per object).
 struct DecLists {
     Key* keys;
     uint32_t* csr;
-    uint32_t* start;
-    uint32_t* cur;
+    uint2* lists;
 };
 
 // ------------------------------------------------------------------ validation
@@ -250,11 +255,11 @@ __device__ __forceinline__ uint32_t block_excl_sum(uint32_t x, uint32_t* red, ui
 // ------------------------------------------------------------------ decimation
 // The live facets of vertex x, 32 at a time, one a lane: fn(facet, valid) is
 // called by the whole warp (where it returns a bool, until that is false).  The
-// chain of vertices merged into x is followed 32 at a
-// time, their lists taken as one row.  Returns the rows' number; `last` is the
-// lane's facet in the last one (UINT_MAX: none).
+// chain of vertices merged into x is followed 32 at a time, their lists taken as
+// one row.  Returns the rows' number; `last` is the lane's facet in the last one
+// (UINT_MAX: none).
 template <typename VI, typename Fn>
-__device__ __forceinline__ int each_facet(uint32_t x, const VI* next, const uint32_t* start, const uint32_t* csr,
+__device__ __forceinline__ int each_facet(uint32_t x, const VI* next, const uint2* lists, const uint32_t* csr,
                                           const uint8_t* fl, int lane, uint32_t& last, Fn fn) {
     constexpr uint32_t kEnd = (uint32_t)(VI)~0u;
     uint32_t s = x;
@@ -266,7 +271,8 @@ __device__ __forceinline__ int each_facet(uint32_t x, const VI* next, const uint
             if (lane == k) mine = s;
             s = next[s];
         }
-        const uint32_t b = lane < k ? start[mine] : 0u, c = lane < k ? start[mine + 1] - b : 0u;
+        const uint2 at_to = lane < k ? lists[mine] : make_uint2(0u, 0u);
+        const uint32_t b = at_to.x, c = at_to.y - b;
         uint32_t end = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -296,6 +302,38 @@ __device__ __forceinline__ int each_facet(uint32_t x, const VI* next, const uint
     return rows;
 }
 
+// The live facets of x to the front of its chain, in the same order, and what is
+// left of the chain dropped; a vertex's list has the room it had in the mesh.
+// (Up to any place in the chain no more are written than were read before it.)
+template <typename VI>
+__device__ __noinline__ void compact_facets(uint32_t x, VI* next, VI* tail, uint2* lists, uint32_t* csr, const uint8_t* fl,
+                                            int lane) {
+    uint32_t w = x, at = lists[x].x, unused;  // where the next one goes, the same on every lane
+    each_facet<VI>(x, next, lists, csr, fl, lane, unused, [&](uint32_t f, bool on) {
+        const unsigned live = __ballot_sync(0xffffffffu, on);
+        const uint32_t rank = __popc(live & ((1u << lane) - 1u)), n = __popc(live);
+        for (uint32_t done = 0; done < n;) {
+            const uint32_t room = lists[w + 1].x - at, take = min(room, n - done);
+            if (on && rank >= done && rank < done + take) csr[at + (rank - done)] = f;
+            at += take;
+            done += take;
+            if (done < n) {  // that list is full
+                __syncwarp();
+                if (lane == 0) lists[w].y = at;
+                w = next[w];
+                at = lists[w].x;
+            }
+        }
+        __syncwarp();
+    });
+    if (lane == 0) {
+        lists[w].y = at;
+        next[w] = (VI)~0u;
+        tail[x] = (VI)w;
+    }
+    __syncwarp();
+}
+
 template <typename VI, int T>
 __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict__ objs, int n_objs, DecLists D,
                                                 uint8_t* gstore, const int64_t* __restrict__ gstore_off,
@@ -305,7 +343,7 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
     extern __shared__ __align__(16) uint8_t dsm[];
     __shared__ Key s_key[NW];
     __shared__ uint32_t s_red[NW], s_third[2], s_cnt[3], s_list[kTouched];
-    __shared__ int s_nsh, s_turn[2], s_alive, s_ng;
+    __shared__ int s_nsh, s_turn[2], s_alive, s_ng, s_long;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int i = blockIdx.x; i < n_objs; i += gridDim.x) {
         const int o = objs[i];
@@ -323,8 +361,7 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
         Key* gk = reinterpret_cast<Key*>(reinterpret_cast<uint8_t*>(tail) + round16((size_t)n * sizeof(VI)));
         Key* keys = D.keys + f0;
         uint32_t* csr = D.csr + 3 * f0;
-        uint32_t* start = D.start + v0 + o;
-        uint32_t* cur = D.cur + v0;
+        uint2* lists = D.lists + v0 + o;
         for (uint32_t f = tid; f < m; f += T) {
             uint32_t t[3];
             for (int k = 0; k < 3; ++k) {
@@ -338,30 +375,29 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
         for (uint32_t v = tid; v < n; v += T) {
             next[v] = (VI)~0u;
             tail[v] = (VI)v;
-            cur[v] = 0;
+            lists[v].y = 0;
         }
         if (tid == 0) {
             s_alive = (int)m;
-            s_nsh = s_turn[0] = s_turn[1] = s_ng = 0;
+            s_nsh = s_turn[0] = s_turn[1] = s_ng = s_long = 0;
         }
         __syncthreads();
         // every vertex's facets
-        for (uint32_t c = tid; c < 3 * m; c += T) atomicAdd(cur + fv[c], 1u);
+        for (uint32_t c = tid; c < 3 * m; c += T) atomicAdd(&lists[fv[c]].y, 1u);
         __syncthreads();
         uint32_t run = 0;
         for (uint32_t c0 = 0; c0 < n; c0 += T) {
-            const uint32_t v = c0 + tid, x = v < n ? cur[v] : 0u;
+            const uint32_t v = c0 + tid, x = v < n ? lists[v].y : 0u;
             uint32_t total;
             const uint32_t at = run + block_excl_sum<T>(x, s_red, total);
             if (v < n) {
-                start[v] = at;
-                cur[v] = at;
+                lists[v] = make_uint2(at, at);
             }
             run += total;
         }
-        if (tid == 0) start[n] = run;
+        if (tid == 0) lists[n] = make_uint2(run, run);
         __syncthreads();
-        for (uint32_t c = tid; c < 3 * m; c += T) csr[atomicAdd(cur + fv[c], 1u)] = c / 3;
+        for (uint32_t c = tid; c < 3 * m; c += T) csr[atomicAdd(&lists[fv[c]].y, 1u)] = c / 3;
         auto redo_group = [&](uint32_t g) {
             const uint32_t f = g * kGroup + lane;
             const Key k = warp_least(f < m ? keys[f] : no_key());
@@ -428,7 +464,7 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
             int rows = 0, nsh = 0;
             if (wid < 2) {
                 uint32_t* mask = wid ? Mv : Mu;
-                rows = each_facet<VI>(own, next, start, csr, fl, lane, row, [&](uint32_t f, bool on) {
+                rows = each_facet<VI>(own, next, lists, csr, fl, lane, row, [&](uint32_t f, bool on) {
                     uint32_t a = 0, b = 0, c = 0;
                     if (on) {
                         a = fv[3 * f];
@@ -444,6 +480,14 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
                     nsh += __popc(sh);
                 });
                 if (tid == 0) s_nsh = nsh;
+                if (rows > kFewRows) {
+                    int live = 0;
+                    uint32_t unused;
+                    each_facet<VI>(own, next, lists, csr, fl, lane, unused, [&](uint32_t, bool on) {
+                        live += __popc(__ballot_sync(0xffffffffu, on));
+                    });
+                    if (lane == 0 && 32 * (rows - kFewRows) > 2 * live) atomicOr(&s_long, 1 << wid);
+                }
             }
             __syncthreads();
             const bool cand = s_nsh == 2 && s_third[0] != s_third[1];
@@ -462,7 +506,7 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
                 uint32_t unused;
                 if (rows == 1) fn(held, row != UINT_MAX);
                 else
-                    each_facet<VI>(own, next, start, csr, fl, lane, unused, [&](uint32_t f, bool on) {
+                    each_facet<VI>(own, next, lists, csr, fl, lane, unused, [&](uint32_t f, bool on) {
                         Facet t{};
                         if (on) t = load(f);
                         fn(t, on);
@@ -489,7 +533,7 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
                     };
                     // (more than three is all that is asked: the apex of a fan of 10,000
                     // facets, the third vertex of every edge around it, is not gone round)
-                    each_facet<VI>(x, next, start, csr, fl, lane, unused, [&](uint32_t f, bool on) {
+                    each_facet<VI>(x, next, lists, csr, fl, lane, unused, [&](uint32_t f, bool on) {
                         if (on) {
                             add(fv[3 * f]);
                             add(fv[3 * f + 1]);
@@ -558,7 +602,7 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
             }
             __syncthreads();
             // the touched groups; k's chain goes on with r's
-            const int ng = s_ng;
+            const int ng = s_ng, is_long = s_long;
             if (ng <= kTouched)
                 for (int q = wid; q < ng; q += NW) redo_group(s_list[q]);
             else
@@ -567,8 +611,12 @@ __global__ void __launch_bounds__(T) k_decimate(Meshes M, const int* __restrict_
                 next[tail[k]] = (VI)r;
                 tail[k] = tail[r];
             }
+            if (is_long && wid < 2) {  // (both chains are one where the edge went)
+                __syncwarp();
+                if (go ? wid == 0 : is_long >> wid & 1) compact_facets<VI>(go ? k : own, next, tail, lists, csr, fl, lane);
+            }
             __syncthreads();
-            if (tid == 0) s_turn[0] = s_turn[1] = s_ng = 0;  // read again after the next barrier
+            if (tid == 0) s_turn[0] = s_turn[1] = s_ng = s_long = 0;  // read again after the next barrier
         }
         __syncthreads();  // the next object reuses the storage
     }
@@ -1099,8 +1147,7 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
         DecLists dls{};
         CU(dm.get(&dls.keys, (size_t)Ftot));
         CU(dm.get(&dls.csr, 3 * (size_t)Ftot));
-        CU(dm.get(&dls.start, (size_t)(Vtot + nb)));
-        CU(dm.get(&dls.cur, (size_t)Vtot));
+        CU(dm.get(&dls.lists, (size_t)(Vtot + nb)));
         int* dl;
         CU(dm.get(&dl, small.size() + large.size() + huge.size()));
         std::vector<int> all(small);
