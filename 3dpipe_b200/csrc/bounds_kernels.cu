@@ -315,6 +315,10 @@ __device__ inline void search(Search<K>& S, int n, const float4* T, const uint32
     // the scan of a voxel is in the kernel once.)
     uint32_t u = first, base = vb;
     unsigned mask = 0;
+    // The lane's own query is near enough to voxel u.  (Where spheres say little, as
+    // those of a double cone's 20,000 needles, a voxel scanned for all 32 queries
+    // when one was near took 279 M distances, 37.8 ms; this way 141 M, 20.6 ms.)
+    bool near = on;
     float ulx = 0.f, uly = 0.f, ulz = 0.f, uhx = 0.f, uhy = 0.f, uhz = 0.f;  // voxel base - 32 + lane
     for (;;) {
         for (uint32_t t0 = VT[u]; t0 < VT[u + 1]; t0 += kStage) {
@@ -324,7 +328,7 @@ __device__ inline void search(Search<K>& S, int n, const float4* T, const uint32
                 const float4 c = S.sph[i];
                 const float reach = (bf + c.w) * 1.000001f;
                 const float gx = Q.gx - c.x, gy = Q.gy - c.y, gz = Q.gz - c.z;
-                bool keep = on && !(gx * gx + gy * gy + gz * gz > reach * reach);
+                bool keep = near && !(gx * gx + gy * gy + gz * gz > reach * reach);
                 unsigned mk = __ballot_sync(0xffffffffu, keep);
                 if (!mk) continue;
                 if (K > 1) {
@@ -374,7 +378,7 @@ __device__ inline void search(Search<K>& S, int n, const float4* T, const uint32
             const float ax = __shfl_sync(0xffffffffu, ulx, k), ay = __shfl_sync(0xffffffffu, uly, k), az = __shfl_sync(0xffffffffu, ulz, k);
             const float ex = __shfl_sync(0xffffffffu, uhx, k), ey = __shfl_sync(0xffffffffu, uhy, k), ez = __shfl_sync(0xffffffffu, uhz, k);
             const float mg = 4e-6f * (fmaxf(fabsf(ax), fabsf(ex)) + fmaxf(fabsf(ay), fabsf(ey)) + fmaxf(fabsf(az), fabsf(ez)) + scale) + 1e-6f;
-            bool near = on;
+            near = on;
 #pragma unroll
             for (int c = 0; c < K; ++c) {
                 const float x = fmaxf(fmaxf(ax - Q.x[c], Q.x[c] - ex), 0.f), y = fmaxf(fmaxf(ay - Q.y[c], Q.y[c] - ey), 0.f),
