@@ -1009,6 +1009,9 @@ struct DevMem {  // allocations of one batch, back to the context's block cache 
     void release() {
         if (ps.empty()) return;
         cudaStreamSynchronize(ctx->stream);  // nothing queued may still use a block
+        hand_on();
+    }
+    void hand_on() {  // to what is queued on the context's stream after this
         for (void* p : ps) block_release(ctx, p);
         ps.clear();
     }
@@ -1144,12 +1147,13 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
             else if (n <= 65535 && b16 <= kSmemLarge) { large.push_back((int)i); s_large = std::max(s_large, b16); }
             else { huge.push_back((int)i); hoff.push_back(hoff.back() + (int64_t)dec_bytes(n, m, 4)); }
         }
+        DevMem dec{ctx, {}};  // what only the decimation needs
         DecLists dls{};
-        CU(dm.get(&dls.keys, (size_t)Ftot));
-        CU(dm.get(&dls.csr, 3 * (size_t)Ftot));
-        CU(dm.get(&dls.lists, (size_t)(Vtot + nb)));
+        CU(dec.get(&dls.keys, (size_t)Ftot));
+        CU(dec.get(&dls.csr, 3 * (size_t)Ftot));
+        CU(dec.get(&dls.lists, (size_t)(Vtot + nb)));
         int* dl;
-        CU(dm.get(&dl, small.size() + large.size() + huge.size()));
+        CU(dec.get(&dl, small.size() + large.size() + huge.size()));
         std::vector<int> all(small);
         all.insert(all.end(), large.begin(), large.end());
         all.insert(all.end(), huge.begin(), huge.end());
@@ -1171,8 +1175,8 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
         if (!huge.empty()) {
             uint8_t* gst;
             int64_t* dho;
-            CU(dm.get(&gst, (size_t)hoff.back()));
-            CU(dm.get(&dho, hoff.size()));
+            CU(dec.get(&gst, (size_t)hoff.back()));
+            CU(dec.get(&dho, hoff.size()));
             CU(cudaMemcpyAsync(dho, hoff.data(), 8 * hoff.size(), cudaMemcpyHostToDevice, s));
             k_decimate<uint32_t, 1024><<<(int)huge.size(), 1024, 0, s>>>(Mh, dl + small.size() + large.size(),
                                                                       (int)huge.size(), dls, gst, dho, lodF, Ftot,
@@ -1180,6 +1184,7 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
             CU(cudaGetLastError());
         }
         CU(cudaEventRecord(ev[1], s));
+        if (ctx->budget) dec.hand_on();  // under a memory cap its room is the next steps'
         // 2-3. voxels
         VoxScratch S{};
         CU(dm.get(&S.dmin, (size_t)Vtot));
