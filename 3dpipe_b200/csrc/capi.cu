@@ -21,21 +21,25 @@ void cache_trim(tdp_ctx* ctx) {
     ctx->small_cached = 0;
 }
 
-bool lod_scratch_drop(tdp_ctx* ctx) {
+bool optional_scratch_drop(tdp_ctx* ctx) {
     if (ctx->lod_busy) return false;
-    Buf& b = ctx->scratch[kLodScratch];
-    if (!b.p) return false;
-    cudaStreamSynchronize(ctx->stream);
-    dfree(ctx, b.p);
-    b = Buf{};
-    return true;
+    bool any = false;
+    for (int k : {kLodScratch, kPrefetchList, kRefineParts}) {
+        Buf& b = ctx->scratch[k];
+        if (!b.p) continue;
+        if (!any) cudaStreamSynchronize(ctx->stream);
+        any = true;
+        dfree(ctx, b.p);
+        b = Buf{};
+    }
+    return any;
 }
 
 cudaError_t dmalloc(tdp_ctx* ctx, void** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
     if (ctx->budget && ctx->in_use + bytes > ctx->budget &&
-        (!lod_scratch_drop(ctx) || ctx->in_use + bytes > ctx->budget))
+        (!optional_scratch_drop(ctx) || ctx->in_use + bytes > ctx->budget))
         return cudaErrorMemoryAllocation;
     if (ctx->budget && ctx->in_use + ctx->cached_bytes + bytes > ctx->budget) cache_trim(ctx);
     cudaError_t e = cudaMalloc(p, bytes);
@@ -44,7 +48,7 @@ cudaError_t dmalloc(tdp_ctx* ctx, void** p, size_t bytes) {
         cache_trim(ctx);
         e = cudaMalloc(p, bytes);
     }
-    if (e != cudaSuccess && lod_scratch_drop(ctx)) {
+    if (e != cudaSuccess && optional_scratch_drop(ctx)) {
         cudaGetLastError();
         e = cudaMalloc(p, bytes);
     }
@@ -387,16 +391,18 @@ int tdp_refine_batch(tdp_ctx* ctx, const float* data, const float* hausdorff, si
     }
     if ((rc = ensure(ctx, ctx->scratch[kSlotItems], pair_num * sizeof(RefineItem)))) return rc;
     if ((rc = ensure(ctx, ctx->scratch[kSlotOut], pair_num * sizeof(float4)))) return rc;
-    if (!parts.empty() && (ensure(ctx, ctx->scratch[kSlotParts], parts.size() * sizeof(RefineItem)) != TDP_OK ||
-                           ensure(ctx, ctx->scratch[kSlotPartOut], n_cut * sizeof(float4)) != TDP_OK)) {
+    Carve part_at;  // the parts with their pairs' first ones, and the parts' results
+    const size_t at_parts = part_at.take(parts.size() * sizeof(RefineItem)), at_part_out = part_at.take(n_cut * sizeof(float4));
+    if (!parts.empty() && ensure(ctx, ctx->scratch[kRefineParts], part_at.bytes) != TDP_OK) {
         cudaGetLastError();
         parts.clear();  // no room for them
     }
+    char* part_mem = (char*)ctx->scratch[kRefineParts].p;
     const size_t n_parts = parts.empty() ? pair_num : n_cut;
     float* d_data = (float*)ctx->scratch[kSlotRawData].p;
     float* d_hd = hausdorff ? (float*)ctx->scratch[kSlotRawHd].p : nullptr;
     float4* d_tri = (float4*)ctx->scratch[kSlotTris].p;
-    RefineItem* d_items = (RefineItem*)ctx->scratch[parts.empty() ? kSlotItems : kSlotParts].p;
+    RefineItem* d_items = parts.empty() ? (RefineItem*)ctx->scratch[kSlotItems].p : (RefineItem*)(part_mem + at_parts);
     float4* d_out = (float4*)ctx->scratch[kSlotOut].p;
     cudaStream_t s = ctx->stream;
     TDP_CUDA_TRY(cudaMemcpyAsync(d_data, data, element_num * 9 * sizeof(float), cudaMemcpyHostToDevice, s));
@@ -409,7 +415,7 @@ int tdp_refine_batch(tdp_ctx* ctx, const float* data, const float* hausdorff, si
     if (form == TDP_FORM_PLAIN) {
         TDP_CUDA_TRY(launch_refine_plain(d_tri, d_tri, d_items, (int)pair_num, d_out, s));
     } else {
-        float4* po = parts.empty() ? d_out : (float4*)ctx->scratch[kSlotPartOut].p;
+        float4* po = parts.empty() ? d_out : (float4*)(part_mem + at_part_out);
         TDP_CUDA_TRY(launch_refine_tuned(d_tri, d_tri, d_items, (int)n_parts, po, ctx->d_counter, ctx->d_stats,
                                          ctx->num_sms, ctx->tuned_cfg, s));
         if (!parts.empty())

@@ -64,7 +64,7 @@ struct tdp_ctx {
     cudaEvent_t pf_ev[16] = {};   // fork / join of the prefetches (no timing)
     std::string last_error;
     std::unordered_map<void*, size_t> allocs;
-    tdp::Buf scratch[120];  // slots: refine-batch 0-6, tile upload 12-13, join 20-48, candidates 50-59 and 88-90, result sort 60-63, exact distances 64-81 and 84-86, per-object queries 82-83, last-LOD presets 91, GPU attach pass 96-100, LOD task form 101
+    tdp::Buf scratch[120];  // slots: refine-batch 0-4, tile upload 12-13, join 20-48, candidates 50-59 and 88-90, result sort 60-63, exact distances 64-81 and 84-86, per-object queries 82-83, last-LOD presets 91, GPU attach pass 96-100, LOD task form 101, optional 102-103
     unsigned* d_counter = nullptr;            // work counters (device)
     bool lod_busy = false;                    // the LOD task scratch is in use (LodScratchUse)
     unsigned long long* d_stats = nullptr;    // device-side statistics
@@ -133,6 +133,9 @@ void cache_trim(tdp_ctx* ctx);
 // allocation that would fail otherwise takes them back while no join is between
 // their set-up and its last use of them.
 constexpr int kLodScratch = 101;
+// Other scratch that a call does without where there is no room: voxels to
+// prefetch, the parts of a refine batch.  Given back like the queues.
+constexpr int kPrefetchList = 102, kRefineParts = 103;
 
 // Offsets of a block's arrays, each on a 256-byte boundary as an allocation is.
 struct Carve {
@@ -146,7 +149,8 @@ struct Carve {
 // the block with at least `bytes`, grown to twice its size where there is room
 // (growing waits for the device twice); false without room
 bool lod_scratch(tdp_ctx* ctx, size_t bytes);
-bool lod_scratch_drop(tdp_ctx* ctx);
+// gives back what no call is using of it and of the other optional scratch
+bool optional_scratch_drop(tdp_ctx* ctx);
 struct LodScratchUse {
     tdp_ctx* ctx;
     explicit LodScratchUse(tdp_ctx* c) : ctx(c) { c->lod_busy = true; }
@@ -154,7 +158,7 @@ struct LodScratchUse {
 };
 
 enum ScratchSlot {
-    kSlotRawData = 0, kSlotRawHd, kSlotTris, kSlotItems, kSlotOut, kSlotParts, kSlotPartOut,
+    kSlotRawData = 0, kSlotRawHd, kSlotTris, kSlotItems, kSlotOut,
 };
 
 }  // namespace tdp

@@ -49,7 +49,6 @@ enum Slot {
     kPexOut = 76,                     // exact distances (64-75 and 78-81 are the exact stage's own)
     kQk = 82, kQtau,                  // per query object queries
     kPreset = 91,                     // the last LOD's item presets (within queries)
-    kPfList = kLodScratch + 1,        // voxels to prefetch
 };
 
 // Up to here the rows of a join whose bound is as good as its rows (kNN) come
@@ -393,6 +392,20 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     ENS(kPq, Pz * 4); ENS(kPt, Pz * 4); ENS(kQoff, (t1->n_obj + 1) * 8);
     ENS(kPmn, Pz * 4); ENS(kPmx, Pz * 4); ENS(kPerr, Pz * 4); ENS(kPstat, Pz);
     ENS(kPvp, (Pz + 1) * 8); ENS(kQconf, (t1->n_obj + 1) * 4); ENS(kCnt, (Pz + 1) * 8); ENS(kRankSt, Pz * 4);
+    // the rows (at most `bound`): their room is taken before the large scratch
+    const bool exact = prm->exact_distances != 0;
+    const bool tight = knn && !mixed;
+    const size_t bound = tight ? std::min<size_t>(P, (size_t)t1->n_obj * (size_t)prm->knn) : (size_t)P;
+    const size_t head = (sizeof(JoinHeader) + 63) / 64 * 64;
+    const size_t row_bytes = exact ? 20 : 12;
+    // n rows' arrays behind the header: FP64 distances, queries, results, distances
+    struct Places { size_t q, t, d, end; };
+    auto places = [&](size_t n) {
+        const size_t q = head + (exact ? n * 8 : 0);
+        return Places{q, q + n * 4, q + n * 8, q + n * 12};
+    };
+    const Places all = places(bound);
+    if (P > 0) ENS(kOut, all.end);
 
     JoinDev d;
     std::memset(&d, 0, sizeof d);  // padding too: the LOD loop's graph key holds these bytes
@@ -543,10 +556,12 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         L.preset = presets ? buf<float>(ctx, kPreset) : nullptr;
         L.side = ctx->side;
         if ((lz1.on || lz2.on) && L.side) {  // without room for the list: no prefetch
-            if (ensure(ctx, ctx->scratch[kPfList], ((size_t)t1->n_vox + (size_t)t2->n_vox + 1) * 4) == TDP_OK)
-                L.pf_list = buf<int>(ctx, kPfList);
-            else
+            if (ensure(ctx, ctx->scratch[kPrefetchList], ((size_t)t1->n_vox + (size_t)t2->n_vox + 1) * 4) == TDP_OK) {
+                L.pf_list = buf<int>(ctx, kPrefetchList);
+            } else {
+                cudaGetLastError();
                 L.side = nullptr;
+            }
         }
         for (int k = 0; k < 16; ++k) L.pf[k] = ctx->pf_ev[k];
         L.tasks = 1;
@@ -630,7 +645,6 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     }
 
     // ---- 4. exact LOD-100 distances of the reported pairs (optional) ----
-    const bool exact = prm->exact_distances != 0;
     double* pex = nullptr;
     ExactInfo xi;
     if (exact) {
@@ -646,24 +660,12 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
     // ---- 5. results ----
     // With the counters come all rows (at most `bound`) or as many as there are
     // places for; the rest once their number is known.
-    const bool tight = knn && !mixed;
-    const size_t bound = tight ? std::min<size_t>(P, (size_t)t1->n_obj * (size_t)prm->knn) : (size_t)P;
-    const size_t head = (sizeof(JoinHeader) + 63) / 64 * 64;
-    const size_t row_bytes = exact ? 20 : 12;
-    // n rows' arrays behind the header: FP64 distances, queries, results, distances
-    struct Places { size_t q, t, d, end; };
-    auto places = [&](size_t n) {
-        const size_t q = head + (exact ? n * 8 : 0);
-        return Places{q, q + n * 4, q + n * 8, q + n * 12};
-    };
-    const Places all = places(bound);
     size_t first = 0;
     if (tight && all.end <= kResultWhole && grow_hres(ctx, all.end)) first = bound;
     else if (!tight && ctx->hres_cap > head) first = std::min({bound, (ctx->hres_cap - head) / row_bytes, kResultLoose});
     JoinHeader H{};
     uint8_t* rows_at = nullptr;
     if (P > 0) {
-        ENS(kOut, all.end);
         rows_at = buf<uint8_t>(ctx, kOut);
         JoinRows rows{(JoinHeader*)rows_at, (int*)(rows_at + all.q), (int*)(rows_at + all.t), (float*)(rows_at + all.d),
                       exact ? (double*)(rows_at + head) : nullptr, (int64_t)bound, ctx->d_counter + 8, ctx->d_stats, fetch_ctr};
