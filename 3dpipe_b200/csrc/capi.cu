@@ -251,6 +251,8 @@ int tdp_last_stats(const tdp_ctx* ctx, tdp_stats* o) {
     o->candidate_redone = s.candidate_redone;
     o->exact_dropped_items = s.exact_dropped_items;
     o->exact_below_items = s.exact_below_items;
+    o->lod_full_items = s.lod_full_items;
+    o->exact_full_items = s.exact_full_items;
     return TDP_OK;
 }
 

@@ -47,6 +47,8 @@ struct LastStats {
     long candidate_redone = 0;       // kNN queries redone with the global ring-search buffer
     long exact_dropped_items = 0;    // exact stage: FP32-pass items dropped by the item-level test
     long exact_below_items = 0;      // exact stage: FP32-pass items below their preset
+    long lod_full_items = 0;         // LOD loop: items that found a queue full
+    long exact_full_items = 0;       // exact stage: the same
 };
 
 }  // namespace tdp

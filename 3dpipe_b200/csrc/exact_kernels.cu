@@ -658,6 +658,7 @@ int read_info(tdp_ctx* ctx, const unsigned* ctr, long dropped, ExactInfo& info) 
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TDP_ERR_CUDA, std::string("exact-distance stage: ") + cudaGetErrorString(e));
     info.f64_items = ns[0];
+    info.full_items = ns[1];
     float e32;
     std::memcpy(&e32, &ns[4], 4);
     info.max_rel_err32 = e32;
@@ -812,6 +813,7 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
         CU(cudaGetLastError());
         CU(cudaEventRecord(ctx->xev[2], s));
         L.n_full = reinterpret_cast<unsigned long long*>(ctr + 12);
+        L.n_over = ctr + 5;
         CU(launch_fetch_list(kNumLods - 1, lz1, lz2, L.list1, L.ctr + cList1, L.self ? nullptr : L.list2, L.ctr + cList2,
                              ctx->num_sms, s));
         CU(launch_lod_exact_begin(L, kChunk, chunks, s));

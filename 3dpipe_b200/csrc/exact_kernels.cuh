@@ -18,6 +18,7 @@ struct ExactInfo {
     unsigned long long full_evals = 0;  // triangle pairs the FP32 pass evaluated fully
     long dropped_items = 0;  // FP32 pass items dropped by the refine's item-level test
     long below_items = 0;    // FP32 pass items with a triangle pair below their preset
+    long full_items = 0;     // items that found a queue of the task form full
 };
 
 // For every object pair with pstat == kReported: the exact minimum triangle

@@ -802,6 +802,7 @@ __global__ void __launch_bounds__(kEvalBlock, 4) k_lod_eval(LodDev L, int k, int
     uint4* q = queues[threadIdx.x >> 5];
     unsigned* ctr = L.ctr + pass * kLodCtrWords;
     const unsigned n = min(ctr[cEvals], L.eval_cap), n_over = ctr[cOver];
+    if (n_over && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.n_over, n_over);
     const float4* tri1 = L.tri1[k];
     const float4* tri2 = L.tri2[k];
     const float4* cl2 = L.self ? L.cl1 : L.cl2;

@@ -72,6 +72,7 @@ struct LodDev {
     unsigned* n_items;         // per LOD item counts (zeroed)
     unsigned long long* tri_pairs;
     unsigned long long* n_full;
+    unsigned* n_over;  // items that found a queue full (statistic)
     int use_preset;  // last LOD of a join with within queries: no distance above the query's
     float tau;
     int num_sms;

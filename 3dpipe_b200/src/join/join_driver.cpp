@@ -628,6 +628,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             t.n_items = ctx->d_counter + 24;
             t.tri_pairs = (unsigned long long*)(ctx->d_counter + 10);
             t.n_full = ctx->d_stats;
+            t.n_over = ctx->d_counter + 12;
             t.use_preset = presets ? 1 : 0; t.tau = within_dist; t.num_sms = ctx->num_sms;
         }
         if ((rc = run_lod_loop(ctx, L, s, &st.lod_graph))) return rc;
@@ -720,6 +721,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
             st.refine_ms_lod[lod_index(lods[k])] = ms;
         }
         full_total = fe;
+        st.lod_full_items = st.lod_tasks ? tc[4] : 0;  // d_counter[12]
         undecided = lods.back() == 100 ? tc[24] : 0;  // d_counter[32]
         st.recheck_pairs = undecided;
     }
@@ -768,6 +770,7 @@ int tdp_join(tdp_ctx* ctx, const tdp_tile* t1, const tdp_tile* t2, const tdp_joi
         st.exact_full_evals = xi.full_evals;
         st.exact_dropped_items = xi.dropped_items;
         st.exact_below_items = xi.below_items;
+        st.exact_full_items = xi.full_items;
     }
     ctx->stats = st;
     *out = R;

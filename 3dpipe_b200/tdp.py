@@ -47,7 +47,7 @@ class Stats(C.Structure):
                 ("refine_ms_lod", C.c_double * 5), ("exact_phase_ms", C.c_double * 4),
                 ("exact_full_evals", C.c_ulonglong), ("candidates_on_device", C.c_long),
                 ("candidate_redone", C.c_long), ("exact_dropped_items", C.c_long),
-                ("exact_below_items", C.c_long)]
+                ("exact_below_items", C.c_long), ("lod_full_items", C.c_long), ("exact_full_items", C.c_long)]
 
     def as_dict(self):
         d = {k: getattr(self, k) for k, _ in self._fields_}

@@ -103,6 +103,10 @@ typedef struct {
                                         bounds left no triangle pair           */
     long exact_below_items;          /* exact stage: FP32-pass voxel pairs with
                                         a triangle pair below their preset     */
+    long lod_full_items;             /* LOD loop: voxel pairs, over all LODs,
+                                        that found a queue full and were gone
+                                        through by one warp each               */
+    long exact_full_items;           /* the same of the exact stage            */
 } tdp_stats;
 int tdp_last_stats(const tdp_ctx *ctx, tdp_stats *out);
 /* measured FP32 FMA throughput of the context's device in TFLOP/s (CUDA cores,
