@@ -1160,14 +1160,14 @@ extern "C" int tdp_raw_from_meshes(tdp_ctx* ctx, const float* vertices, const in
         if (!all.empty()) CU(cudaMemcpyAsync(dl, all.data(), 4 * all.size(), cudaMemcpyHostToDevice, s));
         if (!small.empty()) {
             auto kern = k_decimate<uint16_t, 128>;
-            CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_small));
+            CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSmall));  // (one limit for every thread)
             kern<<<(int)std::min<size_t>(small.size(), 1u << 30), 128, s_small, s>>>(Mh, dl, (int)small.size(), dls,
                                                                                     nullptr, nullptr, lodF, Ftot, lodCnt);
             CU(cudaGetLastError());
         }
         if (!large.empty()) {
             auto kern = k_decimate<uint16_t, 256>;
-            CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_large));
+            CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLarge));
             kern<<<(int)large.size(), 256, s_large, s>>>(Mh, dl + small.size(), (int)large.size(), dls, nullptr, nullptr,
                                                         lodF, Ftot, lodCnt);
             CU(cudaGetLastError());
