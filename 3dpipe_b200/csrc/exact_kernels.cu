@@ -45,6 +45,7 @@
 #include <float.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 
@@ -673,14 +674,38 @@ int read_info(tdp_ctx* ctx, const unsigned* ctr, long dropped, ExactInfo& info) 
     return TDP_OK;
 }
 
-// Candidates that go through the task queues at a time: those hold 16 cluster
-// pairs and 8 triangle pairs a candidate (128 and 64 MB), about twice what the
-// joins measured here bring.
-constexpr int64_t kChunk = 1 << 19;
+// Candidates that go through the task queues at a time, and the queues' sizes (at
+// most 8.4 M cluster pairs and as many triangle pairs, 128 MB each).  Of c cluster
+// pairs a candidate the joins measured here queue c / 13 to c / 50 and, as fewer
+// are told apart by the bounds of larger voxels, c^1.5 / 700 to c^1.5 / 300 triangle
+// pairs (c = 169 to 100,000).  Candidates that find a queue full are gone through
+// by one warp each, which took five times as long as all the rest where every
+// candidate had room for 16 and 8: 5-NN of 2,000 x 50, voxels of 200 triangles
+// 20 -> 4.1 ms, of 500 49 -> 7.9 (the lazy form below: 12.5 and 26).
+struct ChunkSize {
+    int64_t items;
+    size_t tasks, evals;
+};
+constexpr int64_t kChunkMost = 1 << 19, kChunkLeast = 8192;  // (a warp culls one candidate)
+constexpr size_t kQueueLeast = 1 << 17, kQueueMost = 1 << 23;
+
+ChunkSize chunk_size(const tdp_tile* t1, const tdp_tile* t2, int64_t E) {
+    auto clusters = [](const tdp_tile* t) {  // of a voxel, in the mean
+        return (double)t->host.n_tris[kNumLods - 1] / kCl / (double)std::max<long>(t->n_vox, 1) + 0.5;
+    };
+    const double c = clusters(t1) * clusters(t2);
+    const double tasks = std::max(16.0, c / 16), evals = std::max(8.0, c * std::sqrt(c) / 256);
+    const int64_t fit = (int64_t)((double)kQueueMost / std::max(tasks, evals));
+    const int64_t items = std::min(E, std::max(kChunkLeast, std::min(kChunkMost, fit)));
+    auto queue = [&](double each) {
+        return std::max(kQueueLeast, std::min(kQueueMost, (size_t)std::min(each * (double)items, 1e9)));
+    };
+    return ChunkSize{items, queue(tasks), queue(evals)};
+}
 
 // Scratch of the task pass over L.d.V candidates (the LOD loop's, and this
 // stage's own slots); false when it does not fit.
-bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t2, size_t Pz) {
+bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t2, size_t Pz, const ChunkSize& chunk) {
     if (!t1->d_boxes || !t2->d_boxes) return false;
     const size_t E = (size_t)L.d.V;
     L.self = t1 == t2;
@@ -696,9 +721,9 @@ bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t
     L.nvox2 = L.self ? 0 : std::max<long>(t2->n_vox, 1);
     L.num_sms = ctx->num_sms;
     // most candidates end at their clusters; what finds a queue full is evaluated whole
-    const size_t C = std::min<size_t>(E, kChunk);
-    L.task_cap = (unsigned)std::max<size_t>(16 * C, 1 << 17);
-    L.eval_cap = (unsigned)std::max<size_t>(8 * C, 1 << 17);
+    const size_t C = (size_t)chunk.items;
+    L.task_cap = (unsigned)chunk.tasks;
+    L.eval_cap = (unsigned)chunk.evals;
     const size_t c1 = t1->host.n_tris[kNumLods - 1] / 8 + (size_t)L.nvox1 + 1;
     const size_t c2 = t2->host.n_tris[kNumLods - 1] / 8 + (size_t)std::max<long>(t2->n_vox, 1) + 1;
     const size_t nv = (size_t)(L.nvox1 + L.nvox2);
@@ -715,7 +740,7 @@ bool task_scratch(tdp_ctx* ctx, LodDev& L, const tdp_tile* t1, const tdp_tile* t
     // the LOD loop's block: that loop is done with it
     Carve c;
     const size_t over = c.take(C * 4), flag = c.take(nv * 4), list = c.take(nv * 4);
-    const size_t words = c.take((E / kChunk + 1) * kLodCtrWords * sizeof(unsigned));
+    const size_t words = c.take((E / C + 1) * kLodCtrWords * sizeof(unsigned));
     const size_t cl1 = c.take(c1 * 3 * sizeof(float4)), vb1 = c.take((size_t)L.nvox1 * 2 * sizeof(float4));
     const size_t cl2 = c.take(L.self ? 0 : c2 * 3 * sizeof(float4)), vb2 = c.take((size_t)L.nvox2 * 2 * sizeof(float4));
     const size_t tasks = c.take((size_t)L.task_cap * sizeof(LodTask)), evals = c.take((size_t)L.eval_cap * sizeof(LodEval));
@@ -799,12 +824,13 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
     L.d.V = E;
     L.pcap = Ub;
     L.dir = dir;
-    if (LodScratchUse in_use(ctx); E > 0 && task_scratch(ctx, L, t1, t2, Pz)) {
+    const ChunkSize chunk = chunk_size(t1, t2, std::max<int64_t>(E, 1));
+    if (LodScratchUse in_use(ctx); E > 0 && task_scratch(ctx, L, t1, t2, Pz, chunk)) {
         // phases 2 and 3 as one pass of the LOD loop's task kernels, over the
         // candidates as items, with U as the pairs' caps
         unsigned long long* bits = reinterpret_cast<unsigned long long*>(pexact);
         CU(cudaMemsetAsync(ctr, 0, 64, s));
-        const int chunks = (int)((E + kChunk - 1) / kChunk);
+        const int chunks = (int)((E + chunk.items - 1) / chunk.items);
         CU(cudaMemsetAsync(L.ctr, 0, (size_t)chunks * kLodCtrWords * sizeof(unsigned), s));
         CU(cudaMemsetAsync(L.pown, 0, 2 * Pz, s));
         CU(cudaMemsetAsync(L.pd, 0x7f, Pz * 4, s));
@@ -816,15 +842,15 @@ int exact_distances(tdp_ctx* ctx, const JoinDev& d, const tdp_tile* t1, const td
         L.n_over = ctr + 5;
         CU(launch_fetch_list(kNumLods - 1, lz1, lz2, L.list1, L.ctr + cList1, L.self ? nullptr : L.list2, L.ctr + cList2,
                              ctx->num_sms, s));
-        CU(launch_lod_exact_begin(L, kChunk, chunks, s));
+        CU(launch_lod_exact_begin(L, chunk.items, chunks, s));
         for (int c = 0; c < chunks; ++c) {
             LodDev C = L;
-            C.items += c * kChunk;
-            C.ext += c * kChunk;
-            C.vox += c * kChunk;
-            C.mg += c * kChunk;
+            C.items += c * chunk.items;
+            C.ext += c * chunk.items;
+            C.vox += c * chunk.items;
+            C.mg += c * chunk.items;
             C.ctr += (size_t)c * kLodCtrWords;
-            C.d.V = std::min(kChunk, E - c * kChunk);
+            C.d.V = std::min(chunk.items, E - c * chunk.items);
             CU(launch_lod_exact(C, s));
             if (c + 1 == chunks) CU(cudaEventRecord(ctx->xev[3], s));
             CU(launch_lod_f64(C, bits, ctr + 4, s));

@@ -470,6 +470,13 @@ constexpr int kCullWarps = 8;
 constexpr int kCullBuf = 96;  // tasks a warp collects before it claims queue slots (>= 63 + 32)
 constexpr int kSide = 16;     // clusters of one side that are looked at together
 
+// Item w is evaluated whole.  (Looked at first: an item can have thousands of
+// entries that do not fit.)
+__device__ __forceinline__ void go_whole(const LodDev& L, unsigned* ctr, unsigned w) {
+    int* in_over = (int*)&L.mg[w].w;
+    if (__ldcg(in_over) == 0 && atomicExch(in_over, 1) == 0) L.over[atomicAdd(ctr + cOver, 1u)] = w;
+}
+
 // Queue `cnt` of the warp's collected tasks.  Items whose tasks find the
 // queue full go to the list of items that are evaluated whole, once each.
 __device__ __forceinline__ void flush_tasks(const LodDev& L, unsigned* ctr, const LodTask* buf, int cnt, int lane,
@@ -483,7 +490,7 @@ __device__ __forceinline__ void flush_tasks(const LodDev& L, unsigned* ctr, cons
     for (int i = lane; i < cnt; i += 32) {
         const LodTask t = buf[i];
         if (base + i < L.task_cap) L.tasks[base + i] = t;
-        else if (atomicExch((int*)&L.mg[t.w].w, 1) == 0) L.over[atomicAdd(ctr + cOver, 1u)] = t.w;
+        else go_whole(L, ctr, t.w);
     }
     __syncwarp();
 }
@@ -734,7 +741,7 @@ __global__ void __launch_bounds__(kTestWarps * 32, 5) k_lod_test(LodDev L, int k
         for (int i = lane; i < bn; i += 32) {
             const LodEval e = buf[i];
             if (base + i < L.eval_cap) L.evals[base + i] = e;
-            else if (atomicExch((int*)&L.mg[e.w].w, 1) == 0) L.over[atomicAdd(ctr + cOver, 1u)] = e.w;
+            else go_whole(L, ctr, e.w);
         }
         __syncwarp();
         bn = 0;
@@ -751,6 +758,7 @@ __global__ void __launch_bounds__(kTestWarps * 32, 5) k_lod_test(LodDev L, int k
             const float4 g = L.mg[t.w];
             lim = gap_limits<MODE>(L, k, x.y, thresholds<MODE>(L, x.x, x.y, g.y, g.z), g.x);
             have = !(t.z >= lim.x) || (MODE != kLast && !(t.y >= lim.y));
+            have = have && __float_as_int(g.w) == 0;  // (else its item is evaluated whole)
         }
         const unsigned m = __ballot_sync(kFull, have);
         if (!m) continue;

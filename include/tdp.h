@@ -89,9 +89,9 @@ typedef struct {
     double exact_phase_ms[4];        /* exact stage, device time of: upper
                                         bounds (with their FP32 seeds),
                                         candidate voxel pairs, the FP32 pass,
-                                        the FP64 pass (of more than 524,288
-                                        candidates: of the last part; the
-                                        others' FP64 counts as FP32)           */
+                                        the FP64 pass (of candidates that go
+                                        through in several parts: of the last
+                                        part; the others' FP64 counts as FP32) */
     unsigned long long exact_full_evals; /* exact stage: triangle pairs fully
                                         evaluated by its FP32 pass             */
     long candidates_on_device;       /* 1: object candidates were computed on
