@@ -371,7 +371,7 @@ int tdp_refine_batch(tdp_ctx* ctx, const float* data, const float* hausdorff, si
         const double share = std::max((double)kPartLeast, tri_pairs / ((double)ctx->num_sms * kRefineWarpsPerSm * kPartsPerWarp));
         if (share < (double)most) {
             std::vector<uint32_t> first(pair_num + 1);
-            parts.reserve(2 * (size_t)pair_num);
+            parts.reserve(pair_num + 2 * (size_t)ctx->num_sms * kRefineWarpsPerSm * kPartsPerWarp);  // (the share's doing)
             for (uint32_t i = 0; i < pair_num; ++i) {
                 const RefineItem& it = items[i];
                 first[i] = (uint32_t)parts.size();
