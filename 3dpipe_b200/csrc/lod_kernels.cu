@@ -1,8 +1,9 @@
 // lod_kernels.cu -- one LOD of the tuned join as a chain of task kernels.
 //
 // The same decisions as the one-warp-per-voxel-pair refine (refine.cu) with
-// k_apply_results and k_pair_update behind it: every value a decision reads
-// has the same bits.  What differs is which triangle pairs are looked at.
+// k_apply_results and k_pair_update behind it: every bound and distance that a
+// decision reads has the same bits; a voxel pair's error term is another sound
+// one (k_lod_cull).  What differs is which triangle pairs are looked at.
 //
 // A decision reads, of a pair's voxel pairs, only the smallest upper bound
 // (d + h1 + h2) of the pair and each voxel pair's own lower bound
@@ -32,14 +33,14 @@
 // One warp per voxel pair spent half of its issue slots on staging bounds and
 // culling against loose per-item minima, and a LOD of few voxel pairs took as
 // long as its slowest one.  Here most items end after one pass over cluster
-// pairs and the rest of the work is spread over the chip.  Whole joins on one
-// B200, before (configuration 0, or autotuned where noted) and with this file:
-//   10-NN, 20,000 nuclei x 100 vessels   35.4 -> 6.0 ms
-//       (137 M full triangle evaluations -> 1.9 M)
-//   10-NN self-join, 3,000 nuclei        23.9 (autotuned) -> 4.6 ms
-//   within 60 self-join, 4,181 nuclei    3.5 -> 1.0 ms
-//   within 150, 2,000 x 100              1.87 -> 0.74 ms
-//   within 400, 20,000 x 100             1.14 (autotuned) -> 0.86 ms
+// pairs and the rest of the work is spread over the chip.  The loop's refine on
+// one B200 (kernels between a LOD's items and its update, five LODs), with one
+// warp per voxel pair (configuration 0 of it) and with this file:
+//   10-NN, 20,000 nuclei x 100 vessels   30.5 -> 2.9 ms (137 M full evaluations -> 1.9 M)
+//   10-NN self-join, 3,000 nuclei        35.7 -> 3.7 ms (158 M -> 2.4 M)
+//   within 60 self-join, 4,181 nuclei    2.87 -> 0.52 ms
+//   within 150, 2,000 x 100              1.28 -> 0.22 ms
+//   within 400, 20,000 x 100             0.51 -> 0.17 ms
 // Evaluating inside the kernel that tests the triangle pairs (128 registers,
 // 16 warps per SM) took 2.4 times the two kernels' time: the tests wait for
 // loads and want many warps, the evaluations want registers.
@@ -582,7 +583,13 @@ __global__ void __launch_bounds__(kCullWarps * 32) k_lod_cull(LodDev L, int k, i
                 if (MODE == kObjH) L.vres[v] = FLT_MAX;
                 // The voxel pair's own upper bound enters only its error term
                 // (4 u of it); where it is not kept, the middle between the
-                // least it can be and its core distance stands in.
+                // least it can be and its core distance stands in.  That is
+                // sound: the term has to cover the bounds that a decision
+                // takes from this voxel pair.  Its lower bound only falls from
+                // mn; its upper bound is the pair's only where it is the least
+                // of all, so at most th.x and at most every core distance, and
+                // the middle is not below that.  (Not the bits of the one-warp
+                // form's term, which its own minimum enters.)
                 const float mn = d.vmn[v], core = __ldcg(d.vmx + v);
                 const float mx = L.pown[x.y] ? core : 0.5f * (core + fminf(core, fmaxf(mn, th.x)));
                 d.verr[v] = fmaxf(d.verr[v], e + 4.f * kUnitRoundoff * fmaxf(fabsf(mn), fabsf(mx)));

@@ -18,7 +18,8 @@ RAW .dt format.  The reference publishes no numbers, so vs_baseline is null.
                fetching each LOD's refined voxels from the host bytes, result
                read-back, tiles released; fresh tiles every step (the whole
                upload path is reported beside it)
-  roofline     the dominant kernel (tuned refine), FP32 CUDA-core bound
+  roofline     the refine of the LOD loop, FP32 CUDA-core bound: the triangle pairs
+               that it evaluates (the bounds' operations are not counted)
   cpu_baseline the reference's own CPU code (MeshDist, octree; compiled from
                source into oracle/_ref) on a bounded sample of query nuclei,
                all host cores
@@ -48,7 +49,6 @@ WORKLOAD = "within-400 join, 1000 vessels x 200 nuclei (200k nuclei), LODs 20-10
 N_VESSELS, NUCLEI_PER_VESSEL, TAU, SEED = 1000, 200, 400.0, 20260002
 METRIC = "tri-pairs/s of the within-400 spatial join (filter + LOD refine), tuned form"
 F_TRI = 966.0      # FLOPs of one full triangle-pair evaluation (3dpipe_b200/csrc/tridist.cuh)
-F_CULL = 14.0      # FLOPs of one bounding-sphere cull test (refine_tuned_kernel)
 
 
 def log(*a):
@@ -794,7 +794,7 @@ def main():
         plain_value = allsum(st_p["tri_pairs"]) / (plain_ms / 1e3)
         refine_ms = agg_t["refine_ms"]
         launches_refine = max(1, st_t["refine_launches"])
-        flops = agg_t["full_evals"] * F_TRI + agg_t["tri_pairs"] * F_CULL
+        flops = agg_t["full_evals"] * F_TRI
         achieved = flops / (refine_ms / 1e3) / 1e12
 
         # config 3: the 10-NN self-join over the same 200k nuclei (tuned form;
@@ -923,10 +923,11 @@ def main():
     cpu = None
     if rank == 0 and ws == 1 and not a.no_cpu:
         cpu = cpu_reference(nb, vb, 3, 0, a.cpu_sample, target_s=5.0)
-    # DRAM bytes per refine launch from the committed ncu capture of this workload
+    # DRAM bytes per refine launch of the one-warp refine from the committed ncu capture of this workload
+    tasks = all(v == 0 for v in cfg_by_lod.values())
     traffic = None
     prof = ROOT / "profiles" / "refine_within400.md"
-    if prof.exists():
+    if prof.exists() and not tasks:
         for ln in prof.read_text().splitlines():
             if ln.startswith("traffic_bytes_per_launch:"):
                 try:
@@ -967,16 +968,19 @@ def main():
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": achieved / fp32_peak if fp32_peak else None, "traffic": traffic,
                          "traffic_source": "DRAM read+write bytes per launch: ncu capture of the 20k-nuclei case, "
-                                           "scaled by the refined voxel pairs (profiles/refine_within400.md)",
-                         "kernel": "refine_lazy_kernel" if cfg_by_lod[100] >= 3 else "refine_tuned_kernel",
+                                           "scaled by the refined voxel pairs (profiles/refine_within400.md)"
+                                           if traffic is not None else
+                                           "not captured at this size (small cases: profiles/lod_tasks_knn_self_3k.md)",
+                         "kernel": ("k_lod_clusters, k_lod_seed, k_lod_cull, k_lod_test, k_lod_eval (one launch each a LOD)"
+                                    if tasks else "refine_lazy_kernel" if cfg_by_lod[100] >= 3 else "refine_tuned_kernel"),
                          "peak_source": "measured FP32 FMA probe (tdp_fp32_peak); MEASURED_PEAKS.json has no CUDA-core FP32 figure",
-                         "work": f"full evals x {F_TRI:.0f} + culled pairs x {F_CULL:.0f} FLOPs",
+                         "work": f"full evals x {F_TRI:.0f} FLOPs",
                          "tri_pair_equivalent": {
                              "achieved": agg_t["tri_pairs"] * F_TRI / (refine_ms / 1e3) / 1e12,
                              "frac": (agg_t["tri_pairs"] * F_TRI / (refine_ms / 1e3) / 1e12) / fp32_peak
                              if fp32_peak else None,
                              "note": "every triangle pair of every refined voxel pair counted at F_TRI; above 1.0 "
-                                     "because the tuned form proves most pairs irrelevant with a ~14-FLOP bound"},
+                                     "because most pairs end with the bounds of their clusters or voxels"},
                          "launches_per_step": launches_refine},
             "clocks": clocks,
             "cpu_baseline": {k: cpu[k] for k in ("value", "unit", "cores", "kind", "sample")} if cpu else None,
